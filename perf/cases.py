@@ -193,7 +193,7 @@ class _Plan:
     """A plan handle, destroyed with the object."""
 
     def __init__(self, case, x):
-        L = fmm.lib()
+        L = self.L = fmm.lib()
         L.fmm2d_b200_plan_create.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_double,
                                              ctypes.c_int, P] + [ctypes.c_int] * 4 + \
             [P, ctypes.c_int, ctypes.POINTER(P)]
@@ -209,7 +209,7 @@ class _Plan:
 
     def __del__(self):
         if self.h:
-            fmm.lib().fmm2d_b200_plan_destroy(self.h)
+            self.L.fmm2d_b200_plan_destroy(self.h)
 
 
 def prepare(case, seed):
