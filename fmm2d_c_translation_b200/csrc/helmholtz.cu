@@ -23,9 +23,10 @@
 //     (multipoles of list 3) and downward J (the leaf's local expansion),
 //     derivatives from the mk_mpoleg / mk_mpoleh coefficient recurrences
 //     evaluated on the fly.
-//   * P2P (hfmm2dpart_direct -> h2d_direct*): one thread per point over the
-//     sources of list 1; H0, H1 per pair from hankel.cuh (the CUDA libm J0,
-//     J1, Y0, Y1 below argument 8 for real wavenumbers).
+//   * P2P (hfmm2dpart_direct -> h2d_direct*): one warp per leaf over the
+//     sources of list 1 (several densities: one thread per point); H0, H1
+//     per pair from one table for a positive real wavenumber
+//     (helm_bessel.cuh), else from hankel.cuh.
 #include "helmholtz.cuh"
 
 #include <algorithm>
@@ -36,6 +37,7 @@
 #include <vector>
 
 #include "hankel.cuh"
+#include "helm_bessel.cuh"
 #include "laplace.cuh"
 
 namespace fmm2d {
@@ -1134,6 +1136,82 @@ __device__ __forceinline__ void pair_add(Acc &a, double dx, double dy, double2 z
     }
 }
 
+// The same interaction for a real wavenumber k (k2 = k^2), less the factor
+// i/4, which the caller applies to the sums.  With g = H1(kr) / (kr) the
+// radial derivatives of f = H0(kr) are
+//   F1 = f'/r = -k^2 g,  F2 = F1'/r = k^2 (2 g - H0) / r^2,
+//   F3 = F2'/r = -(k^2 F1 + 4 F2) / r^2,
+// so the pair needs H0 and g (one table lookup, helm_bessel.cuh) and one
+// reciprocal.  thresh2 is the threshold's square.
+// (a call: its loops would cost the pair loop registers)
+__device__ __noinline__ void hankel01_far(double s, double2 &h0, double2 &g) {
+    const double x = sqrt(s);
+    double2 h1;
+    hk::hankel01(make_double2(x, 0.0), h0, h1);
+    g = cscal(h1, 1.0 / x);
+}
+
+template <int PGH, bool IFC, bool IFD>
+__device__ __forceinline__ void pair_add_real(Acc &a, double dx, double dy, double k2,
+                                              double thresh2, bool le, double2 q, double2 d,
+                                              double2 v) {
+    const double s = (dx * dx + dy * dy) * k2;
+    if (le ? (s <= thresh2) : (s < thresh2)) return;
+    const double si = 1.0 / s;
+    double2 h0, g;
+    if (s < hb::kSMax) {
+        hb::hankel01_sq(s, si, h0, g);
+    } else {
+        hankel01_far(s, h0, g);
+    }
+    const double2 f1 = cscal(g, -k2);
+    const double rho = k2 * si;  // 1 / r^2
+    double2 f2, f3;
+    if (PGH >= 2) f2 = cscal(csub(cscal(g, 2.0), h0), k2 * rho);
+    if (PGH >= 3 && IFD)
+        f3 = make_double2(-rho * fma(k2, f1.x, 4.0 * f2.x), -rho * fma(k2, f1.y, 4.0 * f2.y));
+    if (IFC) {
+        cfma(a.p, h0, q);
+        if (PGH >= 2) {
+            const double2 t = cmul(f1, q);
+            a.gx = make_double2(fma(t.x, dx, a.gx.x), fma(t.y, dx, a.gx.y));
+            a.gy = make_double2(fma(t.x, dy, a.gy.x), fma(t.y, dy, a.gy.y));
+            if (PGH >= 3) {
+                const double2 u = cmul(f2, q);
+                const double xx = dx * dx, xy = dx * dy, yy = dy * dy;
+                a.hxx = make_double2(fma(u.x, xx, a.hxx.x + t.x), fma(u.y, xx, a.hxx.y + t.y));
+                a.hxy = make_double2(fma(u.x, xy, a.hxy.x), fma(u.y, xy, a.hxy.y));
+                a.hyy = make_double2(fma(u.x, yy, a.hyy.x + t.x), fma(u.y, yy, a.hyy.y + t.y));
+            }
+        }
+    }
+    if (IFD) {
+        const double sv = dx * v.x + dy * v.y;
+        const double2 e1 = cmul(f1, d);
+        a.p = make_double2(fma(e1.x, -sv, a.p.x), fma(e1.y, -sv, a.p.y));
+        if (PGH >= 2) {
+            const double2 e2 = cmul(f2, d);
+            const double xs = dx * sv, ys = dy * sv;
+            a.gx = make_double2(a.gx.x - fma(e2.x, xs, e1.x * v.x),
+                                a.gx.y - fma(e2.y, xs, e1.y * v.x));
+            a.gy = make_double2(a.gy.x - fma(e2.x, ys, e1.x * v.y),
+                                a.gy.y - fma(e2.y, ys, e1.y * v.y));
+            if (PGH >= 3) {
+                const double2 e3 = cmul(f3, d);
+                const double cx = sv + 2.0 * dx * v.x, cy = sv + 2.0 * dy * v.y,
+                             cxy = dx * v.y + dy * v.x;
+                const double xxs = dx * xs, xys = dy * xs, yys = dy * ys;
+                a.hxx = make_double2(a.hxx.x - fma(e3.x, xxs, e2.x * cx),
+                                     a.hxx.y - fma(e3.y, xxs, e2.y * cx));
+                a.hxy = make_double2(a.hxy.x - fma(e3.x, xys, e2.x * cxy),
+                                     a.hxy.y - fma(e3.y, xys, e2.y * cxy));
+                a.hyy = make_double2(a.hyy.x - fma(e3.x, yys, e2.x * cy),
+                                     a.hyy.y - fma(e3.y, yys, e2.y * cy));
+            }
+        }
+    }
+}
+
 template <int PGH>
 __device__ __forceinline__ void store_add(const Acc &a, long long t, int nd, int c, double2 *pot,
                                           double2 *grad, double2 *hess) {
@@ -1209,7 +1287,9 @@ constexpr size_t helm_p2p_flat_warp_bytes() {
            (size_t)kHfItems * hf_outs<PGH>() * sizeof(double2);
 }
 
-template <int PGH, bool REALK>
+// KIND 0: any wavenumber; 1, 2, 3: a positive real one with charges, dipoles,
+// both (pair_add_real).
+template <int PGH, int KIND>
 __global__ void __launch_bounds__(kHfWarps * 32) helm_p2p_flat_kernel(
     int nb, const int *__restrict__ nchild, const int2 *__restrict__ tse,
     const double2 *__restrict__ pos, const int *__restrict__ nlist1,
@@ -1225,6 +1305,7 @@ __global__ void __launch_bounds__(kHfWarps * 32) helm_p2p_flat_kernel(
     double2 *s_tgt = s_v + kHfStage;
     double2 *part = s_tgt + 32;
     const bool le = ifc && !ifd && PGH == 1;
+    const double k2 = zk.x * zk.x, thresh2 = thresh * thresh;
     const double2 zero = make_double2(0.0, 0.0);
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
     for (int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < nb; b += nwarps) {
@@ -1291,8 +1372,14 @@ __global__ void __launch_bounds__(kHfWarps * 32) helm_p2p_flat_kernel(
                     const int j1 = min(nst, blk * sb + sb);
                     for (int kk = blk * sb; kk < j1; kk++) {
                         const double2 y = s_pos[kk];
-                        pair_add<PGH, REALK>(a, x.x - y.x, x.y - y.y, zk, thresh, le, ifc, s_q[kk],
-                                             ifd, s_d[kk], s_v[kk]);
+                        if (KIND == 0)
+                            pair_add<PGH, false>(a, x.x - y.x, x.y - y.y, zk, thresh, le, ifc,
+                                                 s_q[kk], ifd, s_d[kk], s_v[kk]);
+                        else
+                            pair_add_real<PGH, (KIND & 1) != 0, (KIND & 2) != 0>(
+                                a, x.x - y.x, x.y - y.y, k2, thresh2, le,
+                                (KIND & 1) ? s_q[kk] : zero, (KIND & 2) ? s_d[kk] : zero,
+                                (KIND & 2) ? s_v[kk] : zero);
                     }
                     double2 *pp = part + (size_t)it * NO;
                     pp[0] = a.p;
@@ -1323,6 +1410,7 @@ __global__ void __launch_bounds__(kHfWarps * 32) helm_p2p_flat_kernel(
                     }
                 }
             }
+            if (KIND != 0) tot.scale(make_double2(0.0, 0.25));  // i / 4
             if (lane < T) store_add<PGH>(tot, (long long)(tr.x + t0 + lane), 1, 0, pot, grad, hess);
         }
     }
@@ -1804,10 +1892,10 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
                                               T.list1.get(), T.srcse.get(), P.src, P.charge, \
                                               P.dipstr, P.dipvec, ifc, ifd, nd, zk, thresh,  \
                                               X.pot, X.grad, X.hess)
-#define HP2PF(PG, RK)                                                                        \
+#define HP2PF(PG, KD)                                                                        \
     do {                                                                                     \
         constexpr size_t sm = kHfWarps * helm_p2p_flat_warp_bytes<PG>();                     \
-        auto kern = helm_p2p_flat_kernel<PG, RK>;                                            \
+        auto kern = helm_p2p_flat_kernel<PG, KD>;                                            \
         raise_smem_limit((const void *)kern, sm);                                            \
         const int gw = std::max(1, std::min((nb + kHfWarps - 1) / kHfWarps, kNumSM * 16));   \
         kern<<<gw, kHfWarps * 32, sm, s>>>(nb, T.nchild.get(), X.se, X.pos, T.nlist1.get(),   \
@@ -1819,15 +1907,21 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
         const char *pm = getenv("FMM2D_B200_HELM_P2P");
         const bool flat = nd == 1 && !(pm && !strcmp(pm, "point"));
         if (flat) {
-            if (realk) {
-                if (X.pgh == 1) HP2PF(1, true);
-                else if (X.pgh == 2) HP2PF(2, true);
-                else HP2PF(3, true);
+#define HP2PK(KD)                          \
+    do {                                   \
+        if (X.pgh == 1) HP2PF(1, KD);      \
+        else if (X.pgh == 2) HP2PF(2, KD); \
+        else HP2PF(3, KD);                 \
+    } while (0)
+            if (!realk) {
+                HP2PK(0);
             } else {
-                if (X.pgh == 1) HP2PF(1, false);
-                else if (X.pgh == 2) HP2PF(2, false);
-                else HP2PF(3, false);
+                hb::ensure_table();
+                if (ifc && ifd) HP2PK(3);
+                else if (ifd) HP2PK(2);
+                else HP2PK(1);
             }
+#undef HP2PK
         } else if (realk) {
             if (X.pgh == 1) HP2P(1, true);
             else if (X.pgh == 2) HP2P(2, true);
