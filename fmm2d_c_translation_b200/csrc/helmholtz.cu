@@ -938,11 +938,12 @@ __global__ void __launch_bounds__(128) helm_far_kernel(
     const int *__restrict__ level, const double2 *__restrict__ centers,
     const int *__restrict__ nlist3, const int *__restrict__ list3, const HLevel *__restrict__ lv,
     int nlevels, const double2 *__restrict__ mp, const double2 *__restrict__ loc, int nd,
-    double2 zk, double2 *__restrict__ pot, double2 *__restrict__ grad,
+    double2 zk, int lmax, double2 *__restrict__ pot, double2 *__restrict__ grad,
     double2 *__restrict__ hess) {
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
         const int b = leaf[t];
         const int l = level[b];
+        if (l >= lmax) continue;
         const double2 x = pos[t];
         for (int c = 0; c < nd; c++) {
             Acc tot;
@@ -1232,6 +1233,8 @@ __device__ __forceinline__ void store_add(const Acc &a, long long t, int nd, int
         h2 = cadd(h2, a.hyy);
     }
 }
+
+#include "helm_real.cuh"
 
 // P2P over list 1 for one point set (the outputs already hold the far field).
 template <int PGH, bool REALK>
@@ -1697,18 +1700,50 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
     // ---- P2M, P2L ----
     // half warps per leaf when the leaves hold about 12 sources or fewer
     // (leaves are about three quarters of the boxes)
-    if ((double)P.sset.n <= 9.0 * nb)
-        helm_p2m_kernel<16><<<grid_for((int64_t)nb * 16, 256), 256, 0, s>>>(
-            nb, T.nchild.get(), T.level.get(), T.srcse.get(), T.centers.get(), d_lv.get(), P.src,
-            P.charge, P.dipstr, P.dipvec, ifc, ifd, nd, zk, mp.get());
+    const bool half = (double)P.sset.n <= 9.0 * nb;
+    // a positive real wavenumber: the levels from lreal on take the real
+    // kernels of helm_real.cuh, the larger boxes above them (and any other
+    // wavenumber) the general ones
+    const bool realk = zk.y == 0.0 && zk.x > 0.0;
+    int lreal = nl + 1;
+    if (realk) {
+        hb::ensure_table();
+        while (lreal > 0 && hl[lreal - 1].p <= kRealOrderMax &&
+               zk.x * T.boxsize[lreal - 1] * 0.7072 <= kRealXMax)
+            lreal--;
+        // (boxes of levels 0 and 1 have no expansions)
+        if (lreal <= 2) lreal = 0;
+    }
+    // boxes of the levels below lreal come first in the numbering
+    const int nbg = lreal <= nl ? T.lstart[lreal] : nb;
+#define HP2M(KERN, W_, N_, K_)                                                               \
+    KERN<W_><<<grid_for((int64_t)(N_) * W_, 256), 256, 0, s>>>(                              \
+        N_, T.nchild.get(), T.level.get(), T.srcse.get(), T.centers.get(), d_lv.get(), P.src, \
+        P.charge, P.dipstr, P.dipvec, ifc, ifd, nd, K_, mp.get())
+    if (lreal > 2) {
+        if (half) HP2M(helm_p2m_kernel, 16, nbg, zk);
+        else HP2M(helm_p2m_kernel, 32, nbg, zk);
+        FMM_CHECK_LAUNCH();
+    }
+#undef HP2M
+    if (lreal <= nl) {
+#define HP2MR(W_)                                                                            \
+    helm_p2m_real_kernel<W_><<<grid_for((int64_t)nb * W_, 256), 256, 0, s>>>(                \
+        nb, T.nchild.get(), T.level.get(), T.srcse.get(), T.centers.get(), d_lv.get(), P.src, \
+        P.charge, P.dipstr, P.dipvec, ifc, ifd, nd, zk.x, std::max(lreal, 2), mp.get())
+        if (half) HP2MR(16);
+        else HP2MR(32);
+#undef HP2MR
+        FMM_CHECK_LAUNCH();
+    }
+    if (realk)
+        helm_p2l_real_kernel<<<grid_for((int64_t)nb * 32, 256), 256, 0, s>>>(
+            nb, T.level.get(), T.nlist4.get(), T.list4.get(), T.srcse.get(), T.centers.get(),
+            d_lv.get(), P.src, P.charge, P.dipstr, P.dipvec, ifc, ifd, nd, zk.x, loc.get());
     else
-        helm_p2m_kernel<32><<<grid_for((int64_t)nb * 32, 256), 256, 0, s>>>(
-            nb, T.nchild.get(), T.level.get(), T.srcse.get(), T.centers.get(), d_lv.get(), P.src,
-            P.charge, P.dipstr, P.dipvec, ifc, ifd, nd, zk, mp.get());
-    FMM_CHECK_LAUNCH();
-    helm_p2l_kernel<<<grid_for((int64_t)nb * 32, 256), 256, 0, s>>>(
-        nb, T.level.get(), T.nlist4.get(), T.list4.get(), T.srcse.get(), T.centers.get(),
-        d_lv.get(), P.src, P.charge, P.dipstr, P.dipvec, ifc, ifd, nd, zk, loc.get());
+        helm_p2l_kernel<<<grid_for((int64_t)nb * 32, 256), 256, 0, s>>>(
+            nb, T.level.get(), T.nlist4.get(), T.list4.get(), T.srcse.get(), T.centers.get(),
+            d_lv.get(), P.src, P.charge, P.dipstr, P.dipvec, ifc, ifd, nd, zk, loc.get());
     FMM_CHECK_LAUNCH();
     prof_mark("h_p2m_p2l", s);
     // ---- M2M, upward (parents at levels nl-1 .. 2) ----
@@ -1867,7 +1902,6 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
     prof_mark("h_l2l", s);
     // ---- M2P + L2P, then P2P, per point set ----
     const double thresh = hk::cabs_(zk) * T.boxsize[0] * std::ldexp(1.0, -51);
-    const bool realk = zk.y == 0.0 && zk.x > 0.0;
     for (int set = 0; set < 2; set++) {
         const HPointSet &X = set == 0 ? P.sset : P.tset;
         if (X.pgh <= 0 || X.n <= 0) continue;
@@ -1875,16 +1909,23 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
         helm_leaf_of_kernel<<<grid_for(nb, 256), 256, 0, s>>>(nb, T.nchild.get(), X.se, leaf.get());
         FMM_CHECK_LAUNCH();
         const unsigned g = grid_for(X.n, 128);
-#define HFAR(PG)                                                                           \
-    helm_far_kernel<PG><<<g, 128, 0, s>>>(X.n, X.pos, leaf.get(), T.level.get(),           \
-                                          T.centers.get(), T.nlist3.get(), T.list3.get(),  \
-                                          d_lv.get(), nl, mp.get(), loc.get(), nd, zk,     \
-                                          X.pot, X.grad, X.hess)
-        if (X.pgh == 1) HFAR(1);
-        else if (X.pgh == 2) HFAR(2);
-        else HFAR(3);
+#define HFAR(KERN, PG, K_, LV_)                                                            \
+    KERN<PG><<<g, 128, 0, s>>>(X.n, X.pos, leaf.get(), T.level.get(), T.centers.get(),     \
+                               T.nlist3.get(), T.list3.get(), d_lv.get(), nl, mp.get(),    \
+                               loc.get(), nd, K_, LV_, X.pot, X.grad, X.hess)
+#define HFARP(KERN, K_, LV_)                     \
+    do {                                         \
+        if (X.pgh == 1) HFAR(KERN, 1, K_, LV_);  \
+        else if (X.pgh == 2) HFAR(KERN, 2, K_, LV_); \
+        else HFAR(KERN, 3, K_, LV_);             \
+        FMM_CHECK_LAUNCH();                      \
+    } while (0)
+        // (every leaf takes exactly one of the two, which is the first
+        // writer of its points' outputs)
+        if (lreal > 0) HFARP(helm_far_kernel, zk, lreal);
+        if (lreal <= nl) HFARP(helm_far_real_kernel, zk.x, lreal);
+#undef HFARP
 #undef HFAR
-        FMM_CHECK_LAUNCH();
         prof_mark(set == 0 ? "h_eval_src" : "h_eval_trg", s);
         if (!P.ifnear) continue;
 #define HP2P(PG, RK)                                                                        \
