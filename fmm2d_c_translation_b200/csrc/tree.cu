@@ -68,28 +68,180 @@ __device__ __forceinline__ int key_lcp(const KeyView &kv, int nw, int64_t a, int
     return 16 * nw;
 }
 
-// Number of boxes of every level 1..ds that hold more than ndiv of the
-// n key-sorted points: a box of level l is a run of equal l-digit prefixes,
-// and the run starting at k (a start when the prefix differs from k-1's,
-// i.e. l > lcp(k-1, k)) holds more than ndiv points when the point ndiv
-// further on still shares the prefix (l <= lcp(k, k + ndiv)).  Each point
-// adds one to the levels in (lcp(k-1, k), lcp(k, k + ndiv)].
-__global__ void __launch_bounds__(256) refine_count_kernel(KeyView kv, int64_t n, int ndiv,
-                                                           int ds, int nw,
-                                                           unsigned long long *__restrict__ cnt) {
-    __shared__ unsigned int sc[65];
-    for (int l = threadIdx.x; l <= 64; l += blockDim.x) sc[l] = 0;
-    __syncthreads();
-    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n;
-         k += (int64_t)gridDim.x * blockDim.x) {
-        if (k + ndiv >= n) continue;
-        const int a = k == 0 ? 0 : key_lcp(kv, nw, k - 1, k);
-        const int b = min(key_lcp(kv, nw, k, k + ndiv), ds);
-        for (int l = a + 1; l <= b; l++) atomicAdd(&sc[l], 1u);
+// ---------------------------------------------------------------------------
+// All levels of the refinement at once, from the sorted keys.
+//
+// A box of level l that holds sources is a run of equal l-digit prefixes of
+// the key-sorted sources, and it is refined when the run holds more than
+// ndiv points.  The run that starts at position k does so for exactly the
+// levels l with lcp(k-1, k) < l <= lcp(k, k + ndiv) (common leading
+// digits; -1 before the first point of a problem).  The boxes of a level are
+// numbered in path order, four children per refined box of the level above,
+// so a refined box's number, its children's numbers, centers and point
+// ranges follow from its rank among the refined boxes of its level, its
+// parent's rank and its digits: no level waits for the one above it.
+// Before, every level took a selection, a scan, a split and a search launch
+// (forests: and a host synchronisation).  Keys and levels together: 10^5
+// points 0.40 -> 0.24 ms, 64 problems of 2.5e5 points 0.64 -> 0.29 ms, 4e5
+// clustered points 1.05 -> 0.77 ms, 10^7 + 10^7 points 2.11 -> 1.93 ms.
+// ---------------------------------------------------------------------------
+constexpr int kRefLevels = 65;  // levels 0 .. 64
+
+// The runs at position k that are refined: levels (lo, hi].
+__device__ __forceinline__ void refined_levels(const KeyView &kv, const uint32_t *prob, int64_t n,
+                                               int ndiv, int ds, int nw, int64_t k, int &lo,
+                                               int &hi) {
+    lo = 0;
+    hi = -1;
+    if (k + ndiv >= n) return;
+    if (prob && prob[k + ndiv] != prob[k]) return;
+    lo = (k == 0 || (prob && prob[k - 1] != prob[k])) ? -1 : key_lcp(kv, nw, k - 1, k);
+    hi = min(key_lcp(kv, nw, k, k + ndiv), ds);
+}
+
+// Warp w takes the positions [w chunk, (w + 1) chunk).  COUNT: the number of
+// refined boxes per (level, warp) to cnt[level nwarp + w]; otherwise, with
+// cnt scanned in that order, their start positions in (level, path) order.
+template <bool COUNT>
+__global__ void __launch_bounds__(256) refine_runs_kernel(KeyView kv,
+                                                          const uint32_t *__restrict__ prob,
+                                                          int64_t n, int ndiv, int ds, int nw,
+                                                          int64_t chunk, int nwarp,
+                                                          int *__restrict__ cnt,
+                                                          int *__restrict__ start) {
+    __shared__ int run_all[8][kRefLevels];
+    const int lane = threadIdx.x & 31, w = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (w >= nwarp) return;
+    int *run = run_all[threadIdx.x >> 5];
+    for (int l = lane; l <= ds; l += 32) run[l] = COUNT ? 0 : cnt[(size_t)l * nwarp + w];
+    __syncwarp();
+    const int64_t k1 = min(n, (w + 1) * chunk);
+    for (int64_t k0 = w * chunk; k0 < k1; k0 += 32) {
+        const int64_t k = k0 + lane;
+        int lo = 0, hi = -1;
+        if (k < k1) refined_levels(kv, prob, n, ndiv, ds, nw, k, lo, hi);
+        const bool any = hi > lo;
+        const int l0 = __reduce_min_sync(0xffffffffu, any ? lo + 1 : kRefLevels);
+        const int l1 = __reduce_max_sync(0xffffffffu, any ? hi : -1);
+        for (int l = l0; l <= l1; l++) {
+            const bool f = lo < l && l <= hi;
+            const unsigned m = __ballot_sync(0xffffffffu, f);
+            if (!m) continue;
+            const int base = run[l];
+            if (!COUNT && f) start[base + __popc(m & ((1u << lane) - 1u))] = (int)k;
+            __syncwarp();
+            if (lane == 0) run[l] = base + __popc(m);
+            __syncwarp();
+        }
     }
-    __syncthreads();
-    for (int l = threadIdx.x; l <= 64; l += blockDim.x)
-        if (sc[l]) atomicAdd(&cnt[l], (unsigned long long)sc[l]);
+    if (COUNT)
+        for (int l = lane; l <= ds; l += 32) cnt[(size_t)l * nwarp + w] = run[l];
+}
+
+// Per-level counts of the refinement and the first entry of each level.
+struct RefineInfo {
+    int off[kRefLevels + 1];   // first entry of level l in the list of refined boxes
+    int base[kRefLevels + 1];  // first box of level l
+    int nlev;                  // levels with refined boxes
+};
+
+// One thread per refined box (entry e of level l, run start k): its number,
+// its child pointers, and its four children's centers, parents, levels and
+// point ranges.  Child counts start at zero and child pointers at -1 (set
+// before by memsets), so only refined boxes write them.
+__global__ void __launch_bounds__(128) build_boxes_kernel(
+    RefineInfo R, const int *__restrict__ start, KeyView kv, const uint32_t *__restrict__ prob,
+    int64_t n, KeyView kt, const uint32_t *__restrict__ probt, int64_t nt, int ndiv, int nw,
+    double2 c0, const double *__restrict__ bsl, double2 *__restrict__ cen, int *__restrict__ lev,
+    int *__restrict__ par, int *__restrict__ nch, int *__restrict__ chi, int2 *__restrict__ rs,
+    int2 *__restrict__ rt) {
+    const int tot = R.off[R.nlev];
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < tot; e += gridDim.x * blockDim.x) {
+        int l = 0;
+        while (R.off[l + 1] <= e) l++;
+        const int64_t k = start[e];
+        // this box's number: child digit under the refined box of level
+        // l - 1 whose run holds k (the last one starting at or before k)
+        int id;
+        if (l == 0) {
+            id = prob ? (int)prob[k] : 0;
+        } else {
+            int a = R.off[l - 1], b = R.off[l];
+            while (b - a > 1) {
+                const int mid = (a + b) >> 1;
+                if (start[mid] <= k) a = mid; else b = mid;
+            }
+            id = R.base[l] + 4 * (a - R.off[l - 1]) + key_digit(kv, k, l);
+        }
+        const int ch = R.base[l + 1] + 4 * (e - R.off[l]);
+        // end of the run: first position past k + ndiv of another prefix
+        auto same = [&](int64_t q) {
+            return (!prob || prob[q] == prob[k]) && (l == 0 || key_lcp(kv, nw, k, q) >= l);
+        };
+        int64_t a = k + ndiv, step = ndiv > 0 ? ndiv : 1, b = a + step;
+        while (b < n && same(b)) {  // (a is inside, b outside or n)
+            a = b;
+            step <<= 1;
+            b += step;
+        }
+        if (b > n) b = n;
+        while (b - a > 1) {
+            const int64_t mid = (a + b) >> 1;
+            if (same(mid)) a = mid; else b = mid;
+        }
+        const int64_t kend = a + 1;
+        // the box's range among the targets: keys with the same l digits
+        // (order of a key against this prefix: problem, then the words)
+        int64_t ta = 0, tb = 0;
+        if (nt > 0) {
+            auto cmp = [&](int64_t q) {  // -1 below, 0 in, 1 above the box
+                if (probt && probt[q] != prob[k]) return probt[q] < prob[k] ? -1 : 1;
+                for (int w = 0, left = l; left > 0; w++, left -= 16) {
+                    const int sh = left >= 16 ? 0 : 2 * (16 - left);
+                    const uint32_t x = kt.w[w][q] >> sh, y = kv.w[w][k] >> sh;
+                    if (x != y) return x < y ? -1 : 1;
+                }
+                return 0;
+            };
+            int64_t lo = 0, hi = nt;
+            while (lo < hi) {
+                const int64_t mid = (lo + hi) >> 1;
+                if (cmp(mid) < 0) lo = mid + 1; else hi = mid;
+            }
+            ta = lo;
+            hi = nt;
+            while (lo < hi) {
+                const int64_t mid = (lo + hi) >> 1;
+                if (cmp(mid) <= 0) lo = mid + 1; else hi = mid;
+            }
+            tb = lo;
+        }
+        double2 c = c0;
+        for (int m = 1; m <= l; m++) c = child_center(c, bsl[m], key_digit(kv, k, m));
+        const double bs = bsl[l + 1];
+        nch[id] = 4;
+        *reinterpret_cast<int4 *>(chi + 4 * (size_t)id) = make_int4(ch, ch + 1, ch + 2, ch + 3);
+        auto first_ge = [&](const KeyView &v, int64_t lo, int64_t hi, int d) {
+            while (lo < hi) {
+                const int64_t mid = (lo + hi) >> 1;
+                if (key_digit(v, mid, l + 1) < d) lo = mid + 1; else hi = mid;
+            }
+            return lo;
+        };
+        int64_t s0 = k, t0 = ta;
+        for (int j = 0; j < 4; j++) {
+            const int kb = ch + j;
+            const int64_t s1 = j == 3 ? kend : first_ge(kv, s0, kend, j + 1);
+            const int64_t t1 = j == 3 ? tb : first_ge(kt, t0, tb, j + 1);
+            cen[kb] = child_center(c, bs, j);
+            par[kb] = id;
+            lev[kb] = l + 1;
+            rs[kb] = make_int2((int)s0, (int)s1);
+            rt[kb] = make_int2((int)t0, (int)t1);
+            s0 = s1;
+            t0 = t1;
+        }
+    }
 }
 
 // Path keys of n points: nw words per point, word-major (word w of point i
@@ -253,39 +405,19 @@ struct Builder {
     // tree_refine_boxes and, with set_flags, tree_refine_boxes_flag, whose
     // children get flag 3 under a flag-1 parent and 0 otherwise.  `sel` is
     // evaluated before any array grows.
-    // known >= 0: the caller knows the number of refined boxes (no host
-    // synchronisation); the device's own count goes to *check, and no child
-    // is written beyond the capacity in case the two differ.
     template <class Sel>
     int refine_range(int lo, int hi, int newlevel, double bs, Sel sel,
-                     bool set_flags, int known = -1, int *check = nullptr) {
+                     bool set_flags) {
         const int n = hi - lo;
         if (n <= 0) return 0;
         DevBuf<int> f(n, s), off(n, s), tot(1, s);
         int *fp = f.get();
         for_each(n, s, [=] __device__(int64_t i) { fp[i] = sel(lo + (int)i) ? 1 : 0; });
-        exclusive_scan_i32(fp, off.get(), n, check ? check : tot.get(), s);
-        const int nref = known >= 0 ? known : read_scalar(tot.get(), s);
+        exclusive_scan_i32(fp, off.get(), n, tot.get(), s);
+        const int nref = read_scalar(tot.get(), s);
         if (nref == 0) return 0;
         ensure(T.nboxes + 4 * nref);
         const int cap = T.cap;
-        if (known >= 0) {
-            // a known count that was too large must leave no box unset: the
-            // ones no parent fills hang under the root (the check at the end
-            // of the build then rebuilds the tree)
-            const int nb0k = T.nboxes;
-            int *lev = T.level.get(), *par = T.parent.get(), *nch = T.nchild.get(),
-                *chi = T.child.get();
-            double2 *cenk = T.centers.get();
-            for_each(4 * (int64_t)nref, s, [=] __device__(int64_t i) {
-                const int kb = nb0k + (int)i;
-                cenk[kb] = cenk[0];
-                par[kb] = 0;
-                lev[kb] = newlevel;
-                nch[kb] = 0;
-                for (int l = 0; l < 4; l++) chi[4 * kb + l] = -1;
-            });
-        }
         const int nb0 = T.nboxes;
         double2 *cen = T.centers.get();
         int *lev = T.level.get(), *par = T.parent.get(), *nch = T.nchild.get();
@@ -296,7 +428,7 @@ struct Builder {
             if (!fp[i]) return;
             const int b = lo + (int)i;
             const int base = nb0 + 4 * op[i];
-            if (base + 4 > cap) return;  // (a known count that was wrong: caught by *check)
+            if (base + 4 > cap) return;
             const double2 c = cen[b];
             const int cf = (set_flags && flg[b] == 1) ? 3 : 0;
             nch[b] = 4;
@@ -830,6 +962,7 @@ struct Builder {
 struct KeyedPoints {
     DevBuf<uint32_t> idx;
     std::vector<DevBuf<uint32_t>> words;
+    DevBuf<uint32_t> prob;  // problem of every sorted position (forests)
     KeyView view() const {
         KeyView v{};
         for (size_t w = 0; w < words.size() && w < (size_t)kKeyWords; w++) v.w[w] = words[w].get();
@@ -886,6 +1019,7 @@ void key_sort(const double2 *pts, int n, double2 c0, const double *d_bsl, int ds
             for_each(n, s, [=] __device__(int64_t k) { o[k] = src[ip[k]]; });
         }
     }
+    if (prob && pbits > 0) kp.prob = std::move(key);
 }
 
 // Bounding box of sources and targets (pts_tree2d.c:493-513): exact min/max.
@@ -1086,180 +1220,165 @@ struct ForestRoots {
     int pbits = 0;
 };
 
-// Refinement without a host synchronisation per level: for one tree split
-// on the source counts (idivflag 0) the number of boxes refined on every
-// level follows from the sorted keys alone (refine_count_kernel), so the
-// levels are built with known counts, each level's own device count is
-// checked against them at the end, and a mismatch rebuilds the tree the
-// synchronous way.  FMM2D_B200_TREE_SYNC=1 always takes the synchronous way.
-bool presized_refinement(const ForestRoots *F, int idivflag) {
+// Trees split on their source counts (idivflag 0: every FMM call) take all
+// levels at once from the sorted keys (refine_runs_kernel,
+// build_boxes_kernel); the ndiv drivers' other rules, a negative ndiv (which
+// splits empty boxes too) and FMM2D_B200_TREE_SYNC=1 go level by level.
+bool levels_at_once(int idivflag, int ndiv) {
     const char *e = getenv("FMM2D_B200_TREE_SYNC");
-    return !F && idivflag == 0 && !(e && !strcmp(e, "1"));
+    return idivflag == 0 && ndiv >= 0 && !(e && !strcmp(e, "1"));
 }
 
 bool build_by_keys(const double2 *d_src, int ns, const double2 *d_targ, int nt, int ndiv,
                    int idivflag, int nlmax, double2 c0, int ds, cudaStream_t s, Tree &T,
-                   const ForestRoots *F = nullptr, bool sync_levels = false) {
+                   const ForestRoots *F = nullptr) {
     const double bs0 = T.boxsize[0];
     T = Tree();
     T.boxsize.push_back(bs0);
     Builder B(T, s);
     B.ranges = true;
-    std::vector<double> bsl(ds + 1);
+    std::vector<double> bsl(ds + 2);
     bsl[0] = bs0;
-    for (int l = 1; l <= ds; l++) bsl[l] = bsl[l - 1] / 2;
-    DevBuf<double> d_bsl(ds + 1, s);
+    for (int l = 1; l <= ds + 1; l++) bsl[l] = bsl[l - 1] / 2;
+    DevBuf<double> d_bsl(bsl.size(), s);
     FMM_CUDA(cudaMemcpyAsync(d_bsl.get(), bsl.data(), bsl.size() * sizeof(double),
                              cudaMemcpyHostToDevice, s));
     KeyedPoints ks, kt;
     const int nroots = F ? F->nroots : 1;
-    // presized form: the targets are sorted once the source keys have shown
-    // that ds digits suffice (a deeper tree retries with more digits)
-    const bool known = !sync_levels && presized_refinement(F, idivflag);
+    // all levels at once: the targets are sorted once the source keys have
+    // shown that ds digits suffice (a deeper tree retries with more digits)
+    const bool at_once = levels_at_once(idivflag, ndiv);
     auto sort_targets = [&]() {
         key_sort(d_targ, nt, c0, d_bsl.get(), ds, kt, s, F ? F->tprob : nullptr, F ? F->pbits : 0);
         B.kvt = kt.view();
     };
     key_sort(d_src, ns, c0, d_bsl.get(), ds, ks, s, F ? F->sprob : nullptr, F ? F->pbits : 0);
     B.kvs = ks.view();
-    if (!known) sort_targets();
-    B.ensure(std::max(1024, 4 * nroots));
+    RefineInfo R;
+    DevBuf<int> starts;
+    int nboxes = nroots;
+    if (at_once) {
+        // warps of at least 128 positions, at most 32 warps per SM
+        const int64_t chunk =
+            std::max<int64_t>(128, (((int64_t)ns + kNumSM * 32 - 1) / (kNumSM * 32) + 31) & ~31LL);
+        const int nwarp = (int)(((int64_t)ns + chunk - 1) / chunk);
+        const size_t ncnt = (size_t)(ds + 1) * nwarp;
+        DevBuf<int> cnt(ncnt, s), off(ncnt + 1, s);
+        const int nw = (ds + 15) / 16, blocks = (nwarp + 7) / 8;
+        refine_runs_kernel<true><<<blocks, 256, 0, s>>>(B.kvs, ks.prob.get(), ns, ndiv, ds, nw,
+                                                        chunk, nwarp, cnt.get(), nullptr);
+        FMM_CHECK_LAUNCH();
+        exclusive_scan_i32(cnt.get(), off.get(), (int64_t)ncnt, off.get() + ncnt, s);
+        DevBuf<int> lo(ds + 2, s);
+        {
+            int *lp = lo.get();
+            const int *op = off.get();
+            for_each(ds + 2, s, [=] __device__(int64_t l) { lp[l] = op[(size_t)l * nwarp]; });
+        }
+        std::vector<int> h(ds + 2);
+        read_small(h.data(), lo.get(), h.size() * sizeof(int), s);
+        // a box of the deepest digit level still to be split: more digits
+        if (ds < 64 && ds <= nlmax - 1 && h[ds + 1] > h[ds]) return false;
+        sort_targets();
+        R.nlev = 0;
+        R.off[0] = 0;
+        R.base[0] = 0;
+        T.lstart.push_back(0);
+        T.lend.push_back(nroots);
+        int64_t nb = nroots;
+        for (int l = 0; l < std::min(ds, nlmax) && h[l + 1] > h[l]; l++) {
+            R.nlev = l + 1;
+            R.off[l + 1] = h[l + 1];
+            R.base[l + 1] = (int)nb;
+            nb += 4 * (int64_t)(h[l + 1] - h[l]);
+            if (nb > INT32_MAX / 20) throw FmmError(4, "tree too large");
+            T.boxsize.push_back(T.boxsize[l] / 2);
+            T.lstart.push_back(R.base[l + 1]);
+            T.lend.push_back((int)nb);
+        }
+        nboxes = (int)nb;
+        const int tot = h[ds + 1];
+        starts.alloc(std::max(tot, 1), s);
+        if (tot > 0) {
+            refine_runs_kernel<false><<<blocks, 256, 0, s>>>(B.kvs, ks.prob.get(), ns, ndiv, ds,
+                                                             nw, chunk, nwarp, off.get(),
+                                                             starts.get());
+            FMM_CHECK_LAUNCH();
+        }
+    } else {
+        sort_targets();
+        T.lstart.push_back(0);
+        T.lend.push_back(nroots);
+    }
+    B.ensure(std::max(1024, std::max(4 * nroots, nboxes)));
     T.nboxes = nroots;
-    T.lstart.push_back(0);
-    T.lend.push_back(nroots);
     {
         double2 *cen = T.centers.get();
         int *lev = T.level.get(), *par = T.parent.get(), *nch = T.nchild.get(),
             *chi = T.child.get();
         int2 *r0 = B.rs.get(), *r1 = B.rt.get();
         const int *so = F ? F->d_soff : nullptr, *to = F ? F->d_toff : nullptr;
-        for_each(nroots, s, [=] __device__(int64_t i) {
+        // (boxes below the roots: no children yet; the others' are written
+        // by build_boxes_kernel or by the level that makes them)
+        for_each(nboxes, s, [=] __device__(int64_t i) {
             const int b = (int)i;
+            nch[b] = 0;
+            *reinterpret_cast<int4 *>(chi + 4 * (size_t)b) = make_int4(-1, -1, -1, -1);
+            if (b >= nroots) return;
             cen[b] = c0;
             lev[b] = 0;
             par[b] = -1;
-            nch[b] = 0;
-            for (int j = 0; j < 4; j++) chi[4 * b + j] = -1;
             r0[b] = so ? make_int2(so[b], so[b + 1]) : make_int2(0, ns);
             r1[b] = to ? make_int2(to[b], to[b + 1]) : make_int2(0, nt);
         });
     }
-    // known refinement counts per level (presized form): level 0 from the
-    // source count, levels 1..ds from the keys, one synchronisation
-    std::vector<unsigned long long> kc(65, 0);
-    DevBuf<int> chk(known ? nlmax + 1 : 0, s);
-    if (known) {
-        kc[0] = ns > ndiv ? 1 : 0;
-        if (ns > 0 && ds >= 1) {
-            DevBuf<unsigned long long> dc(65, s);
-            dc.zero(s);
-            const int nw = (ds + 15) / 16;
-            const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>(((int64_t)ns + 255) / 256, kNumSM * 8));
-            refine_count_kernel<<<blocks, 256, 0, s>>>(B.kvs, ns, ndiv, ds, nw, dc.get());
+    if (at_once) {
+        if (R.nlev > 0) {
+            const int tot = R.off[R.nlev], nw = (ds + 15) / 16;
+            build_boxes_kernel<<<std::min((tot + 127) / 128, kNumSM * 16), 128, 0, s>>>(
+                R, starts.get(), B.kvs, ks.prob.get(), ns, B.kvt, kt.prob.get(), nt, ndiv, nw, c0,
+                d_bsl.get(), T.centers.get(), T.level.get(), T.parent.get(), T.nchild.get(),
+                T.child.get(), B.rs.get(), B.rt.get());
             FMM_CHECK_LAUNCH();
-            read_small(kc.data() + 1, dc.get() + 1, 64 * sizeof(unsigned long long), s);
         }
-        // a box of the deepest digit level still to be split: more digits
-        if (ds < 64 && ds <= nlmax - 1 && kc[ds] > 0) return false;
-        sort_targets();
-        long long tot = nroots;
-        for (int l = 0; l < std::min(ds, nlmax); l++) {
-            if (kc[l] == 0) break;
-            tot += 4 * (long long)kc[l];
-        }
-        if (tot > (long long)INT32_MAX / 20) throw FmmError(4, "tree too large");
-        B.ensure((int)tot);
-        chk.zero(s);
-    }
-    DevBuf<int> nflag(1, s);
-    int ilev = 0;
-    for (ilev = 0; ilev <= nlmax - 1; ilev++) {
-        const int lo = T.lstart[ilev], hi = T.lend[ilev];
-        const int2 *ra = B.rs.get(), *rb = B.rt.get();
-        const int dflag = idivflag, nd = ndiv;
-        const bool last = ilev + 1 > ds;
-        if (known && last) break;  // (no box of level ds is split: checked above)
-        DevBuf<int> f(hi - lo, s);
-        int *fp = f.get();
-        if (known) {
-            // the capacity holds every level's known count; the new boxes
-            // are set to defaults in the selection's own launch, so a known
-            // count above the device's leaves no box unset (the ones no
-            // parent fills hang under the root, and the count check after
-            // the last level rebuilds the tree)
-            const int nref = (int)kc[ilev], n = hi - lo;
-            if (nref == 0) break;
+        T.nboxes = nboxes;
+        T.nlevels = R.nlev;
+    } else {
+        DevBuf<int> nflag(1, s);
+        int ilev = 0;
+        for (ilev = 0; ilev <= nlmax - 1; ilev++) {
+            const int lo = T.lstart[ilev], hi = T.lend[ilev];
+            const int2 *ra = B.rs.get(), *rb = B.rt.get();
+            const int dflag = idivflag, nd = ndiv;
+            const bool last = ilev + 1 > ds;
+            DevBuf<int> f(hi - lo, s);
+            int *fp = f.get();
+            int *nf = nflag.get();
+            if (last) nflag.zero(s);
+            for_each(hi - lo, s, [=] __device__(int64_t i) {
+                const int b = lo + (int)i;
+                const int nss = ra[b].y - ra[b].x, ntt = rb[b].y - rb[b].x;
+                const int nn = dflag == 0 ? nss : (dflag == 1 ? ntt : (nss > ntt ? nss : ntt));
+                fp[i] = nn > nd ? 1 : 0;
+                if (last && nn > nd) atomicAdd(nf, 1);
+            });
+            if (last) {
+                if (read_scalar(nf, s) > 0) return false;
+                break;
+            }
             T.boxsize.push_back(T.boxsize[ilev] / 2);
             const int nb0 = T.nboxes;
-            const int nset = std::max(n, 4 * nref);
-            DevBuf<int> off(n, s);
-            double2 *cen = T.centers.get();
-            int *lev = T.level.get(), *par = T.parent.get(), *nch = T.nchild.get(),
-                *chi = T.child.get();
-            const int newlevel = ilev + 1;
-            for_each(nset, s, [=] __device__(int64_t i) {
-                if (i < n) {
-                    const int b = lo + (int)i;
-                    const int nss = ra[b].y - ra[b].x, ntt = rb[b].y - rb[b].x;
-                    const int nn = dflag == 0 ? nss : (dflag == 1 ? ntt : (nss > ntt ? nss : ntt));
-                    fp[i] = nn > nd ? 1 : 0;
-                }
-                if (i < 4 * (int64_t)nref) {
-                    const int kb = nb0 + (int)i;
-                    cen[kb] = cen[0];
-                    par[kb] = 0;
-                    lev[kb] = newlevel;
-                    nch[kb] = 0;
-                    for (int l = 0; l < 4; l++) chi[4 * kb + l] = -1;
-                }
-            });
-            exclusive_scan_i32(fp, off.get(), n, chk.get() + ilev, s);
-            B.split_items(lo, n, 0, 0, fp, off.get(), nref, d_bsl.get(), false);
+            const int nref = B.refine_range(
+                lo, hi, ilev + 1, T.boxsize[ilev + 1],
+                [=] __device__(int b) { return fp[b - lo] != 0; }, false);
+            if (nref == 0) {
+                T.boxsize.pop_back();
+                break;
+            }
             T.lstart.push_back(nb0);
             T.lend.push_back(T.nboxes);
-            continue;
         }
-        int *nf = nflag.get();
-        if (last) nflag.zero(s);
-        for_each(hi - lo, s, [=] __device__(int64_t i) {
-            const int b = lo + (int)i;
-            const int nss = ra[b].y - ra[b].x, ntt = rb[b].y - rb[b].x;
-            const int nn = dflag == 0 ? nss : (dflag == 1 ? ntt : (nss > ntt ? nss : ntt));
-            fp[i] = nn > nd ? 1 : 0;
-            if (last && nn > nd) atomicAdd(nf, 1);
-        });
-        if (last) {
-            if (read_scalar(nf, s) > 0) return false;
-            break;
-        }
-        T.boxsize.push_back(T.boxsize[ilev] / 2);
-        const int nb0 = T.nboxes;
-        if (known && kc[ilev] == 0) {
-            T.boxsize.pop_back();
-            break;
-        }
-        const int nref = B.refine_range(
-            lo, hi, ilev + 1, T.boxsize[ilev + 1],
-            [=] __device__(int b) { return fp[b - lo] != 0; }, false,
-            known ? (int)kc[ilev] : -1, known ? chk.get() + ilev : nullptr);
-        if (nref == 0) {
-            T.boxsize.pop_back();
-            break;
-        }
-        T.lstart.push_back(nb0);
-        T.lend.push_back(T.nboxes);
-    }
-    T.nlevels = ilev;
-    if (known && ilev > 0) {
-        // every level's own count must equal the one the keys gave
-        std::vector<int> h(ilev);
-        read_small(h.data(), chk.get(), ilev * sizeof(int), s);
-        for (int l = 0; l < ilev; l++)
-            if ((unsigned long long)h[l] != kc[l]) {
-                T.boxsize.resize(1);
-                return build_by_keys(d_src, ns, d_targ, nt, ndiv, idivflag, nlmax, c0, ds, s, T, F,
-                                     true);
-            }
+        T.nlevels = ilev;
     }
     prof_mark("tree_refine", s);
     B.computecoll(0, T.nlevels);
