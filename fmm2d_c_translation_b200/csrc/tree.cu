@@ -14,6 +14,7 @@
 #include "tree.cuh"
 
 #include <algorithm>
+#include <cooperative_groups.h>
 #include <cstring>
 
 namespace fmm2d {
@@ -458,10 +459,9 @@ struct Builder {
     // per-level calls (a level range before its tail).  A child's level and
     // size follow from its parent's level (d_bsl: box size per level), so
     // the items may span several levels in box order.  Children get flag 3
-    // under a flag-1 parent and 0 otherwise (tree_refine_boxes_flag); with
-    // set_flags false the flags are left alone (tree_refine_boxes).
+    // under a flag-1 parent and 0 otherwise (tree_refine_boxes_flag).
     void split_items(int lo, int n1, int tlo, int n2, const int *fp, const int *op, int nref,
-                     const double *d_bsl, bool set_flags = true) {
+                     const double *d_bsl) {
         if (nref <= 0) return;
         ensure(T.nboxes + 4 * nref);
         const int nb0 = T.nboxes, cap = T.cap;
@@ -477,7 +477,7 @@ struct Builder {
             const double2 c = cen[b];
             const int nl = lev[b] + 1;
             const double bs = d_bsl[nl];
-            const int cf = set_flags && flg[b] == 1 ? 3 : 0;
+            const int cf = flg[b] == 1 ? 3 : 0;
             nch[b] = 4;
             for (int j = 0; j < 4; j++) {
                 const int kb = base + j;
@@ -487,13 +487,12 @@ struct Builder {
                 lev[kb] = nl;
                 for (int l = 0; l < 4; l++) chi[4 * kb + l] = -1;
                 chi[4 * b + j] = kb;
-                if (set_flags) flg[kb] = cf;
+                flg[kb] = cf;
                 if (cs) cs[kb] = 0;
                 if (ct) ct[kb] = 0;
             }
         });
         T.nboxes += 4 * nref;
-        set_child_ranges(nb0, T.nboxes);
     }
 
     std::vector<double> host_dist(int kind) const {
@@ -604,25 +603,14 @@ struct Builder {
         DevBuf<double2> cen2(T.cap, s);
         DevBuf<int> lev2(T.cap, s), par2(T.cap, s), nch2(T.cap, s),
             chi2((size_t)4 * T.cap, s), flg2(T.cap, s);
-        DevBuf<int2> rs2, rt2;
-        if (ranges) {
-            rs2.alloc(T.cap, s);
-            rt2.alloc(T.cap, s);
-        }
         const double2 *cen = T.centers.get();
         const int *par = T.parent.get(), *nch = T.nchild.get(),
                   *chi = T.child.get(), *flg = iflag.get();
-        const int2 *ra = rs.get(), *rb = rt.get();
         double2 *c2 = cen2.get();
         int *l2 = lev2.get(), *p2 = par2.get(), *n2 = nch2.get(),
             *h2 = chi2.get(), *f2 = flg2.get();
-        int2 *ra2 = rs2.get(), *rb2 = rt2.get();
         for_each(nb, s, [=] __device__(int64_t i) {
             const int b = (int)i, m = mp[b];
-            if (ra2) {
-                ra2[m] = ra[b];
-                rb2[m] = rb[b];
-            }
             c2[m] = cen[b];
             l2[m] = levp[b];
             n2[m] = nch[b];
@@ -639,10 +627,6 @@ struct Builder {
         T.nchild = std::move(nch2);
         T.child = std::move(chi2);
         iflag = std::move(flg2);
-        if (ranges) {
-            rs = std::move(rs2);
-            rt = std::move(rt2);
-        }
         for (int l = 2; l <= L; l++) {
             T.lstart[l] = nstart[l];
             T.lend[l] = nend[l];
@@ -664,7 +648,8 @@ struct Builder {
         return read_scalar(cp, s);
     }
 
-    // pts_tree_fix_lr (pts_tree2d.c:767-964).
+    // pts_tree_fix_lr (pts_tree2d.c:767-964), of the levelwise build (a key
+    // build's runs in one launch: tree_lr_kernel).
     void fix_lr() {
         const int L = T.nlevels;
         int *flg = iflag.get();
@@ -913,8 +898,10 @@ struct Builder {
     // reference's sorted arrays); inside every leaf the points go back to
     // input order.  `idx` maps key-sorted positions to input indices.
     // prob (forests): the problem, i.e. the root, of every input point.
+    // big: whether a leaf holds more than kLeafSort of these points.
     void finish_points(const uint32_t *idx, const KeyView &kv, int n, const DevBuf<int2> &R,
-                       DevBuf<int2> &se, DevBuf<int> &perm, const uint32_t *prob = nullptr) {
+                       DevBuf<int2> &se, DevBuf<int> &perm, bool big,
+                       const uint32_t *prob = nullptr) {
         const int nb = T.nboxes;
         se.alloc(nb, s);
         FMM_CUDA(cudaMemcpyAsync(se.get(), R.get(), (size_t)nb * sizeof(int2),
@@ -923,14 +910,7 @@ struct Builder {
         if (n == 0) return;
         const int *nch = T.nchild.get(), *chi = T.child.get();
         const int2 *rp = R.get();
-        DevBuf<int> big(1, s);
-        big.zero(s);
-        int *bp = big.get();
-        for_each(nb, s, [=] __device__(int64_t i) {
-            const int2 r = rp[i];
-            if (nch[i] == 0 && r.y - r.x > kLeafSort) atomicExch(bp, 1);
-        });
-        if (read_scalar(bp, s) == 0) {
+        if (!big) {
             const int blocks = std::max(1, std::min((nb + 7) / 8, kNumSM * 16));
             leaf_order_kernel<<<blocks, 256, 0, s>>>(nb, nch, rp, idx, perm.get());
             FMM_CHECK_LAUNCH();
@@ -956,6 +936,85 @@ struct Builder {
                                  cudaMemcpyDeviceToDevice, s));
     }
 };
+
+#include "tree_lr.cuh"
+
+// Colleagues and level restriction of a key-built tree (tree_lr_kernel);
+// returns its status and leaf flags.
+LrOut restrict_levels(Builder &B, const double *d_bsl, int nroots, cudaStream_t s) {
+    Tree &T = B.T;
+    const int L = T.nlevels;
+    LrArgs A;
+    DevBuf<double2> cen2(T.cap, s);
+    DevBuf<int> lev2(T.cap, s), par2(T.cap, s), nch2(T.cap, s), chi2((size_t)4 * T.cap, s),
+        flg2(T.cap, s);
+    DevBuf<int2> rs2(T.cap, s), rt2(T.cap, s);
+    A.a = LrSet{T.centers.get(), T.level.get(), T.parent.get(), T.nchild.get(), T.child.get(),
+                B.iflag.get(), B.rs.get(), B.rt.get()};
+    A.b = LrSet{cen2.get(), lev2.get(), par2.get(), nch2.get(), chi2.get(),
+                flg2.get(), rs2.get(), rt2.get()};
+    A.nnb = T.nnbors.get();
+    A.nb = T.nbors.get();
+    A.ks = B.kvs;
+    A.kt = B.kvt;
+    std::vector<double> hd;
+    for (int kind = 0; kind < 4; kind++) {
+        const std::vector<double> d = B.host_dist(kind);
+        hd.insert(hd.end(), d.begin(), d.end());
+    }
+    DevBuf<double> dd(hd.size(), s);
+    FMM_CUDA(cudaMemcpyAsync(dd.get(), hd.data(), hd.size() * sizeof(double),
+                             cudaMemcpyHostToDevice, s));
+    const int nd = L + 2;
+    A.dcol = dd.get();
+    A.d1 = A.dcol + nd;
+    A.d2 = A.d1 + nd;
+    A.d3 = A.d2 + nd;
+    A.bsl = d_bsl;
+    A.L = L;
+    A.nroots = nroots;
+    A.nboxes = T.nboxes;
+    A.cap = T.cap;
+    A.leaf_sort = kLeafSort;
+    for (int l = 0; l <= L; l++) {
+        A.lstart[l] = T.lstart[l];
+        A.lend[l] = T.lend[l];
+    }
+    constexpr int kOutInts = (int)(sizeof(LrOut) / sizeof(int));
+    DevBuf<int> w(kOutInts + 2 + kRefLevels + 2 * kLrBlocks, s);
+    FMM_CUDA(cudaMemsetAsync(w.get(), 0, (kOutInts + 2 + kRefLevels) * sizeof(int), s));
+    A.out = reinterpret_cast<LrOut *>(w.get());
+    A.any = w.get() + kOutInts;
+    A.levcnt = A.any + 2;
+    A.blkcnt = A.levcnt + kRefLevels;
+    int per_sm = 0;
+    FMM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tree_lr_kernel, kLrThreads, 0));
+    // (a block takes 32 boxes at a time with a warp per four)
+    const int blocks = std::max(1, std::min(std::min(kLrBlocks, per_sm * kNumSM), T.nboxes / 64));
+    void *args[] = {&A};
+    FMM_CUDA(cudaLaunchCooperativeKernel((const void *)tree_lr_kernel, dim3(blocks),
+                                         dim3(kLrThreads), args, 0, s));
+    FMM_CHECK_LAUNCH();
+    LrOut o;
+    read_small(&o, w.get(), sizeof(o), s);
+    if (o.status != 0) return o;
+    if (o.set == 1) {
+        T.centers = std::move(cen2);
+        T.level = std::move(lev2);
+        T.parent = std::move(par2);
+        T.nchild = std::move(nch2);
+        T.child = std::move(chi2);
+        B.iflag = std::move(flg2);
+        B.rs = std::move(rs2);
+        B.rt = std::move(rt2);
+    }
+    T.nboxes = o.nboxes;
+    for (int l = 0; l <= L; l++) {
+        T.lstart[l] = o.lstart[l];
+        T.lend[l] = o.lend[l];
+    }
+    return o;
+}
 
 // Key-sorted order of one point set: the input index of every sorted
 // position and the sorted key words.
@@ -1231,7 +1290,7 @@ bool levels_at_once(int idivflag, int ndiv) {
 
 bool build_by_keys(const double2 *d_src, int ns, const double2 *d_targ, int nt, int ndiv,
                    int idivflag, int nlmax, double2 c0, int ds, cudaStream_t s, Tree &T,
-                   const ForestRoots *F = nullptr) {
+                   const ForestRoots *F = nullptr, double room = 0.0) {
     const double bs0 = T.boxsize[0];
     T = Tree();
     T.boxsize.push_back(bs0);
@@ -1310,7 +1369,18 @@ bool build_by_keys(const double2 *d_src, int ns, const double2 *d_targ, int nt, 
         T.lstart.push_back(0);
         T.lend.push_back(nroots);
     }
-    B.ensure(std::max(1024, std::max(4 * nroots, nboxes)));
+    // with room for the boxes the level restriction adds: none on uniform
+    // points, a tenth on clusters, more than the first build's own number on
+    // curves (trees much deeper than uniform points would make)
+    int flat = 2;
+    for (int64_t q = std::max(ndiv, 1); q < std::max(ns, nt) && flat < nlmax; q *= 4) flat++;
+    auto with_room = [&](int n) {
+        const double f = std::max(room, T.boxsize.size() > (size_t)flat + 2 ? 2.0 : 0.5);
+        const double c = n + std::max(1024.0, f * n);
+        if (c > INT32_MAX / 20) throw FmmError(4, "tree too large");
+        return (int)c;
+    };
+    B.ensure(with_room(std::max(4 * nroots, nboxes)));
     T.nboxes = nroots;
     {
         double2 *cen = T.centers.get();
@@ -1381,11 +1451,18 @@ bool build_by_keys(const double2 *d_src, int ns, const double2 *d_targ, int nt, 
         T.nlevels = ilev;
     }
     prof_mark("tree_refine", s);
-    B.computecoll(0, T.nlevels);
-    if (T.nlevels >= 2) B.fix_lr();
+    B.ensure(with_room(T.nboxes));
+    const LrOut lr = restrict_levels(B, d_bsl.get(), nroots, s);
+    if (lr.status != 0) {
+        T.boxsize.resize(1);
+        return build_by_keys(d_src, ns, d_targ, nt, ndiv, idivflag, nlmax, c0, ds, s, T, F,
+                             std::max(4.0, 4.0 * room));
+    }
     prof_mark("tree_fixlr", s);
-    B.finish_points(ks.idx.get(), B.kvs, ns, B.rs, T.srcse, T.isrc, F ? F->sprob : nullptr);
-    B.finish_points(kt.idx.get(), B.kvt, nt, B.rt, T.trgse, T.itarg, F ? F->tprob : nullptr);
+    B.finish_points(ks.idx.get(), B.kvs, ns, B.rs, T.srcse, T.isrc, (lr.big & 1) != 0,
+                    F ? F->sprob : nullptr);
+    B.finish_points(kt.idx.get(), B.kvt, nt, B.rt, T.trgse, T.itarg, (lr.big & 2) != 0,
+                    F ? F->tprob : nullptr);
     prof_mark("tree_sort", s);
     return true;
 }
