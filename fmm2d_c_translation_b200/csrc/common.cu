@@ -14,22 +14,33 @@ std::mutex g_err_mu;
 std::string g_last_error;
 
 constexpr int kScanThreads = 256;
-constexpr int kScanItems = 4;
-constexpr int kScanTile = kScanThreads * kScanItems;  // 1024 values per block
+constexpr int kScanItems = 8;
+constexpr int kScanTile = kScanThreads * kScanItems;  // 2048 values per block
+constexpr int kScanSpin = 1 << 20;
+// tile states: a flag over the tile's own sum or its inclusive prefix
+constexpr unsigned long long kScanOwn = 1ull << 32, kScanIncl = 2ull << 32;
 
-// Block-local exclusive scan of one 1024-value tile; writes the tile total
-// to block_sums[blockIdx.x], and, for a scan of one tile, to *total (when
-// not null).
-__global__ void scan_tile_kernel(const int *__restrict__ in,
-                                 int *__restrict__ out, int64_t n,
-                                 int *__restrict__ block_sums, int *__restrict__ total) {
+// Exclusive scan in one launch: a tile publishes its sum, one warp looks
+// back over what the tiles before it published (decoupled look-back; the
+// tiles are numbered by a counter, so those have all begun), 32 at a time,
+// and the tile publishes its inclusive prefix.  A wait that lasts too long
+// ends with the warp summing the earlier values itself.  One tile needs no
+// state.  (Tile sums scanned recursively took three launches above 1,024
+// values, five above 10^6.)
+__global__ void __launch_bounds__(kScanThreads) scan_kernel(
+    const int *__restrict__ in, int *__restrict__ out, int64_t n, int *__restrict__ total,
+    volatile unsigned long long *state, int *__restrict__ next) {
     __shared__ int warp_tot[kScanThreads / 32];
-    const int64_t base = (int64_t)blockIdx.x * kScanTile + threadIdx.x * kScanItems;
+    __shared__ int s_tile, s_sum, s_before;
+    if (threadIdx.x == 0) s_tile = next ? atomicAdd(next, 1) : 0;
+    __syncthreads();
+    const int tile = s_tile;
+    const int64_t base = (int64_t)tile * kScanTile + threadIdx.x * kScanItems;
     int v[kScanItems];
     int tsum = 0;
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
-        int64_t idx = base + k;
+        const int64_t idx = base + k;
         v[k] = idx < n ? in[idx] : 0;
         tsum += v[k];
     }
@@ -50,46 +61,50 @@ __global__ void scan_tile_kernel(const int *__restrict__ in,
             int y = __shfl_up_sync(0xffffffffu, wi, d);
             if (lane >= d) wi += y;
         }
+        const int sum = __shfl_sync(0xffffffffu, wi, kScanThreads / 32 - 1);
         if (lane < kScanThreads / 32) warp_tot[lane] = wi - w;  // exclusive
-        if (lane == kScanThreads / 32 - 1) {
-            block_sums[blockIdx.x] = wi;
-            if (total && gridDim.x == 1) *total = wi;
+        int before = 0;
+        if (tile > 0) {
+            if (lane == 0) state[tile] = kScanOwn | (unsigned)sum;
+            int spins = 0;
+            for (int t = tile - 1; t >= 0;) {
+                // lane i holds tile t - i
+                unsigned long long st = kScanIncl;  // (nothing before the first)
+                if (t - lane >= 0) st = state[t - lane];
+                const unsigned have = __ballot_sync(0xffffffffu, st >= kScanOwn);
+                const unsigned inc = __ballot_sync(0xffffffffu, st >= kScanIncl);
+                // the tiles up to the first missing one or the first prefix
+                const int miss = have == 0xffffffffu ? 32 : __ffs(~have) - 1;
+                const int stop = inc ? __ffs(inc) : 33;  // tiles to take with it
+                const int take = min(miss, min(stop, 32));
+                const int add = lane < take ? (int)(unsigned)st : 0;
+                before += __reduce_add_sync(0xffffffffu, add);
+                if (stop <= miss) break;
+                t -= take;
+                if (take == 0 && ++spins > kScanSpin) {
+                    int sum2 = 0;
+                    for (int64_t i = lane; i < (int64_t)tile * kScanTile; i += 32) sum2 += in[i];
+                    before = __reduce_add_sync(0xffffffffu, sum2);
+                    break;
+                }
+            }
+        }
+        if (lane == 0) {
+            if (next) state[tile] = kScanIncl | (unsigned)(before + sum);
+            s_before = before;
+            s_sum = sum;
         }
     }
     __syncthreads();
-    int run = warp_tot[warp] + incl - tsum;
+    if (total && threadIdx.x == 0 && (int64_t)(tile + 1) * kScanTile >= n)
+        *total = s_before + s_sum;
+    int run = s_before + warp_tot[warp] + incl - tsum;
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
-        int64_t idx = base + k;
+        const int64_t idx = base + k;
         if (idx < n) out[idx] = run;
         run += v[k];
     }
-}
-
-__global__ void scan_add_kernel(int *__restrict__ out, int64_t n,
-                                const int *__restrict__ offs) {
-    const int64_t base = (int64_t)blockIdx.x * kScanTile;
-    const int add = offs[blockIdx.x];
-    for (int k = threadIdx.x; k < kScanTile; k += blockDim.x) {
-        int64_t idx = base + k;
-        if (idx < n) out[idx] += add;
-    }
-}
-
-// Exclusive scan; also leaves the inclusive grand total in *d_total_out
-// when requested.
-void scan_rec(const int *in, int *out, int64_t n, int *d_total,
-              cudaStream_t s) {
-    const int64_t nb = (n + kScanTile - 1) / kScanTile;
-    DevBuf<int> sums(nb + 1, s);
-    scan_tile_kernel<<<(unsigned)nb, kScanThreads, 0, s>>>(in, out, n, sums.get(),
-                                                           nb == 1 ? d_total : nullptr);
-    FMM_CHECK_LAUNCH();
-    if (nb == 1) return;
-    DevBuf<int> offs(nb, s);
-    scan_rec(sums.get(), offs.get(), nb, d_total, s);
-    scan_add_kernel<<<(unsigned)nb, kScanThreads, 0, s>>>(out, n, offs.get());
-    FMM_CHECK_LAUNCH();
 }
 }  // namespace
 
@@ -257,7 +272,16 @@ void exclusive_scan_i32(const int *in, int *out, int64_t n, int *d_total,
         if (d_total) FMM_CUDA(cudaMemsetAsync(d_total, 0, sizeof(int), s));
         return;
     }
-    scan_rec(in, out, n, d_total, s);
+    const int64_t nb = (n + kScanTile - 1) / kScanTile;
+    DevBuf<unsigned long long> state;
+    int *next = nullptr;
+    if (nb > 1) {
+        state.alloc(nb + 1, s);
+        state.zero(s);
+        next = reinterpret_cast<int *>(state.get() + nb);
+    }
+    scan_kernel<<<(unsigned)nb, kScanThreads, 0, s>>>(in, out, n, d_total, state.get(), next);
+    FMM_CHECK_LAUNCH();
 }
 
 }  // namespace fmm2d

@@ -1,147 +1,286 @@
 // sort.cu -- stable LSD radix sort of (uint32 key, uint32 value) pairs.
 //
-// Used by the tree builder: once to order the points by their path keys
-// (the child digits of every level, most significant first), and once to
-// put the points of every leaf back in input order, which is the stable
+// Used by the tree builder: to order the points by their path keys (the
+// child digits of every level, most significant first), and to put the
+// points of large leaves back in input order, which is the stable
 // permutation the reference's repeated partition
 // (c_translation/src/pts_tree2d.c:670-765) produces.
 //
-// One pass per 8-bit digit: a per-tile histogram, a scan of the digit-major
-// histogram table, and a scatter in which every tile first ranks its items
-// stably into shared memory (warp match for ties inside a warp, per-warp
-// counts across warps, a running per-digit count across rounds) and then
-// writes them out in digit order, so that consecutive threads write
-// consecutive addresses of the same digit run.
+// 8-bit digits.  One pass over the keys counts the digits of every pass;
+// then each pass reads and writes the pairs once: a tile counts its digits,
+// publishes the counts, finds the counts of the tiles before it by looking
+// back over what they published (Merrill and Garland's decoupled look-back),
+// ranks its items stably in shared memory (warp match for ties inside a
+// warp, per-warp counts across warps, a running per-digit count across
+// rounds) and writes them out in digit order, so that consecutive threads
+// write consecutive addresses of the same digit run.  Tiles take their
+// number from a counter, so the tiles before a running one have all begun;
+// a wait that lasts too long all the same ends with the thread counting the
+// earlier keys itself.  Up to one tile, all passes run in one block.
+//
+// Counting and scanning per pass instead (a histogram, three scan launches
+// and a scatter per digit) took 15 launches for the three digits of 10^5
+// points and read the keys twice per pass.  Keys and levels of the tree: 300
+// points 0.18 -> 0.11 ms, 10^5 0.24 -> 0.15, 4e5 clustered 0.77 -> 0.45,
+// 10^7 + 10^7 1.92 -> 1.74 ms.
 #include "common.cuh"
 #include "sort.cuh"
+
+#include <algorithm>
 
 namespace fmm2d {
 namespace {
 
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
-constexpr int kRounds = 16;
-constexpr int kTile = kThreads * kRounds;  // 4096 items per block
 constexpr int kRadix = 256;
+constexpr int kMaxPasses = 4;
+// tile states: 2 flag bits over a 30-bit count
+constexpr uint32_t kOwn = 1u << 30, kIncl = 2u << 30, kCount = kOwn - 1;
+constexpr int kMaxSpin = 1 << 20;
 
-__global__ void __launch_bounds__(kThreads) radix_hist_kernel(
-    const uint32_t *__restrict__ keys, int64_t n, int shift, int nblocks,
-    int *__restrict__ hist) {
-    __shared__ int h[kRadix];
-    h[threadIdx.x] = 0;
+// Digit counts of every pass.
+__global__ void __launch_bounds__(kThreads) radix_hist_kernel(const uint32_t *__restrict__ keys,
+                                                              int64_t n, int lo_bit, int passes,
+                                                              int *__restrict__ hist) {
+    __shared__ int h[kMaxPasses][kRadix];
+    for (int p = 0; p < passes; p++) h[p][threadIdx.x] = 0;
     __syncthreads();
-    const int64_t base = (int64_t)blockIdx.x * kTile;
-#pragma unroll 4
-    for (int r = 0; r < kRounds; r++) {
-        int64_t idx = base + (int64_t)r * kThreads + threadIdx.x;
-        if (idx < n) atomicAdd(&h[(keys[idx] >> shift) & 0xff], 1);
+    const int64_t stride = (int64_t)gridDim.x * kThreads;
+    for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < n; i += stride) {
+        const uint32_t k = keys[i] >> lo_bit;
+        for (int p = 0; p < passes; p++) atomicAdd(&h[p][(k >> (8 * p)) & 0xff], 1);
     }
     __syncthreads();
-    hist[threadIdx.x * nblocks + blockIdx.x] = h[threadIdx.x];
+    for (int p = 0; p < passes; p++)
+        if (h[p][threadIdx.x]) atomicAdd(&hist[p * kRadix + threadIdx.x], h[p][threadIdx.x]);
 }
 
-__global__ void __launch_bounds__(kThreads) radix_scatter_kernel(
-    const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vin,
-    uint32_t *__restrict__ kout, uint32_t *__restrict__ vout, int64_t n, int shift,
-    int nblocks, const int *__restrict__ hist, const int *__restrict__ offs) {
-    __shared__ uint32_t sk[kTile];
-    __shared__ uint32_t sv[kTile];
-    __shared__ int lstart[kRadix];  // tile-local start of each digit
-    __shared__ int gdelta[kRadix];  // global position - local position
-    __shared__ int run[kRadix];
-    __shared__ int wc[kWarps][kRadix];
-    __shared__ int wsum[kWarps];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // exclusive scan of this tile's digit counts
-    const int h = hist[tid * nblocks + blockIdx.x];
-    int incl = h;
+// Exclusive scan of one value per thread over the block.
+__device__ __forceinline__ int block_excl(int v, int *wsum) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int incl = v;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
         const int y = __shfl_up_sync(0xffffffffu, incl, d);
         if (lane >= d) incl += y;
     }
+    __syncthreads();
     if (lane == 31) wsum[warp] = incl;
     __syncthreads();
-    int wpre = 0;
-    for (int w = 0; w < warp; w++) wpre += wsum[w];
-    const int excl = wpre + incl - h;
-    lstart[tid] = excl;
-    gdelta[tid] = offs[tid * nblocks + blockIdx.x] - excl;
-    run[tid] = 0;
+    int pre = 0;
+    for (int w = 0; w < warp; w++) pre += wsum[w];
+    return pre + incl - v;
+}
+
+template <int ROUNDS>
+struct TileSmem {
+    uint32_t sk[kThreads * ROUNDS], sv[kThreads * ROUNDS];
+    int lstart[kRadix];  // tile-local start of each digit
+    int gdelta[kRadix];  // global position - local position
+    int run[kRadix];
+    int wc[kWarps][kRadix];
+    int wsum[kWarps];
+    int tile;
+};
+
+// Ranks the tile's items (kr, vr in round order) stably by the digit at
+// `shift` into S.sk, S.sv; S.lstart holds the digits' starts.
+template <int ROUNDS>
+__device__ __forceinline__ void rank_tile(TileSmem<ROUNDS> &S, const uint32_t *kr,
+                                          const uint32_t *vr, int cnt, int shift) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned lt_mask = (1u << lane) - 1u;
-    const int64_t base = (int64_t)blockIdx.x * kTile;
-    // the tile's items, loaded up front (coalesced, all in flight at once)
-    uint32_t kr[kRounds], vr[kRounds];
+    S.run[tid] = 0;
 #pragma unroll
-    for (int r = 0; r < kRounds; r++) {
-        const int64_t idx = base + (int64_t)r * kThreads + tid;
-        kr[r] = idx < n ? kin[idx] : 0u;
-        vr[r] = idx < n ? vin[idx] : 0u;
-    }
+    for (int r = 0; r < ROUNDS; r++) {
+        if (r * kThreads >= cnt) break;
 #pragma unroll
-    for (int r = 0; r < kRounds; r++) {
-#pragma unroll
-        for (int w = 0; w < kWarps; w++) wc[w][tid] = 0;
+        for (int w = 0; w < kWarps; w++) S.wc[w][tid] = 0;
         __syncthreads();
-        const int64_t idx = base + (int64_t)r * kThreads + tid;
-        const bool valid = idx < n;
-        const uint32_t key = kr[r], val = vr[r];
-        const int d = valid ? (int)((key >> shift) & 0xff) : -1;
+        const bool valid = r * kThreads + tid < cnt;
+        const int d = valid ? (int)((kr[r] >> shift) & 0xff) : -1;
         const unsigned peers = __match_any_sync(0xffffffffu, d);
         const int rank = __popc(peers & lt_mask);
-        if (valid && rank == 0) wc[warp][d] = __popc(peers);
+        if (valid && rank == 0) S.wc[warp][d] = __popc(peers);
         __syncthreads();
         if (valid) {
-            int pos = lstart[d] + run[d] + rank;
-            for (int w = 0; w < warp; w++) pos += wc[w][d];
-            sk[pos] = key;
-            sv[pos] = val;
+            int pos = S.lstart[d] + S.run[d] + rank;
+            for (int w = 0; w < warp; w++) pos += S.wc[w][d];
+            S.sk[pos] = kr[r];
+            S.sv[pos] = vr[r];
         }
         __syncthreads();
         int add = 0;
 #pragma unroll
-        for (int w = 0; w < kWarps; w++) add += wc[w][tid];
-        run[tid] += add;
+        for (int w = 0; w < kWarps; w++) add += S.wc[w][tid];
+        S.run[tid] += add;
     }
     __syncthreads();
+}
+
+// One pass over all tiles; vin null: the values are the positions.
+template <int ROUNDS>
+__global__ void __launch_bounds__(kThreads) radix_pass_kernel(
+    const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vin,
+    uint32_t *__restrict__ kout, uint32_t *__restrict__ vout, int64_t n, int shift,
+    const int *__restrict__ hist, int *__restrict__ next, volatile uint32_t *state) {
+    constexpr int kTile = kThreads * ROUNDS;
+    __shared__ TileSmem<ROUNDS> S;
+    const int tid = threadIdx.x;
+    if (tid == 0) S.tile = atomicAdd(next, 1);
+    S.run[tid] = 0;
+    __syncthreads();
+    const int tile = S.tile;
+    const int64_t base = (int64_t)tile * kTile;
     const int cnt = n - base < kTile ? (int)(n - base) : kTile;
+    uint32_t kr[ROUNDS], vr[ROUNDS];
+#pragma unroll
+    for (int r = 0; r < ROUNDS; r++) {
+        const int o = r * kThreads + tid;
+        kr[r] = o < cnt ? kin[base + o] : 0u;
+        vr[r] = o < cnt ? (vin ? vin[base + o] : (uint32_t)(base + o)) : 0u;
+    }
+#pragma unroll
+    for (int r = 0; r < ROUNDS; r++)
+        if (r * kThreads + tid < cnt) atomicAdd(&S.run[(kr[r] >> shift) & 0xff], 1);
+    __syncthreads();
+    const int own = S.run[tid];
+    volatile uint32_t *st = state + (size_t)tile * kRadix + tid;
+    *st = (tile == 0 ? kIncl : kOwn) | (uint32_t)own;
+    const int lst = block_excl(own, S.wsum);
+    const int gst = block_excl(hist[tid], S.wsum);  // the digit's first place
+    S.lstart[tid] = lst;
+    __syncthreads();
+    rank_tile<ROUNDS>(S, kr, vr, cnt, shift);
+    // the digit's items in the tiles before this one
+    uint32_t before = 0;
+    int spins = 0;
+    for (int t = tile - 1; t >= 0;) {
+        const uint32_t v = state[(size_t)t * kRadix + tid];
+        if (v >= kOwn) {
+            before += v & kCount;
+            if (v >= kIncl) break;
+            t--;
+        } else if (++spins > kMaxSpin) {
+            before = 0;
+            for (int64_t i = 0; i < base; i++) before += ((kin[i] >> shift) & 0xff) == (uint32_t)tid;
+            break;
+        }
+    }
+    if (tile > 0) *st = kIncl | (before + (uint32_t)own);
+    S.gdelta[tid] = gst + (int)before - lst;
+    __syncthreads();
     for (int i = tid; i < cnt; i += kThreads) {
-        const uint32_t key = sk[i];
-        const int64_t g = (int64_t)gdelta[(key >> shift) & 0xff] + i;
+        const uint32_t key = S.sk[i];
+        const int64_t g = (int64_t)S.gdelta[(key >> shift) & 0xff] + i;
         kout[g] = key;
-        vout[g] = sv[i];
+        vout[g] = S.sv[i];
+    }
+}
+
+// All passes of at most one tile in one block.
+constexpr int kOneRounds = 16;
+__global__ void __launch_bounds__(kThreads) radix_one_kernel(
+    const uint32_t *kin, const uint32_t *vin, uint32_t *kout, uint32_t *vout, int n, int lo_bit,
+    int key_bits) {
+    __shared__ TileSmem<kOneRounds> S;
+    const int tid = threadIdx.x;
+    uint32_t kr[kOneRounds], vr[kOneRounds];
+#pragma unroll
+    for (int r = 0; r < kOneRounds; r++) {
+        const int o = r * kThreads + tid;
+        kr[r] = o < n ? kin[o] : 0u;
+        vr[r] = o < n ? (vin ? vin[o] : (uint32_t)o) : 0u;
+    }
+    for (int shift = lo_bit; shift < key_bits; shift += 8) {
+        S.run[tid] = 0;
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kOneRounds; r++)
+            if (r * kThreads + tid < n) atomicAdd(&S.run[(kr[r] >> shift) & 0xff], 1);
+        __syncthreads();
+        const int lst = block_excl(S.run[tid], S.wsum);
+        S.lstart[tid] = lst;
+        __syncthreads();
+        rank_tile<kOneRounds>(S, kr, vr, n, shift);
+#pragma unroll
+        for (int r = 0; r < kOneRounds; r++) {
+            const int o = r * kThreads + tid;
+            if (o < n) {
+                kr[r] = S.sk[o];
+                vr[r] = S.sv[o];
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int r = 0; r < kOneRounds; r++) {
+        const int o = r * kThreads + tid;
+        if (o < n) {
+            kout[o] = kr[r];
+            vout[o] = vr[r];
+        }
+    }
+}
+
+template <int ROUNDS>
+void sort_passes(const uint32_t *kin, const uint32_t *vin, uint32_t *const k[2],
+                 uint32_t *const v[2], int64_t n, int lo_bit, int passes, cudaStream_t s) {
+    const int64_t tile = (int64_t)kThreads * ROUNDS;
+    const int ntiles = (int)((n + tile - 1) / tile);
+    // per pass: digit counts and the tile counter, then the tile states
+    const size_t head = (size_t)passes * (kRadix + 1), per = (size_t)ntiles * kRadix;
+    DevBuf<int> work(head + passes * per, s);
+    work.zero(s);
+    int *hist = work.get(), *next = hist + passes * kRadix;
+    uint32_t *state = reinterpret_cast<uint32_t *>(work.get()) + head;
+    const int blocks = (int)std::min<int64_t>((n + 2047) / 2048, kNumSM * 4);
+    radix_hist_kernel<<<blocks, kThreads, 0, s>>>(kin, n, lo_bit, passes, hist);
+    FMM_CHECK_LAUNCH();
+    for (int p = 0; p < passes; p++) {
+        radix_pass_kernel<ROUNDS><<<ntiles, kThreads, 0, s>>>(
+            p == 0 ? kin : k[(p - 1) & 1], p == 0 ? vin : v[(p - 1) & 1], k[p & 1], v[p & 1], n,
+            lo_bit + 8 * p, hist + p * kRadix, next + p, state + p * per);
+        FMM_CHECK_LAUNCH();
     }
 }
 
 }  // namespace
 
+int radix_sort_into(const uint32_t *kin, const uint32_t *vin, uint32_t *const k[2],
+                    uint32_t *const v[2], int64_t n, int key_bits, cudaStream_t s, int lo_bit) {
+    if (n <= 0) return 0;
+    if (n >= (int64_t)kOwn) throw FmmError(4, "sort: more than 2^30 items");
+    const int passes = std::max(1, (key_bits - lo_bit + 7) / 8);
+    if (passes > kMaxPasses) throw FmmError(4, "sort: more than 32 key bits");
+    if (n <= kThreads * kOneRounds) {
+        radix_one_kernel<<<1, kThreads, 0, s>>>(kin, vin, k[0], v[0], (int)n, lo_bit, key_bits);
+        FMM_CHECK_LAUNCH();
+        return 0;
+    }
+    // tiles of 1,024 items while larger ones would leave SMs without one
+    if (n < (int64_t)kThreads * 16 * kNumSM)
+        sort_passes<4>(kin, vin, k, v, n, lo_bit, passes, s);
+    else
+        sort_passes<16>(kin, vin, k, v, n, lo_bit, passes, s);
+    return (passes - 1) & 1;
+}
+
 void radix_sort_pairs(uint32_t *keys, uint32_t *vals, uint32_t *keys_tmp,
                       uint32_t *vals_tmp, int64_t n, int key_bits,
                       cudaStream_t s, int lo_bit) {
     if (n <= 1 || key_bits <= lo_bit) return;
-    const int nblocks = (int)((n + kTile - 1) / kTile);
-    DevBuf<int> hist((size_t)kRadix * nblocks, s);
-    DevBuf<int> offs((size_t)kRadix * nblocks, s);
-    uint32_t *ka = keys, *va = vals, *kb = keys_tmp, *vb = vals_tmp;
-    int passes = 0;
-    for (int shift = lo_bit; shift < key_bits; shift += 8) {
-        radix_hist_kernel<<<nblocks, kThreads, 0, s>>>(ka, n, shift, nblocks,
-                                                       hist.get());
+    if (n <= kThreads * kOneRounds) {
+        // (one block reads everything before it writes)
+        radix_one_kernel<<<1, kThreads, 0, s>>>(keys, vals, keys, vals, (int)n, lo_bit, key_bits);
         FMM_CHECK_LAUNCH();
-        exclusive_scan_i32(hist.get(), offs.get(), (int64_t)kRadix * nblocks,
-                           nullptr, s);
-        radix_scatter_kernel<<<nblocks, kThreads, 0, s>>>(
-            ka, va, kb, vb, n, shift, nblocks, hist.get(), offs.get());
-        FMM_CHECK_LAUNCH();
-        std::swap(ka, kb);
-        std::swap(va, vb);
-        passes++;
+        return;
     }
-    if (passes & 1) {
-        FMM_CUDA(cudaMemcpyAsync(keys, ka, n * sizeof(uint32_t),
-                                 cudaMemcpyDeviceToDevice, s));
-        FMM_CUDA(cudaMemcpyAsync(vals, va, n * sizeof(uint32_t),
-                                 cudaMemcpyDeviceToDevice, s));
+    uint32_t *const k[2] = {keys_tmp, keys}, *const v[2] = {vals_tmp, vals};
+    if (radix_sort_into(keys, vals, k, v, n, key_bits, s, lo_bit) == 0) {
+        FMM_CUDA(cudaMemcpyAsync(keys, keys_tmp, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
+        FMM_CUDA(cudaMemcpyAsync(vals, vals_tmp, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
     }
 }
 

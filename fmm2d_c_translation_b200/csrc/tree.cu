@@ -1045,40 +1045,51 @@ void key_sort(const double2 *pts, int n, double2 c0, const double *d_bsl, int ds
         path_key_kernel<<<blocks, 256, 0, s>>>(pts, n, c0, d_bsl, ds, nw, raw.get());
         FMM_CHECK_LAUNCH();
     }
-    kp.idx.alloc(n, s);
-    uint32_t *ip = kp.idx.get();
-    for_each(n, s, [=] __device__(int64_t i) { ip[i] = (uint32_t)i; });
-    DevBuf<uint32_t> key(n, s), kt(n, s), vt(n, s);
-    uint32_t *kp0 = key.get();
+    DevBuf<uint32_t> kb[2], vb[2], kin;
+    for (int r = 0; r < 2; r++) {
+        kb[r].alloc(n, s);
+        vb[r].alloc(n, s);
+    }
+    int r = 0;  // the sorted keys and indices are kb[r], vb[r]
+    auto sort_by = [&](const uint32_t *key, bool first, int bits, int lo) {
+        uint32_t *const ko[2] = {kb[0].get(), kb[1].get()};
+        uint32_t *const vo[2] = {vb[1 - r].get(), vb[r].get()};
+        const int o = radix_sort_into(key, first ? nullptr : vb[r].get(), ko, vo, n, bits, s, lo);
+        if (o == 0) r = 1 - r;
+        if (o != r) std::swap(kb[0], kb[1]);  // (keys and indices under one number)
+    };
     const uint32_t *rw = raw.get();
+    // the words in the sorted order so far
+    auto in_order = [&](const uint32_t *src, uint32_t *dst) {
+        const uint32_t *ip = vb[r].get();
+        for_each(n, s, [=] __device__(int64_t k) { dst[k] = src[ip[k]]; });
+    };
     // least significant word first; only the bits of levels <= ds
     for (int w = nw - 1; w >= 0; w--) {
         const uint32_t *src = rw + (size_t)w * n;
-        if (w == nw - 1)
-            FMM_CUDA(cudaMemcpyAsync(kp0, src, (size_t)n * sizeof(uint32_t),
-                                     cudaMemcpyDeviceToDevice, s));
-        else
-            for_each(n, s, [=] __device__(int64_t k) { kp0[k] = src[ip[k]]; });
+        const bool first = w == nw - 1;
+        if (!first) {
+            if (!kin.get()) kin.alloc(n, s);
+            in_order(src, kin.get());
+        }
         const int used = 2 * std::min(16, ds - 16 * w);
         const int lo = (32 - used) & ~7;
-        radix_sort_pairs(kp0, ip, kt.get(), vt.get(), n, 32, s, lo);
+        sort_by(first ? src : kin.get(), first, 32, lo);
     }
-    if (prob && pbits > 0) {
-        for_each(n, s, [=] __device__(int64_t k) { kp0[k] = prob[ip[k]]; });
-        radix_sort_pairs(kp0, ip, kt.get(), vt.get(), n, pbits, s);
+    const bool forest = prob && pbits > 0;
+    if (forest) {
+        if (!kin.get()) kin.alloc(n, s);
+        in_order(prob, kin.get());
+        sort_by(kin.get(), false, pbits, 0);
     }
     for (int w = 0; w < nw; w++) {
+        if (w == 0 && !forest) continue;
         kp.words[w].alloc(n, s);
-        uint32_t *o = kp.words[w].get();
-        if (w == 0 && !(prob && pbits > 0)) {
-            FMM_CUDA(cudaMemcpyAsync(o, kp0, (size_t)n * sizeof(uint32_t),
-                                     cudaMemcpyDeviceToDevice, s));
-        } else {
-            const uint32_t *src = rw + (size_t)w * n;
-            for_each(n, s, [=] __device__(int64_t k) { o[k] = src[ip[k]]; });
-        }
+        in_order(rw + (size_t)w * n, kp.words[w].get());
     }
-    if (prob && pbits > 0) kp.prob = std::move(key);
+    if (forest) kp.prob = std::move(kb[r]);
+    else kp.words[0] = std::move(kb[r]);
+    kp.idx = std::move(vb[r]);
 }
 
 // Bounding box of sources and targets (pts_tree2d.c:493-513): exact min/max.
