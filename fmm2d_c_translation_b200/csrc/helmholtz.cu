@@ -1769,8 +1769,13 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
     // mixed mode: levels of order <= 23 on the tensor cores (tiles of
     // 128 / nd target boxes)
     SlotPlan spl_tc;
-    const bool tc = P.mixed && nd <= 128 && helm_m2l_tc_enabled() &&
-                    plan_slots(T, sp, tp, 128 / nd, s, spl_tc);
+    bool tc = P.mixed && nd <= 128 && helm_m2l_tc_enabled();
+    if (tc && tiled) {
+        spl_tc = spl;
+        if (spl.ntarg > 0) retile_slots(spl_tc, 128 / nd);
+    } else if (tc) {
+        tc = plan_slots(T, sp, tp, 128 / nd, s, spl_tc);
+    }
     DevBuf<int> tc_err(tc ? 1 : 0, s);
     if (tc) FMM_CUDA(cudaMemsetAsync(tc_err.get(), 0, sizeof(int), s));
     bool tc_used = false;

@@ -167,6 +167,8 @@ struct SlotPlan {
     int nseg = 0, ntarg = 0, ntiles = 0;
 };
 bool plan_slots(const Tree &T, int spgh, int tpgh, int tile, cudaStream_t s, SlotPlan &sp);
+// The same plan cut into tiles of another size.
+void retile_slots(SlotPlan &sp, int tile);
 
 // Slot GEMMs of one level on the tensor cores (helm_m2l_tc.cu): for every
 // plan row q of the level's four segments (child positions cp) and every

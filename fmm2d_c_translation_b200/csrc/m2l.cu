@@ -21,7 +21,6 @@
 // list 2.  If any list-2 entry falls outside the 27 slots (not expected of
 // the reference's trees) the caller falls back to the per-box kernel.
 #include "laplace.cuh"
-#include "sort.cuh"
 #include "tc_common.cuh"
 
 #include <algorithm>
@@ -254,15 +253,26 @@ void launch_dmma(const SegTable &sg, const int *boxes, const int *slots,
 
 
 // The tiles of one M2L evaluation: target boxes of levels >= 2 that hold
-// points, sorted by (level, child position) = segment, and the source box of
-// every (target, slot).
+// points, grouped by (level, child position) = segment in box order, the
+// source box of every (target, slot), and the segment tables for one or more
+// tile sizes.
 struct M2LWork {
-    DevBuf<uint32_t> keys, vals, kt, vt;
-    DevBuf<int> segd, slots;
-    std::vector<int> hseg;  // host copy of segd
-    int nseg = 0, ntarg = 0, ntiles = 0;
-    SegTable seg() const {
+    DevBuf<int> boxes, slots, segd;
+    struct Tab {
+        int tile, off, ntiles;  // tile size, offset of its table in segd
+    };
+    std::vector<Tab> tabs;
+    std::vector<int> start, count;  // per segment
+    int nseg = 0, ntarg = 0;
+    int ntiles(int tile) const {
+        for (const Tab &t : tabs)
+            if (t.tile == tile) return t.ntiles;
+        return 0;
+    }
+    SegTable seg(int tile) const {
         const int *h = segd.get();
+        for (const Tab &t : tabs)
+            if (t.tile == tile) h += t.off;
         return SegTable{h, h + nseg + 1, h + 2 * nseg + 1, h + 3 * nseg + 1, h + 4 * nseg + 1,
                         nseg};
     }
@@ -289,110 +299,132 @@ void ensure_slot_tables(cudaStream_t s) {
     }
 }
 
-// Builds the segments (tiles of `tile` boxes) and the slot table, leaving
-// out the target levels set in skip_levels; false when a list-2 entry
-// falls outside the 27 slots or there are too many segments.
-bool m2l_work(const Tree &T, const CauchyProblem &P, int tile, cudaStream_t s, M2LWork &w,
-              uint64_t skip_levels = 0) {
+// Tile bases of the segments for tiles of `tile` boxes.
+std::vector<int> tile_bases(const std::vector<int> &count, int tile) {
+    std::vector<int> tb(count.size() + 1, 0);
+    for (size_t k = 0; k < count.size(); k++) tb[k + 1] = tb[k] + (count[k] + tile - 1) / tile;
+    return tb;
+}
+
+// Place of every box of levels >= 2 in segment order: level by level, the
+// boxes that are child 0 of their parent first, then child 1, ...  (Boxes
+// come in groups of four siblings, in child order, on every level.)
+struct SegOrder {
+    int start[kMaxLevels + 2];
+    __device__ __forceinline__ int at(int b, int l) const {
+        const int m = b - start[l], n4 = (start[l + 1] - start[l]) >> 2;
+        return start[l] - start[2] + (m & 3) * n4 + (m >> 2);
+    }
+};
+
+// Builds the segments, the slot table and the segment tables for the given
+// tile sizes, leaving out the target levels set in skip_levels; false when a
+// list-2 entry falls outside the 27 slots or there are too many segments.
+// The boxes of a segment are placed by one prefix sum over flags kept in
+// segment order, and the host reads the segments' ends and the check in one
+// synchronisation.  (Sorting the boxes by segment, once per tile size, took
+// 0.1 ms and two synchronisations each at any size.)
+bool m2l_work(const Tree &T, const CauchyProblem &P, const std::vector<int> &tiles,
+              cudaStream_t s, M2LWork &w, uint64_t skip_levels = 0) {
     const int L = T.nlevels;
     ensure_slot_tables(s);
     const int lo = T.lstart[2], n = T.nboxes - lo;
     const int nseg = 4 * (L - 1);
     w.nseg = nseg;
+    w.start.assign(nseg, 0);
+    w.count.assign(nseg, 0);
+    if (nseg + 1 > 257) return false;
+    SegOrder so;
+    int most = 0;  // boxes of the levels that are not left out
+    for (int l = 0; l <= L; l++) {
+        so.start[l] = T.lstart[l];
+        if (l >= 2 && !((skip_levels >> l) & 1ull)) most += T.lend[l] - T.lstart[l];
+    }
+    so.start[L + 1] = T.nboxes;
+    if (most == 0) return true;
     const int2 *sse = T.srcse.get(), *tse = T.trgse.get();
     const int spgh = P.sset.pgh, tpgh = P.tset.pgh;
-    const int *lev = T.level.get(), *par = T.parent.get(), *chi = T.child.get();
-    // ---- keys: (level - 2) * 4 + child position, or nseg when not a target
-    w.keys.alloc(n, s);
-    w.vals.alloc(n, s);
-    w.kt.alloc(n, s);
-    w.vt.alloc(n, s);
-    DevBuf<int> cnt(nseg + 1, s);
-    cnt.zero(s);
-    uint32_t *kp = w.keys.get(), *vp = w.vals.get();
-    int *cp = cnt.get();
+    const int *lev = T.level.get();
+    DevBuf<int> flag(n, s), pos(n + 1, s), ends(nseg + 2, s), err(1, s);
+    err.zero(s);
+    w.boxes.alloc(most, s);
+    w.slots.alloc((size_t)most * kSlots, s);
+    int *fp = flag.get(), *pp = pos.get(), *ep = err.get(), *en = ends.get();
     for_each(n, s, [=] __device__(int64_t i) {
-        const int b = lo + (int)i;
+        const int b = lo + (int)i, l = lev[b];
         int np = 0;
         if (tpgh > 0) np += tse[b].y - tse[b].x;
         if (spgh > 0) np += sse[b].y - sse[b].x;
-        int key = nseg;
-        if (np > 0 && !((skip_levels >> lev[b]) & 1ull)) {
-            const int pb = par[b];
-            int c = 0;
-            for (int j = 0; j < 4; j++)
-                if (chi[4 * pb + j] == b) c = j;
-            key = (lev[b] - 2) * 4 + c;
-        }
-        kp[i] = (uint32_t)key;
-        vp[i] = (uint32_t)b;
-        // one atomic per group of lanes with the same segment
-        const unsigned am = __activemask();
-        const unsigned peers = __match_any_sync(am, key);
-        if (key < nseg && (int)(threadIdx.x & 31) == __ffs(peers) - 1)
-            atomicAdd(&cp[key], __popc(peers));
+        fp[so.at(b, l)] = np > 0 && !((skip_levels >> l) & 1ull) ? 1 : 0;
     });
-    int bits = 1;
-    while ((1 << bits) <= nseg) bits++;
-    radix_sort_pairs(kp, vp, w.kt.get(), w.vt.get(), n, bits, s);
-    std::vector<int> hc(nseg + 1);
-    read_small(hc.data(), cp, (nseg + 1) * sizeof(int), s);
-    std::vector<int> h(5 * nseg + 1);
-    int *tb = h.data(), *st = tb + nseg + 1, *ct = st + nseg, *lv = ct + nseg, *cpv = lv + nseg;
-    int run = 0, start = 0;
-    for (int k = 0; k < nseg; k++) {
-        tb[k] = run;
-        st[k] = start;
-        ct[k] = hc[k];
-        lv[k] = 2 + k / 4;
-        cpv[k] = k % 4;
-        run += (hc[k] + tile - 1) / tile;
-        start += hc[k];
-    }
-    tb[nseg] = run;
-    w.ntiles = run;
-    w.ntarg = start;
-    w.hseg = h;
-    if (w.ntiles == 0) return true;
-    if (nseg + 1 > 257) return false;
-    w.segd.alloc(h.size(), s);
-    FMM_CUDA(cudaMemcpyAsync(w.segd.get(), h.data(), h.size() * sizeof(int), cudaMemcpyHostToDevice, s));
-    // ---- the source box of every (target, slot), from list 2
-    const int ntarg = w.ntarg;
-    w.slots.alloc((size_t)ntarg * kSlots, s);
-    DevBuf<int> err(1, s);
-    FMM_CUDA(cudaMemsetAsync(w.slots.get(), 0xff, (size_t)ntarg * kSlots * sizeof(int), s));
-    err.zero(s);
+    exclusive_scan_i32(fp, pp, n, pp + n, s);
+    // ---- the targets and the source box of every (target, slot), from list 2
     {
-        int *sl = w.slots.get(), *ep = err.get();
+        int *bx = w.boxes.get(), *sl = w.slots.get();
         const int *n2 = T.nlist2.get(), *l2 = T.list2.get();
         const double2 *cen = T.centers.get();
         const double *bsd = T.d_boxsize.get();
-        const uint32_t *bx = vp;
-        for_each(ntarg, s, [=] __device__(int64_t q) {
-            const int b = (int)bx[q];
-            const int pb = par[b];
-            int c = 0;
-            for (int j = 0; j < 4; j++)
-                if (chi[4 * pb + j] == b) c = j;
-            const double r = bsd[lev[b]];
+        for_each(n, s, [=] __device__(int64_t i) {
+            const int b = lo + (int)i, l = lev[b], f = so.at(b, l);
+            if (!fp[f]) return;
+            const int q = pp[f], c = (b - so.start[l]) & 3;
+            bx[q] = b;
+            int *row = sl + (size_t)q * kSlots;
+            const double ri = 1.0 / bsd[l];
             const double2 cb = cen[b];
-            for (int e = 0; e < n2[b]; e++) {
+            unsigned have = 0;
+            const int m = n2[b];
+            for (int e = 0; e < m; e++) {
                 const int sb = l2[kMaxList2 * b + e];
                 if (sse[sb].y <= sse[sb].x) continue;  // no multipole
                 const double2 cs = cen[sb];
-                const int dx = (int)rint((cs.x - cb.x) / r), dy = (int)rint((cs.y - cb.y) / r);
+                const int dx = (int)rint((cs.x - cb.x) * ri), dy = (int)rint((cs.y - cb.y) * ri);
                 const int k = (dx >= -3 && dx <= 3 && dy >= -3 && dy <= 3)
                                   ? c_slot_of[c][dx + 3][dy + 3] : -1;
                 if (k < 0) {
                     atomicExch(ep, 1);
                     continue;
                 }
-                sl[q * kSlots + k] = sb;
+                have |= 1u << k;
+                row[k] = sb;
             }
+            for (int k = 0; k < kSlots; k++)
+                if (!((have >> k) & 1u)) row[k] = -1;
         });
     }
-    return read_scalar(err.get(), s) == 0;
+    for_each(nseg + 2, s, [=] __device__(int64_t k) {
+        if (k == nseg + 1) {
+            en[k] = *ep;
+        } else if (k == nseg) {
+            en[k] = pp[n];
+        } else {
+            const int l = 2 + (int)k / 4, c = (int)k & 3;
+            en[k] = pp[so.start[l] - lo + c * ((so.start[l + 1] - so.start[l]) >> 2)];
+        }
+    });
+    std::vector<int> h(nseg + 2);
+    read_small(h.data(), en, h.size() * sizeof(int), s);
+    if (h[nseg + 1] != 0) return false;
+    for (int k = 0; k < nseg; k++) {
+        w.start[k] = h[k];
+        w.count[k] = h[k + 1] - h[k];
+    }
+    w.ntarg = h[nseg];
+    if (w.ntarg == 0) return true;
+    std::vector<int> all;
+    for (int tile : tiles) {
+        const std::vector<int> tb = tile_bases(w.count, tile);
+        w.tabs.push_back({tile, (int)all.size(), tb[nseg]});
+        all.insert(all.end(), tb.begin(), tb.end());
+        all.insert(all.end(), w.start.begin(), w.start.end());
+        all.insert(all.end(), w.count.begin(), w.count.end());
+        for (int k = 0; k < nseg; k++) all.push_back(2 + k / 4);
+        for (int k = 0; k < nseg; k++) all.push_back(k % 4);
+    }
+    w.segd.alloc(all.size(), s);
+    FMM_CUDA(cudaMemcpyAsync(w.segd.get(), all.data(), all.size() * sizeof(int),
+                             cudaMemcpyHostToDevice, s));
+    return true;
 }
 
 // ---------------------------------------------------------------------------
@@ -407,17 +439,14 @@ bool m2l_work(const Tree &T, const CauchyProblem &P, int tile, cudaStream_t s, M
 // the P1 x CH accumulators in registers (FP32 arithmetic, FP32
 // accumulation over the 27 slots, stored as FP64).
 // ---------------------------------------------------------------------------
-// NR < P1: only the rows i < NR (the leading local coefficients) are
-// computed and stored; the tensor-core forms use this to recompute the rows
-// that carry most of the gradient in FP32 (see the end of m2l_fp32).
 constexpr int kFp32Tile = 128;
 
-template <int P1, int CH, int NR = P1>
+template <int P1, int CH>
 __global__ void __launch_bounds__(kFp32Tile) m2l_fp32_kernel(
     SegTable seg, const int *__restrict__ boxes, const int *__restrict__ slots,
     const double *__restrict__ bs, int ndc, int c0, int p, const float2 *__restrict__ Tall,
     const float2 *__restrict__ mp32, double2 *__restrict__ loc, int ntiles) {
-    __shared__ float2 sT[NR * P1];
+    __shared__ float2 sT[P1 * P1];
     __shared__ int s_tb[257];
     for (int e = threadIdx.x; e <= seg.nseg && e < 257; e += blockDim.x) s_tb[e] = seg.tile_base[e];
     __syncthreads();
@@ -433,18 +462,18 @@ __global__ void __launch_bounds__(kFp32Tile) m2l_fp32_kernel(
         const bool valid = q < seg.start[sg] + seg.count[sg];
         const int cp = seg.cpos[sg];
         const float lr = (float)log(bs[seg.level[sg]]);
-        float2 acc[CH][NR];
+        float2 acc[CH][P1];
         float2 s0[CH];
 #pragma unroll
         for (int c = 0; c < CH; c++) {
             s0[c] = make_float2(0.f, 0.f);
 #pragma unroll
-            for (int i = 0; i < NR; i++) acc[c][i] = make_float2(0.f, 0.f);
+            for (int i = 0; i < P1; i++) acc[c][i] = make_float2(0.f, 0.f);
         }
         for (int k = 0; k < kSlots; k++) {
             __syncthreads();  // the previous slot's matrix is no longer read
             const float2 *Tk = Tall + ((size_t)cp * kSlots + k) * P1 * P1;
-            for (int e = threadIdx.x; e < NR * P1; e += blockDim.x) sT[e] = Tk[e];
+            for (int e = threadIdx.x; e < P1 * P1; e += blockDim.x) sT[e] = Tk[e];
             __syncthreads();
             const int sb = valid ? slots[(size_t)q * kSlots + k] : -1;
             if (sb < 0) continue;
@@ -463,7 +492,7 @@ __global__ void __launch_bounds__(kFp32Tile) m2l_fp32_kernel(
                     }
                 }
 #pragma unroll
-                for (int i = 0; i < NR; i++) {
+                for (int i = 0; i < P1; i++) {
                     const float2 t = sT[i * P1 + j];
 #pragma unroll
                     for (int c = 0; c < CH; c++) {
@@ -481,13 +510,93 @@ __global__ void __launch_bounds__(kFp32Tile) m2l_fp32_kernel(
                 acc[c][0].y += lr * s0[c].y;
             }
 #pragma unroll
-            for (int i = 0; i < NR; i++) {
+            for (int i = 0; i < P1; i++) {
                 if (i > p) break;
 #pragma unroll
                 for (int c = 0; c < CH; c++)
                     loc[(size_t)b * stride + (size_t)i * ndc + c0 + c] =
                         make_double2((double)acc[c][i].x, (double)acc[c][i].y);
             }
+        }
+    }
+}
+
+// The leading NR rows (local coefficients) of the same sums, which the
+// tensor-core forms recompute in FP32 (see the end of m2l_fp32): one thread
+// per (box, row), so the 27 slots' matrices of the rows fit into shared
+// memory at once and a thread's chain is its row's terms alone; every
+// accumulator adds the same terms in the same order as m2l_fp32_kernel's.
+// Bound by the latency of the source rows' loads.  (With a thread per box and
+// the matrices staged slot by slot, a tile took 79 us whatever it held.)
+constexpr int kRowsTile = 32;
+
+template <int P1, int CH, int NR>
+__global__ void __launch_bounds__(kRowsTile * NR) m2l_rows_kernel(
+    SegTable seg, const int *__restrict__ boxes, const int *__restrict__ slots,
+    const double *__restrict__ bs, int ndc, int c0, int p, const float2 *__restrict__ Tall,
+    const float2 *__restrict__ mp32, double2 *__restrict__ loc, int ntiles) {
+    __shared__ __align__(16) float2 sT[kSlots * NR * P1];
+    __shared__ int s_tb[257];
+    for (int e = threadIdx.x; e <= seg.nseg && e < 257; e += blockDim.x) s_tb[e] = seg.tile_base[e];
+    const int stride = (p + 1) * ndc;
+    const int row = threadIdx.x % NR, bx = threadIdx.x / NR;
+    int cp_in = -1;
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        __syncthreads();
+        int lo = 0, hi = seg.nseg;
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (s_tb[mid] <= tile) lo = mid; else hi = mid;
+        }
+        const int cp = seg.cpos[lo];
+        if (cp != cp_in) {
+            const float2 *Tc = Tall + (size_t)cp * kSlots * P1 * P1;
+            for (int e = threadIdx.x; e < kSlots * NR * P1; e += blockDim.x)
+                sT[e] = Tc[(size_t)(e / (NR * P1)) * P1 * P1 + e % (NR * P1)];
+            cp_in = cp;
+            __syncthreads();
+        }
+        const int q = seg.start[lo] + (tile - s_tb[lo]) * kRowsTile + bx;
+        if (q >= seg.start[lo] + seg.count[lo] || row > p) continue;
+        float2 acc[CH], s0[CH];
+#pragma unroll
+        for (int c = 0; c < CH; c++) acc[c] = s0[c] = make_float2(0.f, 0.f);
+        for (int k = 0; k < kSlots; k++) {
+            const int sb = slots[(size_t)q * kSlots + k];
+            if (sb < 0) continue;
+            const float2 *M = mp32 + (size_t)sb * stride + c0;
+            float2 m[P1][CH];
+#pragma unroll
+            for (int j = 0; j < P1; j++)
+#pragma unroll
+                for (int c = 0; c < CH; c++)
+                    m[j][c] = j <= p ? M[(size_t)j * ndc + c] : make_float2(0.f, 0.f);
+            const float2 *t0 = sT + (k * NR + row) * P1;
+#pragma unroll
+            for (int c = 0; c < CH; c++) {
+                s0[c].x += m[0][c].x;
+                s0[c].y += m[0][c].y;
+            }
+#pragma unroll
+            for (int j = 0; j < P1; j++) {
+                const float2 t = t0[j];
+#pragma unroll
+                for (int c = 0; c < CH; c++) {
+                    acc[c].x = fmaf(t.x, m[j][c].x, fmaf(-t.y, m[j][c].y, acc[c].x));
+                    acc[c].y = fmaf(t.x, m[j][c].y, fmaf(t.y, m[j][c].x, acc[c].y));
+                }
+            }
+        }
+        const int b = boxes[q];
+#pragma unroll
+        for (int c = 0; c < CH; c++) {
+            if (row == 0) {
+                const float lr = (float)log(bs[seg.level[lo]]);
+                acc[c].x += lr * s0[c].x;
+                acc[c].y += lr * s0[c].y;
+            }
+            loc[(size_t)b * stride + (size_t)row * ndc + c0 + c] =
+                make_double2((double)acc[c].x, (double)acc[c].y);
         }
     }
 }
@@ -544,25 +653,42 @@ const float2 *fp32_tables(int p, int P1, cudaStream_t s) {
     return d;
 }
 
-template <int P1, int NR = P1>
+template <int P1>
 void launch_fp32(const M2LWork &w, const Tree &T, const CauchyProblem &P, const float2 *Tab,
                  const float2 *mp32, double2 *loc, cudaStream_t s) {
-    const int blocks = std::max(1, std::min(w.ntiles, kNumSM * 16));
-    const SegTable sg = w.seg();
-    const int *boxes = (const int *)w.vals.get();
+    const int ntiles = w.ntiles(kFp32Tile);
+    const int blocks = std::max(1, std::min(ntiles, kNumSM * 16));
+    const SegTable sg = w.seg(kFp32Tile);
+    const int *boxes = w.boxes.get();
     for (int c0 = 0; c0 < P.ndc;) {
         if (P.ndc - c0 >= 2) {
-            m2l_fp32_kernel<P1, 2, NR><<<blocks, kFp32Tile, 0, s>>>(
+            m2l_fp32_kernel<P1, 2><<<blocks, kFp32Tile, 0, s>>>(
                 sg, boxes, w.slots.get(), T.d_boxsize.get(), P.ndc, c0, P.p, Tab, mp32, loc,
-                w.ntiles);
+                ntiles);
             c0 += 2;
         } else {
-            m2l_fp32_kernel<P1, 1, NR><<<blocks, kFp32Tile, 0, s>>>(
+            m2l_fp32_kernel<P1, 1><<<blocks, kFp32Tile, 0, s>>>(
                 sg, boxes, w.slots.get(), T.d_boxsize.get(), P.ndc, c0, P.p, Tab, mp32, loc,
-                w.ntiles);
+                ntiles);
             c0 += 1;
         }
         FMM_CHECK_LAUNCH();
+    }
+}
+
+template <int P1, int NR>
+void launch_rows(const M2LWork &w, const Tree &T, const CauchyProblem &P, const float2 *Tab,
+                 const float2 *mp32, double2 *loc, cudaStream_t s) {
+    const int ntiles = w.ntiles(kRowsTile);
+    const int blocks = std::max(1, std::min(ntiles, kNumSM * 16));
+    for (int c0 = 0; c0 < P.ndc;) {
+        const int ch = P.ndc - c0 >= 2 ? 2 : 1;
+        auto kern = ch == 2 ? m2l_rows_kernel<P1, 2, NR> : m2l_rows_kernel<P1, 1, NR>;
+        kern<<<blocks, kRowsTile * NR, 0, s>>>(w.seg(kRowsTile), w.boxes.get(), w.slots.get(),
+                                               T.d_boxsize.get(), P.ndc, c0, P.p, Tab, mp32, loc,
+                                               ntiles);
+        FMM_CHECK_LAUNCH();
+        c0 += ch;
     }
 }
 
@@ -928,15 +1054,15 @@ bool m2l_tensor_fp64(const Tree &T, const CauchyProblem &P, const double2 *mp,
     if (L < 2 || p > 63) return false;
     bool ok = false;
     const auto wp = m2l_cached<M2LWork>(P.m2l_cache, m2l_key(1, 8, 0), ok,
-                                        [&](M2LWork &x) { return m2l_work(T, P, 8, s, x); });
+                                        [&](M2LWork &x) { return m2l_work(T, P, {8}, s, x); });
     if (!ok) return false;
     const M2LWork &w = *wp;
-    if (w.ntiles == 0) return true;
-    const SegTable sg = w.seg();
-    const int *boxes = (const int *)w.vals.get();
+    if (w.ntarg == 0) return true;
+    const SegTable sg = w.seg(8);
+    const int *boxes = w.boxes.get();
     const double *bs = T.d_boxsize.get();
     const double *binom = device_binomials(s);
-    const int ntiles = w.ntiles;
+    const int ntiles = w.ntiles(8);
     const int ks = (p + 1 + 3) / 4;
     const int mt = (p + 1 + 7) / 8;
 #define FMM_M2L_CASE(MT_, KS_)                                                   \
@@ -1085,7 +1211,7 @@ bool m2l_split_fp64(const Tree &T, const CauchyProblem &P, const double2 *mp, do
     // planning first (nothing is launched when it fails)
     bool ok = false;
     const auto wp = m2l_cached<M2LWork>(P.m2l_cache, m2l_key(1, 8, 0), ok,
-                                        [&](M2LWork &x) { return m2l_work(T, P, 8, s, x); });
+                                        [&](M2LWork &x) { return m2l_work(T, P, {8}, s, x); });
     if (!ok) return false;
     bool ok2 = false;
     const int tpt = 128 / P.ndc;
@@ -1094,22 +1220,23 @@ bool m2l_split_fp64(const Tree &T, const CauchyProblem &P, const double2 *mp, do
     });
     if (!ok2) return false;
     const M2LWork &w = *wp;
-    if (w.ntiles == 0) return true;
+    if (w.ntarg == 0) return true;
+    const int ntiles = w.ntiles(8);
     const float *bimg = split_tail_tables(p, KP, nt, s);
     // 1. the FP64 triangle, storing every local of levels >= 2 with points
     const double *binom = device_binomials(s);
-    const SegTable sg = w.seg();
-    const int *boxes = (const int *)w.vals.get();
+    const SegTable sg = w.seg(8);
+    const int *boxes = w.boxes.get();
     const double *bs = T.d_boxsize.get();
     bool launched = false;
     switch (nt) {
-        case 8: launched = launch_split_triangle<8>(sg, boxes, w.slots.get(), bs, P.ndc, p, binom, mp, loc, w.ntiles, s); break;
-        case 12: launched = launch_split_triangle<12>(sg, boxes, w.slots.get(), bs, P.ndc, p, binom, mp, loc, w.ntiles, s); break;
-        case 16: launched = launch_split_triangle<16>(sg, boxes, w.slots.get(), bs, P.ndc, p, binom, mp, loc, w.ntiles, s); break;
-        case 20: launched = launch_split_triangle<20>(sg, boxes, w.slots.get(), bs, P.ndc, p, binom, mp, loc, w.ntiles, s); break;
-        case 24: launched = launch_split_triangle<24>(sg, boxes, w.slots.get(), bs, P.ndc, p, binom, mp, loc, w.ntiles, s); break;
-        case 28: launched = launch_split_triangle<28>(sg, boxes, w.slots.get(), bs, P.ndc, p, binom, mp, loc, w.ntiles, s); break;
-        case 32: launched = launch_split_triangle<32>(sg, boxes, w.slots.get(), bs, P.ndc, p, binom, mp, loc, w.ntiles, s); break;
+        case 8: launched = launch_split_triangle<8>(sg, boxes, w.slots.get(), bs, P.ndc, p, binom, mp, loc, ntiles, s); break;
+        case 12: launched = launch_split_triangle<12>(sg, boxes, w.slots.get(), bs, P.ndc, p, binom, mp, loc, ntiles, s); break;
+        case 16: launched = launch_split_triangle<16>(sg, boxes, w.slots.get(), bs, P.ndc, p, binom, mp, loc, ntiles, s); break;
+        case 20: launched = launch_split_triangle<20>(sg, boxes, w.slots.get(), bs, P.ndc, p, binom, mp, loc, ntiles, s); break;
+        case 24: launched = launch_split_triangle<24>(sg, boxes, w.slots.get(), bs, P.ndc, p, binom, mp, loc, ntiles, s); break;
+        case 28: launched = launch_split_triangle<28>(sg, boxes, w.slots.get(), bs, P.ndc, p, binom, mp, loc, ntiles, s); break;
+        case 32: launched = launch_split_triangle<32>(sg, boxes, w.slots.get(), bs, P.ndc, p, binom, mp, loc, ntiles, s); break;
         default: break;
     }
     if (!launched) return false;
@@ -1165,29 +1292,32 @@ bool plan_slots(const Tree &T, int spgh, int tpgh, int tile, cudaStream_t s, Slo
     P.sset.pgh = spgh;
     P.tset.pgh = tpgh;
     auto h = std::make_shared<SlotHold>();
-    if (!m2l_work(T, P, tile, s, h->w)) return false;
+    if (!m2l_work(T, P, {}, s, h->w)) return false;
     const M2LWork &w = h->w;
     sp.nseg = w.nseg;
     sp.ntarg = w.ntarg;
-    sp.ntiles = w.ntiles;
-    if (w.ntiles == 0) return true;
-    const int n = w.nseg;
-    sp.tile_base.assign(w.hseg.begin(), w.hseg.begin() + n + 1);
-    sp.start.assign(w.hseg.begin() + n + 1, w.hseg.begin() + 2 * n + 1);
-    sp.count.assign(w.hseg.begin() + 2 * n + 1, w.hseg.begin() + 3 * n + 1);
+    sp.start = w.start;
+    sp.count = w.count;
+    if (w.ntarg == 0) return true;
     const SlotTables st = make_slot_tables();
     std::vector<int2> d(4 * kSlots);
     for (int c = 0; c < 4; c++)
         for (int k = 0; k < kSlots; k++) d[c * kSlots + k] = make_int2(st.dx[c][k], st.dy[c][k]);
     h->dxy.alloc(d.size(), s);
+    // (a small pageable source is staged before the call returns)
     FMM_CUDA(cudaMemcpyAsync(h->dxy.get(), d.data(), d.size() * sizeof(int2),
                              cudaMemcpyHostToDevice, s));
-    FMM_CUDA(cudaStreamSynchronize(s));  // (d is a pageable host vector)
-    sp.boxes = (const int *)w.vals.get();
+    sp.boxes = w.boxes.get();
     sp.slots = w.slots.get();
     sp.dxy = h->dxy.get();
     sp.hold = h;
+    retile_slots(sp, tile);
     return true;
+}
+
+void retile_slots(SlotPlan &sp, int tile) {
+    sp.tile_base = tile_bases(sp.count, tile);
+    sp.ntiles = sp.tile_base[sp.nseg];
 }
 
 namespace {
@@ -1242,54 +1372,50 @@ bool m2l_fp32(const Tree &T, const CauchyProblem &P, const double2 *mp, double2 
     const uint64_t done =
         (simt || tile_only) ? 0 : m2l_window_fp32(T, P, mp32p, loc, errp, s);
     const int wtile = simt ? kFp32Tile : kTcRows / CH;
+    const bool rows = !simt && m2l_exact_rows(p);
     bool ok = false;
-    const auto wp = m2l_cached<M2LWork>(cache, m2l_key(3, wtile, done), ok,
-                                        [&](M2LWork &x) { return m2l_work(T, P, wtile, s, x, done); });
+    // (tiles of the tensor-core form, of its single remaining channels and
+    // of the leading rows from one plan)
+    const auto wp = m2l_cached<M2LWork>(cache, m2l_key(3, wtile, done), ok, [&](M2LWork &x) {
+        std::vector<int> tiles{wtile};
+        if (!simt && CH == 2 && P.ndc % 2 != 0) tiles.push_back(kTcRows);
+        if (rows) tiles.push_back(kRowsTile);
+        return m2l_work(T, P, tiles, s, x, done);
+    });
     if (!ok) return false;
     const M2LWork &w = *wp;
-    if (w.ntiles > 0 && simt) {
+    if (w.ntarg > 0 && simt) {
         if (p + 1 <= 12)
             launch_fp32<12>(w, T, P, fp32_tables(p, 12, s), mp32p, loc, s);
         else
             launch_fp32<20>(w, T, P, fp32_tables(p, 20, s), mp32p, loc, s);
-    } else if (w.ntiles > 0) {
+    } else if (w.ntarg > 0) {
         // tensor cores: K = N = 2 HALF with HALF = 12 (p < 12) or 20
         const int HALF = p + 1 <= 12 ? 12 : 20;
         const int KP = 2 * HALF;
         const float2 *tab0 = nullptr;
         const float *tab = tc_tables(p, KP, s, &tab0);
         const size_t smem = (size_t)(2 * kTcRows * KP + 2 * KP * KP) * sizeof(float);
-        auto launch = [&](auto kern, const M2LWork &ww, int c0) {
+        auto launch = [&](auto kern, int tile, int c0) {
             raise_smem_limit(kern, (int)smem);
-            const int blocks = std::max(1, std::min(ww.ntiles, kNumSM * 4));
-            kern<<<blocks, kTcRows, smem, s>>>(ww.seg(), (const int *)ww.vals.get(), ww.slots.get(),
+            const int ntiles = w.ntiles(tile);
+            const int blocks = std::max(1, std::min(ntiles, kNumSM * 4));
+            kern<<<blocks, kTcRows, smem, s>>>(w.seg(tile), w.boxes.get(), w.slots.get(),
                                                T.d_boxsize.get(), P.ndc, c0, p, tab, tab0,
-                                               mp32p, loc, ww.ntiles, errp);
+                                               mp32p, loc, ntiles, errp);
             FMM_CHECK_LAUNCH();
         };
         int c0 = 0;
         if (CH == 2) {
             for (; P.ndc - c0 >= 2; c0 += 2) {
-                if (HALF == 12) launch(m2l_tc_kernel<2, 12>, w, c0);
-                else launch(m2l_tc_kernel<2, 20>, w, c0);
+                if (HALF == 12) launch(m2l_tc_kernel<2, 12>, wtile, c0);
+                else launch(m2l_tc_kernel<2, 20>, wtile, c0);
             }
         }
-        if (c0 < P.ndc) {
-            // remaining single channels, one channel per row
-            std::shared_ptr<M2LWork> w1;
-            const M2LWork *pw = &w;
-            if (CH != 1) {
-                bool ok1 = false;
-                w1 = m2l_cached<M2LWork>(cache, m2l_key(4, kTcRows, done), ok1, [&](M2LWork &x) {
-                    return m2l_work(T, P, kTcRows, s, x, done);
-                });
-                if (!ok1) return false;
-                pw = w1.get();
-            }
-            for (; c0 < P.ndc; c0++) {
-                if (HALF == 12) launch(m2l_tc_kernel<1, 12>, *pw, c0);
-                else launch(m2l_tc_kernel<1, 20>, *pw, c0);
-            }
+        // remaining single channels, one channel per row
+        for (; c0 < P.ndc; c0++) {
+            if (HALF == 12) launch(m2l_tc_kernel<1, 12>, kTcRows, c0);
+            else launch(m2l_tc_kernel<1, 20>, kTcRows, c0);
         }
     }
     if (!deferred && read_scalar(errp, s) != 0)
@@ -1303,20 +1429,12 @@ bool m2l_fp32(const Tree &T, const CauchyProblem &P, const double2 *mp, double2 
     // leaf's points -- are therefore recomputed in FP32 on the CUDA cores:
     // on the window levels from the windows (m2l_window.cu), on the other
     // levels here with the slot tables.
-    if (!simt && m2l_exact_rows(p)) {
-        bool okr = false;
-        const auto wr = m2l_cached<M2LWork>(cache, m2l_key(5, kFp32Tile, done), okr,
-                                            [&](M2LWork &x) {
-                                                return m2l_work(T, P, kFp32Tile, s, x, done);
-                                            });
-        if (!okr) return false;
-        if (wr->ntiles > 0) {
-            const bool hess = std::max(P.sset.n > 0 ? P.sset.pgh : 0, P.tset.n > 0 ? P.tset.pgh : 0) >= 3;
-            if (hess)
-                launch_fp32<20, kM2LExactRowsHess>(*wr, T, P, fp32_tables(p, 20, s), mp32p, loc, s);
-            else
-                launch_fp32<20, kM2LExactRows>(*wr, T, P, fp32_tables(p, 20, s), mp32p, loc, s);
-        }
+    if (rows && w.ntarg > 0) {
+        const bool hess = std::max(P.sset.n > 0 ? P.sset.pgh : 0, P.tset.n > 0 ? P.tset.pgh : 0) >= 3;
+        if (hess)
+            launch_rows<20, kM2LExactRowsHess>(w, T, P, fp32_tables(p, 20, s), mp32p, loc, s);
+        else
+            launch_rows<20, kM2LExactRows>(w, T, P, fp32_tables(p, 20, s), mp32p, loc, s);
     }
     return true;
 }

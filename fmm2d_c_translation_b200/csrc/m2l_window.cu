@@ -53,7 +53,6 @@
 // with mbarriers; every wait is bounded in time and a wait that runs out
 // stops all roles of the block and sets *err.
 #include "laplace.cuh"
-#include "sort.cuh"
 #include "tc_common.cuh"
 
 #include <algorithm>
@@ -661,7 +660,7 @@ WinTables win_tables(int p, int HALF, cudaStream_t s) {
 }
 
 // Runs of one evaluation: the parents of the targets, grouped by (level,
-// row, column / TB) with a 64-bit key sorted in two stable 32-bit passes.
+// row, column / TB).
 struct WinPlan {
     DevBuf<int> wbox, tbox, rlev;
     std::vector<std::pair<int, int>> ranges;  // [first run, count) per launch
@@ -681,117 +680,135 @@ struct WinCounts {
     }
 };
 
+// First run of every window level.
+struct WinBase {
+    int v[64];
+    uint64_t levels;
+};
+
+// The runs come from a hash table over the parents' (level, row, column /
+// TB) keys: the parent that inserts a key numbers its run within the level,
+// in about box order (neighbouring runs share windows in L2), and one read
+// of the per-level counts decides the window levels.  Sorting the keys
+// instead (two 32-bit radix sorts, two scans, three synchronisations) took
+// most of the 0.55 ms M2L of a 300-point call and 0.3 ms of the 10^5-point
+// one's; the order of the runs does not enter the results.
 bool win_plan(const Tree &T, const CauchyProblem &P, int CH, cudaStream_t s, WinPlan &W) {
     const int L = T.nlevels;
     if (L < 2 || L - 1 > kWinMaxParentLevel) return false;
     const int TB = 128 / CH, WP = TB + 2;
-    const int nb = T.nboxes, lo1 = T.lstart[1], lo2 = T.lstart[2];
+    const int lo1 = T.lstart[1];
     const int npar = T.lend[L - 1] - lo1;
     if (npar <= 0) return false;
+    // a level goes through the windows when its runs are at least 1/8 full:
+    // one with fewer boxes than that has none
+    uint64_t cand = 0;
+    for (int l = 2; l <= L; l++)
+        if ((long long)(T.lend[l] - T.lstart[l]) * 8 >= 4 * TB) cand |= 1ull << l;
+    if (!cand) return true;
     const int2 *sse = T.srcse.get(), *tse = T.trgse.get();
     const int spgh = P.sset.pgh, tpgh = P.tset.pgh;
-    const int *lev = T.level.get(), *par = T.parent.get(), *chi = T.child.get();
+    const int *lev = T.level.get(), *chi = T.child.get();
     const int *nnb = T.nnbors.get(), *nbr = T.nbors.get();
     const double2 *cen = T.centers.get();
     const double *bsd = T.d_boxsize.get();
     const WinCounts npts{sse, tse, spgh, tpgh};
-    // parents of the boxes that receive an M2L
-    DevBuf<int> flag(npar, s), pos(npar, s), total(1, s);
-    flag.zero(s);
+    size_t cap = 1024;
+    while (cap < 2 * (size_t)npar) cap <<= 1;
+    // keys (empty: all ones), run numbers within their level, table slot of
+    // every parent, [64] runs and [64] targets per level
+    DevBuf<unsigned long long> keys(cap, s);
+    DevBuf<int> num(cap, s), slot(npar, s), cnt(128, s);
+    FMM_CUDA(cudaMemsetAsync(keys.get(), 0xff, cap * sizeof(unsigned long long), s));
+    cnt.zero(s);
     {
-        int *fl = flag.get();
-        for_each(nb - lo2, s, [=] __device__(int64_t i) {
-            const int b = lo2 + (int)i;
-            if (npts(b) > 0) fl[par[b] - lo1] = 1;
-        });
-    }
-    exclusive_scan_i32(flag.get(), pos.get(), npar, total.get(), s);
-    const int m = read_scalar(total.get(), s);
-    if (m == 0) return true;
-    DevBuf<uint32_t> klo(m, s), khi(m, s), k0(m, s), k1(m, s), idx(m, s), ktmp(m, s), vtmp(m, s);
-    DevBuf<int> pbox(m, s);
-    {
-        const int *fl = flag.get(), *ps = pos.get();
-        uint32_t *kl = klo.get(), *kh = khi.get(), *a0 = k0.get(), *a1 = k1.get(), *ix = idx.get();
-        int *pb = pbox.get();
+        unsigned long long *ky = keys.get();
+        int *nm = num.get(), *sl = slot.get(), *ct = cnt.get();
         const int tb = TB;
+        const unsigned mask = (unsigned)(cap - 1);
         for_each(npar, s, [=] __device__(int64_t i) {
-            if (!fl[i]) return;
-            const int q = ps[i], b = lo1 + (int)i, lp = lev[b];
-            const double bsl = bsd[lp], half = 0.5 * (double)((1ll << lp) - 1);
-            const double2 c = cen[b], c0 = cen[0];
-            const long long X = llrint((c.x - c0.x) / bsl + half);
-            const long long Y = llrint((c.y - c0.y) / bsl + half);
-            const uint64_t key = ((uint64_t)lp << 58) | ((uint64_t)Y << 29) | (uint64_t)(X / tb);
-            kl[q] = (uint32_t)key;
-            kh[q] = (uint32_t)(key >> 32);
-            a0[q] = (uint32_t)key;
-            a1[q] = (uint32_t)(key >> 32);
-            ix[q] = (uint32_t)q;
-            pb[q] = b;
-        });
-    }
-    radix_sort_pairs(klo.get(), idx.get(), ktmp.get(), vtmp.get(), m, 32, s);
-    {
-        const uint32_t *ix = idx.get(), *a1 = k1.get();
-        uint32_t *kh = khi.get();
-        for_each(m, s, [=] __device__(int64_t q) { kh[q] = a1[ix[q]]; });
-    }
-    radix_sort_pairs(khi.get(), idx.get(), ktmp.get(), vtmp.get(), m, 32, s);
-    // runs: a new run where the key changes
-    DevBuf<int> head(m, s), rid(m, s), nrun_d(1, s);
-    {
-        const uint32_t *ix = idx.get(), *a0 = k0.get(), *a1 = k1.get();
-        int *hd = head.get();
-        for_each(m, s, [=] __device__(int64_t q) {
-            const uint32_t i = ix[q];
-            int h = 1;
-            if (q > 0) {
-                const uint32_t j = ix[q - 1];
-                h = (a0[i] != a0[j] || a1[i] != a1[j]) ? 1 : 0;
+            const int b = lo1 + (int)i, lp = lev[b];
+            int ntq = 0;
+            if ((cand >> (lp + 1)) & 1ull) {
+                const int4 ch = *reinterpret_cast<const int4 *>(chi + 4 * (size_t)b);
+                if (ch.x >= 0)
+                    ntq = (npts(ch.x) > 0) + (npts(ch.y) > 0) + (npts(ch.z) > 0) + (npts(ch.w) > 0);
             }
-            hd[q] = h;
+            int at = -1, fresh = 0;
+            if (ntq > 0) {
+                const double bsl = bsd[lp], half = 0.5 * (double)((1ll << lp) - 1);
+                const double2 c = cen[b], c0 = cen[0];
+                const long long X = llrint((c.x - c0.x) / bsl + half);
+                const long long Y = llrint((c.y - c0.y) / bsl + half);
+                const unsigned long long key =
+                    ((unsigned long long)lp << 58) | ((unsigned long long)Y << 29) |
+                    (unsigned long long)(X / tb);
+                unsigned h = (unsigned)((key * 0x9e3779b97f4a7c15ull) >> 32) & mask;
+                // (the table is at most half full, so an empty slot is found)
+                for (;;) {
+                    unsigned long long v = *(volatile unsigned long long *)(ky + h);
+                    if (v == ~0ull) v = atomicCAS(ky + h, ~0ull, key);
+                    if (v == ~0ull) fresh = 1;
+                    if (v == ~0ull || v == key) break;
+                    h = (h + 1) & mask;
+                }
+                at = (int)h;
+            }
+            sl[i] = at;
+            // runs and targets per level, one atomic per group of lanes of
+            // the same level (consecutive parents share levels)
+            const unsigned am = __activemask();
+            const unsigned peers = __match_any_sync(am, lp);
+            const int lane = (int)(threadIdx.x & 31), lead = __ffs(peers) - 1;
+            const unsigned fm = __ballot_sync(am, fresh) & peers;
+            const int nt = __reduce_add_sync(peers, ntq);
+            int base = 0;
+            if (lane == lead) {
+                if (fm) base = atomicAdd(&ct[lp + 1], __popc(fm));
+                if (nt) atomicAdd(&ct[64 + lp + 1], nt);
+            }
+            base = __shfl_sync(peers, base, lead);
+            if (fresh) nm[at] = base + __popc(fm & ((1u << lane) - 1u));
         });
     }
-    exclusive_scan_i32(head.get(), rid.get(), m, nrun_d.get(), s);
-    const int nrun = read_scalar(nrun_d.get(), s);
+    std::vector<int> hc(128);
+    read_small(hc.data(), cnt.get(), 128 * sizeof(int), s);
+    WinBase base;
+    base.levels = 0;
+    int nrun = 0;
+    for (int l = 0; l < 64; l++) {
+        base.v[l] = nrun;
+        const int nr = hc[l], nt = hc[64 + l];
+        if (l < 2 || l > L || nr <= 0 || (long long)nt * 8 < (long long)nr * 4 * TB) continue;
+        base.levels |= 1ull << l;
+        nrun += nr;
+    }
+    if (nrun == 0) return true;
+    W.levels = base.levels;
+    W.ranges.push_back({0, nrun});
     W.wbox.alloc((size_t)nrun * 12 * WP, s);
     W.tbox.alloc((size_t)nrun * 4 * TB, s);
     W.rlev.alloc(nrun, s);
     FMM_CUDA(cudaMemsetAsync(W.wbox.get(), 0xff, (size_t)nrun * 12 * WP * sizeof(int), s));
     FMM_CUDA(cudaMemsetAsync(W.tbox.get(), 0xff, (size_t)nrun * 4 * TB * sizeof(int), s));
-    DevBuf<int> cnt(128, s);
-    cnt.zero(s);
     {
-        const uint32_t *ix = idx.get();
-        const int *pb = pbox.get(), *hd = head.get(), *rd = rid.get();
-        int *wb = W.wbox.get(), *tbx = W.tbox.get(), *rl = W.rlev.get(), *ct = cnt.get();
+        const int *nm = num.get(), *sl = slot.get();
+        int *wb = W.wbox.get(), *tbx = W.tbox.get(), *rl = W.rlev.get();
         const int tb = TB, wp = WP;
-        for_each(m, s, [=] __device__(int64_t q) {
-            const int b = pb[ix[q]], run = rd[q] + hd[q] - 1;
-            const int lp = lev[b];
+        for_each(npar, s, [=] __device__(int64_t i) {
+            const int at = sl[i];
+            if (at < 0) return;
+            const int b = lo1 + (int)i, lp = lev[b];
+            if (!((base.levels >> (lp + 1)) & 1ull)) return;
+            const int run = base.v[lp + 1] + nm[at];
             const double bsl = bsd[lp], half = 0.5 * (double)((1ll << lp) - 1);
             const double2 cb = cen[b], c0 = cen[0];
             const long long X = llrint((cb.x - c0.x) / bsl + half);
             const int t = (int)(X % tb);
-            if (hd[q]) rl[run] = lp + 1;
-            int ntq = 0;
+            rl[run] = lp + 1;
             for (int c = 0; c < 4; c++) {
                 const int kb = chi[4 * b + c];
-                if (kb >= 0 && npts(kb) > 0) {
-                    tbx[((size_t)run * 4 + c) * tb + t] = kb;
-                    ntq++;
-                }
-            }
-            // runs and targets per level, one atomic per group of lanes
-            // of the same level (consecutive parents share levels)
-            const unsigned am = __activemask();
-            const unsigned peers = __match_any_sync(am, lp);
-            const int nr = __reduce_add_sync(peers, hd[q] ? 1 : 0);
-            const int nt = __reduce_add_sync(peers, ntq);
-            if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) {
-                if (nr) atomicAdd(&ct[lp + 1], nr);
-                if (nt) atomicAdd(&ct[64 + lp + 1], nt);
+                if (kb >= 0 && npts(kb) > 0) tbx[((size_t)run * 4 + c) * tb + t] = kb;
             }
             for (int k = 0; k < nnb[b]; k++) {
                 const int cb2 = nbr[9 * b + k];
@@ -808,23 +825,6 @@ bool win_plan(const Tree &T, const CauchyProblem &P, int CH, cudaStream_t s, Win
             }
         });
     }
-    std::vector<int> hc(128);
-    read_small(hc.data(), cnt.get(), 128 * sizeof(int), s);
-    // a level goes through the windows when its runs are at least 1/8 full
-    int start = 0, open = -1;
-    for (int l = 0; l <= L + 1 && l < 64; l++) {
-        const int nr = hc[l], nt = hc[64 + l];
-        const bool win = l >= 2 && l <= L && nr > 0 && (long long)nt * 8 >= (long long)nr * 4 * TB;
-        if (win) {
-            W.levels |= 1ull << l;
-            if (open < 0) open = start;
-        } else if (open >= 0) {
-            W.ranges.push_back({open, start - open});
-            open = -1;
-        }
-        start += nr;
-    }
-    if (open >= 0) W.ranges.push_back({open, start - open});
     return true;
 }
 
