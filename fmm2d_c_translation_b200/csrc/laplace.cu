@@ -9,6 +9,7 @@
 // writer, so no pass needs atomics.  Formulas follow
 // c_translation/src/laprouts2d.c and cauchykernels2d.c term by term.
 #include "laplace.cuh"
+#include "pairmath.cuh"
 
 #include <algorithm>
 #include <complex>
@@ -476,10 +477,17 @@ __device__ __forceinline__ float half_ln_fast(float x) {  // 0.5 * ln(x)
     asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r * 0.34657359027997264f;  // ln(2) / 2
 }
-__device__ __forceinline__ double rcp_pair(double x) { return 1.0 / x; }
-__device__ __forceinline__ float rcp_pair(float x) { return rcp_fast(x); }
-__device__ __forceinline__ double half_ln_pair(double x) { return 0.5 * log(x); }
-__device__ __forceinline__ float half_ln_pair(float x) { return half_ln_fast(x); }
+// (FAST, FP64: normal numbers only, pairmath.cuh)
+template <bool FAST> __device__ __forceinline__ double rcp_pair(double x) {
+    return FAST ? rcp_pos(x) : 1.0 / x;
+}
+template <bool FAST> __device__ __forceinline__ float rcp_pair(float x) { return rcp_fast(x); }
+template <bool FAST> __device__ __forceinline__ double half_ln_pair(double x) {
+    return FAST ? half_ln_pos(x) : 0.5 * log(x);
+}
+template <bool FAST> __device__ __forceinline__ float half_ln_pair(float x) {
+    return half_ln_fast(x);
+}
 
 // Steps 6 and 7 with one warp per leaf: the warp evaluates the leaf's
 // list-3 multipoles and local expansion at all of the leaf's points and
@@ -641,7 +649,7 @@ __global__ void __launch_bounds__(kFarWarps * 32) far_leaf_kernel(
 // log|z| + d/z, grad += q/z - d/z^2, hess += -q/z^2 + 2d/z^3 (z = t - s),
 // with `st` the source's strengths (charges of the CH channels, then
 // dipoles).  Pairs inside the threshold contribute exactly zero.
-template <int CH, int PGH, bool IFC, bool IFD, bool MIXED, bool LAPR>
+template <int CH, int PGH, bool IFC, bool IFD, bool MIXED, bool LAPR, bool FAST>
 __device__ __forceinline__ void p2p_pair(const typename PosT<MIXED>::T &x,
                                          const typename PosT<MIXED>::T &sp,
                                          const typename Real<MIXED>::T2 *st,
@@ -657,7 +665,7 @@ __device__ __forceinline__ void p2p_pair(const typename PosT<MIXED>::T &x,
     // skipped pairs contribute exactly zero, without a branch
     const bool skip = PGH == 1 ? (rr <= th2) : (rr < th2);
     const R rrs = skip ? (R)1 : rr;
-    const R ri = skip ? (R)0 : rcp_pair(rrs);
+    const R ri = skip ? (R)0 : rcp_pair<FAST>(rrs);
     R2 zi;
     zi.x = dx * ri;
     zi.y = -dy * ri;
@@ -665,7 +673,7 @@ __device__ __forceinline__ void p2p_pair(const typename PosT<MIXED>::T &x,
     if (PGH >= 2 || IFD) zi2 = zmul(zi, zi);
     if (PGH >= 3 && IFD) zi3 = zmul(zi2, zi);
     R rl = 0;
-    if (IFC) rl = skip ? (R)0 : half_ln_pair(rrs);
+    if (IFC) rl = skip ? (R)0 : half_ln_pair<FAST>(rrs);
 #pragma unroll
     for (int q = 0; q < CH; q++) {
         if (IFC) {
@@ -813,7 +821,7 @@ __global__ void __launch_bounds__(kP2PWarps * 32) p2p_kernel(
                 if (act) {
 #pragma unroll 4
                     for (int kk = g; kk < nst; kk += G)
-                        p2p_pair<CH, PGH, IFC, IFD, MIXED, LAPR>(x, s_pos[kk], s_str + kk * kStr,
+                        p2p_pair<CH, PGH, IFC, IFD, MIXED, LAPR, true>(x, s_pos[kk], s_str + kk * kStr,
                                                                  th2, po, gr, he);
                 }
             }
@@ -978,7 +986,7 @@ __global__ void __launch_bounds__(kP2PWarps * 32) p2p_flat_kernel(
                     const int j0 = blk * sb, j1 = min(nst, j0 + sb);
 #pragma unroll 4
                     for (int kk = j0; kk < j1; kk++)
-                        p2p_pair<CH, PGH, IFC, IFD, MIXED, LAPR>(x, s_pos[kk], s_str + kk * kStr,
+                        p2p_pair<CH, PGH, IFC, IFD, MIXED, LAPR, false>(x, s_pos[kk], s_str + kk * kStr,
                                                                  th2, apo, agr, ahe);
                     R2 *pp = part + (size_t)i * kNo;
 #pragma unroll
@@ -1049,9 +1057,14 @@ void launch_p2p_t(const Tree &T, const CauchyProblem &P, int c0, double th2,
     // on a B200 (10^7 + 10^7 uniform points, lfmm2d_st_cd_g) 5.56 against
     // 5.75 ms mixed, 19.1 against 17.1 ms FP64, where the flattened form's
     // larger register and shared-memory footprint costs occupancy.
-    // FMM2D_B200_P2P=flat / group overrides.
+    // FMM2D_B200_P2P=flat / group overrides.  In FP64 the groups take the
+    // reciprocal and logarithm of normal numbers: the pairs that count lie
+    // between thresh^2 and 2^103 thresh^2 (the threshold is 2^-51 of the
+    // domain's side).  Domains so small or large that those leave the normal
+    // range take the flattened form, which divides and calls log().
     const char *mode = getenv("FMM2D_B200_P2P");
-    const bool flat = mode ? !strcmp(mode, "flat") : MIXED;
+    const bool normal = MIXED || (th2 >= 2.3e-308 && th2 <= 1e276);
+    const bool flat = !normal || (mode ? !strcmp(mode, "flat") : MIXED);
 #define FMM_P2P_CASE(IFC, IFD)                                                  \
     do {                                                                        \
         if (flat) {                                                             \
