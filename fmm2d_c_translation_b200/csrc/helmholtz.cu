@@ -599,6 +599,8 @@ __global__ void __launch_bounds__(256) helm_l2l_kernel(
     }
 }
 
+#include "helm_shift.cuh"
+
 // M2L over list 2 at level l; tables per offset (ix, iy) in [-3, 3]^2.
 __global__ void __launch_bounds__(256) helm_m2l_kernel(
     int lo, int hi, int nd, const int *__restrict__ nlist2, const int *__restrict__ list2,
@@ -1513,6 +1515,10 @@ namespace {
 struct LevTab {
     size_t m2m = 0, m2m_s = 0, m2m_pw = 0, l2l = 0, l2l_s = 0, l2l_pw = 0, m2l = 0, m2l_pw = 0;
     size_t m2l_sc = 0;   // M2L table of the scaled form, T_q rs^-|q|
+    // folded M2M and L2L: child 0's table T_q r^|q| and the factors of the
+    // input and output orders
+    size_t m2m_f = 0, m2m_in = 0, m2m_out = 0, l2l_f = 0, l2l_in = 0, l2l_out = 0;
+    bool m2m_ok = false, l2l_ok = false;
     bool sc_ok = false;  // the scaled form applies on this level
     double m2l_max = 0;  // largest |T_q| of the M2L table (tensor-core form's scale)
 };
@@ -1594,6 +1600,25 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
             }
             return o;
         };
+        // The folded form of the shift whose child-0 table (2N + 1 entries)
+        // is at ct[tab] and whose output factors S are at rt[sf]: table
+        // T_q r^|q|, input order j times r^(sign |j|), output order i times
+        // S_i r^(-sign |i|); false where a power leaves 1e+-220.
+        auto folded = [&](size_t tab, size_t sf, int N, int n1, int n2, double r, int sign,
+                          size_t &o_tab, size_t &o_in, size_t &o_out) {
+            if (!(r > 0.0) || N * std::fabs(std::log10(r)) > 220.0) return false;
+            std::vector<double> pw(N + 1);
+            pw[0] = 1.0;
+            for (int e = 1; e <= N; e++) pw[e] = pw[e - 1] * r;
+            o_tab = ct.size();
+            for (int q = -N; q <= N; q++) ct.push_back(cscal(ct[tab + q + N], pw[std::abs(q)]));
+            o_in = rt.size();
+            for (int j = 0; j <= n1; j++) rt.push_back(sign > 0 ? pw[j] : 1.0 / pw[j]);
+            o_out = rt.size();
+            for (int i = 0; i <= n2; i++)
+                rt.push_back(rt[sf + i] * (sign > 0 ? 1.0 / pw[i] : pw[i]));
+            return true;
+        };
         for (int l = 2; l <= nl; l++) {
             const HLevel &L = hl[l];
             if (l + 1 <= nl) {
@@ -1616,6 +1641,8 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
                         f = f * C.rs / L.rs;
                     }
                     lt[l].m2m_pw = powtab(C.rs, 2 * n1);
+                    lt[l].m2m_ok = folded(lt[l].m2m, lt[l].m2m_s, N, n1, n2, C.rs, 1, lt[l].m2m_f,
+                                          lt[l].m2m_in, lt[l].m2m_out);
                 }
                 // L2L: parent (scale r1) -> child (scale r2), d = child - parent
                 {
@@ -1634,6 +1661,8 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
                         f = f * C.rs / L.rs;
                     }
                     lt[l].l2l_pw = powtab(L.rs, 2 * n2);
+                    lt[l].l2l_ok = folded(lt[l].l2l, lt[l].l2l_s, N, n1, n2, L.rs, -1, lt[l].l2l_f,
+                                          lt[l].l2l_in, lt[l].l2l_out);
                 }
             }
             // M2L: d = target - source = (ix, iy) * boxsize
@@ -1747,9 +1776,31 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
     FMM_CHECK_LAUNCH();
     prof_mark("h_p2m_p2l", s);
     // ---- M2M, upward (parents at levels nl-1 .. 2) ----
+    // Folded shifts: boxes per block so that a level gives every SM a few
+    // blocks; levels whose staging does not fit into shared memory (orders
+    // above about 120) keep the general kernels
+    auto fold_range = [&](int n) {
+        return std::max(4, std::min(kShRange, (n + kNumSM * 8 - 1) / (kNumSM * 8)));
+    };
+    auto fold_smem = [&](int n1, int n2, int per) {
+        return ((size_t)2 * (n1 + n2) + 1 + (size_t)shift_units(2 * n2 + 1) * (2 * n1 + 1) * per) *
+               sizeof(double2);
+    };
+    constexpr size_t kFoldSmem = 200 * 1024;
     for (int l = nl - 1; l >= 2; l--) {
         if (!hl[l].flag) continue;
         const int lo = T.lstart[l], hi = T.lend[l];
+        const size_t fsm = fold_smem(hl[l + 1].p, hl[l].p, 4);
+        if (lt[l].m2m_ok && fsm <= kFoldSmem) {
+            const int range = fold_range(hi - lo);
+            raise_smem_limit(helm_m2m_fold_kernel, fsm);
+            helm_m2m_fold_kernel<<<(hi - lo + range - 1) / range, kShThreads, fsm, s>>>(
+                lo, hi, range, nd, T.nchild.get(), T.child.get(), T.srcse.get(), d_lv.get(), l,
+                d_ct.get() + lt[l].m2m_f, d_rt.get() + lt[l].m2m_in, d_rt.get() + lt[l].m2m_out,
+                mp.get());
+            FMM_CHECK_LAUNCH();
+            continue;
+        }
         const int64_t work = (int64_t)(hi - lo) * (2 * hl[l].p + 1) * nd;
         helm_m2m_kernel<<<grid_for(work, 256), 256, 0, s>>>(
             lo, hi, nd, T.nchild.get(), T.child.get(), T.srcse.get(), d_lv.get(), l,
@@ -1897,6 +1948,17 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
     // ---- L2L, downward (parents at levels 2 .. nl-1) ----
     for (int l = 2; l <= nl - 1; l++) {
         if (!hl[l].flag) continue;
+        const size_t fsm = fold_smem(hl[l].p, hl[l + 1].p, 1);
+        if (lt[l].l2l_ok && fsm <= kFoldSmem) {
+            const int plo = T.lstart[l], phi = T.lend[l], range = fold_range(phi - plo);
+            raise_smem_limit(helm_l2l_fold_kernel, fsm);
+            helm_l2l_fold_kernel<<<(phi - plo + range - 1) / range, kShThreads, fsm, s>>>(
+                plo, phi, range, nd, T.nchild.get(), T.child.get(), d_lv.get(), l,
+                d_ct.get() + lt[l].l2l_f, d_rt.get() + lt[l].l2l_in, d_rt.get() + lt[l].l2l_out,
+                loc.get());
+            FMM_CHECK_LAUNCH();
+            continue;
+        }
         const int lo = T.lstart[l + 1], hi = T.lend[l + 1];
         const int64_t work = (int64_t)(hi - lo) * (2 * hl[l + 1].p + 1) * nd;
         helm_l2l_kernel<<<grid_for(work, 256), 256, 0, s>>>(
