@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <memory>
 #include <mutex>
 #include <stdlib.h>
 #include <string.h>
@@ -426,6 +427,8 @@ bool m2l_work(const Tree &T, const CauchyProblem &P, const std::vector<int> &til
                              cudaMemcpyHostToDevice, s));
     return true;
 }
+
+#include "m2l_orbit.cuh"
 
 // ---------------------------------------------------------------------------
 // FP32 M2L of the mixed-precision mode.  With t the slot offset in box
@@ -1062,6 +1065,7 @@ bool m2l_tensor_fp64(const Tree &T, const CauchyProblem &P, const double2 *mp,
     const int *boxes = w.boxes.get();
     const double *bs = T.d_boxsize.get();
     const double *binom = device_binomials(s);
+    if (m2l_orbit(w, T, P.ndc, p, binom, mp, loc, s)) return true;
     const int ntiles = w.ntiles(8);
     const int ks = (p + 1 + 3) / 4;
     const int mt = (p + 1 + 7) / 8;
