@@ -16,6 +16,7 @@
 #include <mutex>
 #include <stdlib.h>
 #include <string.h>
+#include <type_traits>
 
 namespace fmm2d {
 
@@ -1261,65 +1262,87 @@ __device__ __forceinline__ int child_pos(const int *__restrict__ child, int pb, 
 // Step 3, M2M (l2dmpmp, laprouts2d.c:666-775) for the parents of one level:
 //   H_i = sum over children with sources of sum_j A[cpos][i][j] M_j,
 // with the fixed shift matrices A of the four child positions.
+// The parents visited come from a BoxList or, with ids null, are all boxes of
+// [lo, hi) with children.
+// Four lanes per output, one per child.
 template <int CH>
 __global__ void __launch_bounds__(256) m2m_coef_kernel(
-    int lo, int hi, int p, const int *__restrict__ nchild,
-    const int *__restrict__ child, const int2 *__restrict__ sse,
+    int lo, int hi, int p, const int *__restrict__ ids, const int *__restrict__ nids,
+    const int *__restrict__ nchild, const int *__restrict__ child, const int2 *__restrict__ sse,
     const double2 *__restrict__ A, int ndc, int c0, double2 *__restrict__ mp) {
     const int np1 = p + 1, stride = np1 * ndc;
-    const int64_t n = (int64_t)(hi - lo) * np1;
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n;
-         t += (int64_t)gridDim.x * blockDim.x) {
-        const int b = lo + (int)(t / np1), i = (int)(t % np1);
-        if (nchild[b] == 0) continue;
+    const int64_t n = (int64_t)(ids ? *nids : hi - lo) * np1 * 4;
+    // warp-uniform trip count: the lanes of an output meet in the shuffles
+    for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n;
+         base += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t t = base + threadIdx.x;
+        const bool valid = t < n;
+        const int64_t o = valid ? t >> 2 : 0;
+        const int k = (int)(o / np1), i = (int)(o % np1), cp = (int)(t & 3);
+        const int b = ids ? ids[k] : lo + k;
+        const bool par = valid && nchild[b] != 0;
+        const int cb = par ? child[4 * b + cp] : -1;
         double2 acc[CH];
 #pragma unroll
         for (int q = 0; q < CH; q++) acc[q] = make_double2(0.0, 0.0);
-        for (int cp = 0; cp < 4; cp++) {
-            const int cb = child[4 * b + cp];
-            if (count(sse, cb) <= 0) continue;
-            const double2 *Arow = A + ((size_t)cp * np1 + i) * np1;
+        if (cb >= 0 && count(sse, cb) > 0) {
+            const double2 *At = A + (size_t)cp * np1 * np1 + i;
             const double2 *M = mp + (size_t)cb * stride + c0;
-            for (int j = 0; j <= i; j++) {
-                const double2 a = Arow[j];
+#pragma unroll 8
+            for (int j = 0; j < np1; j++) {  // (entries j > i are zero)
+                const double2 a = __ldg(At + (size_t)j * np1);
 #pragma unroll
                 for (int q = 0; q < CH; q++) cfma(acc[q], a, M[(size_t)j * ndc + q]);
             }
         }
 #pragma unroll
-        for (int q = 0; q < CH; q++) mp[(size_t)b * stride + (size_t)i * ndc + c0 + q] = acc[q];
+        for (int q = 0; q < CH; q++) {
+#pragma unroll
+            for (int d = 1; d < 4; d <<= 1) {
+                acc[q].x += __shfl_xor_sync(0xffffffffu, acc[q].x, d);
+                acc[q].y += __shfl_xor_sync(0xffffffffu, acc[q].y, d);
+            }
+            if (par && cp == 0) mp[(size_t)b * stride + (size_t)i * ndc + c0 + q] = acc[q];
+        }
     }
 }
 
 // Step 5, L2L (l2dlocloc, laprouts2d.c:777-884) for the children of one
 // level whose parent holds points:  L_i += sum_{j>=i} A[cpos][i][j] Lp_j.
+// The children visited come from a BoxList or, with ids null, are all boxes
+// of [lo, hi); loc32 (optional) receives the FP32 copy of the final sums.
 template <int CH>
 __global__ void __launch_bounds__(256) l2l_coef_kernel(
-    int lo, int hi, int p, EvalCounts ec, const int *__restrict__ parent,
+    int lo, int hi, int p, EvalCounts ec, const int *__restrict__ ids,
+    const int *__restrict__ nids, const int *__restrict__ parent,
     const int *__restrict__ child, const double2 *__restrict__ A, int ndc,
-    int c0, double2 *__restrict__ loc) {
+    int c0, double2 *__restrict__ loc, float2 *__restrict__ loc32) {
     const int np1 = p + 1, stride = np1 * ndc;
-    const int64_t n = (int64_t)(hi - lo) * np1;
+    const int64_t n = (int64_t)(ids ? *nids : hi - lo) * np1;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n;
          t += (int64_t)gridDim.x * blockDim.x) {
-        const int b = lo + (int)(t / np1), i = (int)(t % np1);
+        const int k = (int)(t / np1), i = (int)(t % np1);
+        const int b = ids ? ids[k] : lo + k;
         const int pb = parent[b];
-        if (ec.npts(pb) <= 0) continue;
+        if (!ids && ec.npts(pb) <= 0) continue;
         const int cp = child_pos(child, pb, b);
-        const double2 *Arow = A + ((size_t)cp * np1 + i) * np1;
+        const double2 *At = A + (size_t)cp * np1 * np1 + i;
         const double2 *Lp = loc + (size_t)pb * stride + c0;
         double2 acc[CH];
 #pragma unroll
         for (int q = 0; q < CH; q++) acc[q] = make_double2(0.0, 0.0);
-        for (int j = i; j <= p; j++) {
-            const double2 a = Arow[j];
+#pragma unroll 8
+        for (int j = 0; j < np1; j++) {  // (entries j < i are zero)
+            const double2 a = __ldg(At + (size_t)j * np1);
 #pragma unroll
             for (int q = 0; q < CH; q++) cfma(acc[q], a, Lp[(size_t)j * ndc + q]);
         }
 #pragma unroll
         for (int q = 0; q < CH; q++) {
-            double2 &o = loc[(size_t)b * stride + (size_t)i * ndc + c0 + q];
-            o = cadd(o, acc[q]);
+            const size_t o = (size_t)b * stride + (size_t)i * ndc + c0 + q;
+            const double2 r = cadd(loc[o], acc[q]);
+            loc[o] = r;
+            if (loc32) loc32[o] = make_float2((float)r.x, (float)r.y);
         }
     }
 }
@@ -1329,7 +1352,8 @@ __global__ void __launch_bounds__(256) l2l_coef_kernel(
 // in x and y (r_c the child's box size), so with s = sx + i sy, sx, sy = +-1,
 //   M2M: z0/r_child = s/2, z0/r_parent = s/4;  L2L: z0/r_parent = s/4,
 //   r_child/z0 = 2/s,
-// all exact in binary.  Layout [cpos][i][j], (p+1)^2 per position.
+// all exact in binary.  Layout [cpos][j][i], (p+1)^2 per position, so that
+// threads of consecutive outputs i read consecutive entries.
 const double2 *shift_tables(int p, bool m2m, cudaStream_t s) {
     static std::mutex mu;
     static std::vector<std::pair<long, const double2 *>> cache;
@@ -1351,6 +1375,13 @@ const double2 *shift_tables(int p, bool m2m, cudaStream_t s) {
     }
     auto binom = [&](int l, int m) { return (m < 0 || m > l) ? 0.0 : C[(size_t)l * nc + m]; };
     typedef std::complex<double> cd;
+    // (exact: the powers of (+-1 +- i) / 4 and 1 -+ i are binary fractions)
+    auto ipow = [](cd z, int e) {
+        cd v(1.0, 0.0);
+        for (int k = 0; k < e; k++)
+            v = cd(v.real() * z.real() - v.imag() * z.imag(), v.real() * z.imag() + v.imag() * z.real());
+        return v;
+    };
     std::vector<double2> h((size_t)4 * n * n, make_double2(0.0, 0.0));
     for (int cp = 0; cp < 4; cp++) {
         const cd sgn((cp & 1) ? 1.0 : -1.0, (cp & 2) ? 1.0 : -1.0);
@@ -1362,14 +1393,14 @@ const double2 *shift_tables(int p, bool m2m, cudaStream_t s) {
                     if (i == 0)
                         v = (j == 0) ? cd(1.0, 0.0) : cd(0.0, 0.0);
                     else if (j == 0)
-                        v = std::pow(z_par, i) * (-1.0 / i);
+                        v = ipow(z_par, i) * (-1.0 / i);
                     else if (j <= i)
-                        v = std::pow(z_par, i) * binom(i - 1, j - 1) * std::pow(rz_ch, j);
+                        v = ipow(z_par, i) * binom(i - 1, j - 1) * ipow(rz_ch, j);
                 } else {
                     const cd z_par = sgn / 4.0, rz_ch = 2.0 / sgn;  // z0/r1, r2/z0
-                    if (j >= i) v = std::pow(rz_ch, i) * binom(j, i) * std::pow(z_par, j);
+                    if (j >= i) v = ipow(rz_ch, i) * binom(j, i) * ipow(z_par, j);
                 }
-                h[((size_t)cp * n + i) * n + j] = make_double2(v.real(), v.imag());
+                h[((size_t)cp * n + j) * n + i] = make_double2(v.real(), v.imag());
             }
     }
     double2 *d = nullptr;
@@ -1557,27 +1588,49 @@ void make_box_lists(const Tree &T, const LevelStarts &ls, Sel sel, BoxLists &B, 
     });
 }
 
+// Levels of at most this many (child, channel) pairs take the matrix form (a
+// thread per output coefficient) in FP64: the Pascal passes need less than
+// half of its arithmetic, but one thread's passes take their latency whatever
+// the level holds.  The mixed mode keeps the Pascal passes on every level: its
+// FP32 M2L and evaluation round what these passes give, so another order of
+// their sums moves single results by an FP32 rounding.
+constexpr int64_t kShiftMatrixPairs = 40000;
+inline bool shift_matrix(const CauchyProblem &P, int64_t pairs) {
+    return P.p + 1 > 40 || (!P.mixed && pairs <= kShiftMatrixPairs);
+}
+
 inline int pascal_grid(int64_t nthreads) {
     return (int)std::max<int64_t>(1, std::min<int64_t>((nthreads + 127) / 128, kNumSM * 16));
 }
 
 // ---------------------------------------------------------------------------
 // P2M (leaves of levels >= 2 with sources) and P2L (list 4) with one warp
-// per box.  Sources go in chunks of kPowSrc: the chunk's lanes build each
-// source's powers b^k (b = (x - c) / r for P2M, r / (x - c) for P2L) by
-// the same recurrence as the per-box form and stage them with the
-// strengths; then lane k sums coefficient k over the chunk.  P2M stores the
-// multipoles (their first writer), P2L adds to the locals.
-//   P2M: M_0 += q,  M_k += -q z^k / k + (d / r) z^(k-1)
-//   P2L: L_0 += q log|z0| - d / z0,  L_k += -q w^k / k - (d / z0) w^k
+// per box.  The box's sources (P2L: of all its list-4 leaves, one after the
+// other) go in chunks of kPowSrc: four lanes per source build its powers b^k
+// (b = (x - c) / r for P2M, r / (x - c) for P2L), every fourth each, and stage
+// them with the strengths; then lane k sums coefficient k over the chunk,
+// charges and dipoles separately,
+//   Q_k = sum q b^k,   D_k = sum d' b^k   (d' = d / r; P2L: -d / z0),
+// so a power is read once.  The coefficients above 31 are shared out over all
+// lanes, each lane a part of the sources.  P2M stores the multipoles (their
+// first writer), P2L adds to the locals:
+//   P2M: M_0 = Q_0,  M_k = -Q_k / k + D_(k-1)
+//   P2L: L_0 += sum q log|z0| + D_0,  L_k += -Q_k / k + D_k
+// Bound by the shared-memory wavefronts of the powers (four per warp and
+// source) beside the FP64 pipe.  (Two power reads per term, 16-source chunks
+// built by half a warp with a division each, and the coefficients above 31 in
+// a second pass with most lanes idle: 1.57 ms for both at 3e6 points, order
+// 37; 1.81 ms at the 8e6 points of the boundary curve, order 28.)
 // ---------------------------------------------------------------------------
-constexpr int kPowSrc = 16;
+constexpr int kPowSrc = 8;
 constexpr int kPowWarps = 8;
 
+// Row of a source's powers: an odd number of 16-byte words.
+__host__ __device__ inline int pow_row(int p) { return (p + 1) | 1; }
+
 inline size_t pow_warp_smem(int p, int CH) {
-    // per warp: powers [kPowSrc][P], strengths [kPowSrc][2 CH], log|z0| [kPowSrc]
-    return (size_t)kPowWarps * ((size_t)kPowSrc * (p + 1 + 2 * CH) * sizeof(double2) +
-                                (size_t)kPowSrc * sizeof(double));
+    // per warp: powers [kPowSrc][row], strengths [kPowSrc][2 CH]
+    return (size_t)kPowWarps * kPowSrc * (pow_row(p) + 2 * CH) * sizeof(double2);
 }
 
 // Strengths as the passes read them: FP64, or the FP32 copies of the mixed
@@ -1585,105 +1638,172 @@ inline size_t pow_warp_smem(int p, int CH) {
 __device__ __forceinline__ double2 str_d2(double2 v) { return v; }
 __device__ __forceinline__ double2 str_d2(float2 v) { return make_double2(v.x, v.y); }
 
-template <int CH, bool P2L, class S>
-__device__ __forceinline__ void pow_warp_box(int b, int p, int lane, double2 *sPw, double2 *sSt,
-                                             double *sLz, const double2 c, const double r,
-                                             const int2 *rgs, int nrg,
-                                             const double2 *__restrict__ src,
-                                             const S *__restrict__ chg,
-                                             const S *__restrict__ dip, int ifc, int ifd,
-                                             int ndc, int c0, double2 (&acc)[2][CH]) {
-    const int P = p + 1;
-    for (int g = 0; g < nrg; g++) {
-        const int2 rg = rgs[g];
-        for (int j0 = rg.x; j0 < rg.y; j0 += kPowSrc) {
-            const int n = min(kPowSrc, rg.y - j0);
-            __syncwarp();
-            if (lane < n) {
-                const int j = j0 + lane;
-                const double2 x = src[j];
-                double2 base;
-                double2 dv[CH];
-                if (P2L) {
-                    const double2 z0 = make_double2(x.x - c.x, x.y - c.y);
-                    const double2 zi = cinv(z0);
-                    base = cscal(zi, r);  // r / z0
-                    sLz[lane] = 0.5 * log(z0.x * z0.x + z0.y * z0.y);
+// KIND: bit 0 charges, bit 1 dipoles; LAPR: the charges are real.  out[h][q]:
+// coefficient lane + 32 h of channel q (h = 1: lanes below p - 31).
+template <int CH, bool P2L, class S, int KIND, bool LAPR>
+__device__ __forceinline__ void pow_warp_box(int p, int lane, double2 *sPw, double2 *sSt,
+                                             const double2 c, const double r, const int2 *rgs,
+                                             int nrg, const double2 *__restrict__ src,
+                                             const S *__restrict__ chg, const S *__restrict__ dip,
+                                             int ndc, int c0, double2 (&out)[2][CH]) {
+    constexpr bool IFC = (KIND & 1) != 0, IFD = (KIND & 2) != 0;
+    const int P = p + 1, row = pow_row(p), NL = P > 32 ? P - 32 : 0;
+    const int sl = lane >> 2, t = lane & 3;          // source and power residue of this lane
+    const int grp = NL ? lane / NL : 0, ngrp = NL ? 32 / NL : 0;
+    const bool left = NL && grp < ngrp;              // a lane of the coefficients above 31
+    const int kl = left ? 32 + lane - grp * NL : 0;
+    double2 Q[2][CH], D[2][CH];
 #pragma unroll
-                    for (int q = 0; q < CH; q++)
-                        dv[q] = ifd ? cscal(cmul(str_d2(dip[(size_t)j * ndc + c0 + q]), zi), -1.0)
-                                    : make_double2(0.0, 0.0);
+    for (int h = 0; h < 2; h++)
+#pragma unroll
+        for (int q = 0; q < CH; q++) Q[h][q] = D[h][q] = make_double2(0.0, 0.0);
+    auto add = [&](double2 (&q_)[CH], double2 (&d_)[CH], const double2 pq, const double2 pd, int s) {
+#pragma unroll
+        for (int q = 0; q < CH; q++) {
+            if (IFC) {
+                const double2 v = sSt[s * 2 * CH + q];
+                if (LAPR) {
+                    q_[q].x = fma(v.x, pq.x, q_[q].x);
+                    q_[q].y = fma(v.x, pq.y, q_[q].y);
                 } else {
-                    base = make_double2((x.x - c.x) / r, (x.y - c.y) / r);
-                    const double rinv = 1.0 / r;
-#pragma unroll
-                    for (int q = 0; q < CH; q++)
-                        dv[q] = ifd ? cscal(str_d2(dip[(size_t)j * ndc + c0 + q]), rinv)
-                                    : make_double2(0.0, 0.0);
-                }
-#pragma unroll
-                for (int q = 0; q < CH; q++) {
-                    sSt[lane * 2 * CH + q] =
-                        ifc ? str_d2(chg[(size_t)j * ndc + c0 + q]) : make_double2(0.0, 0.0);
-                    sSt[lane * 2 * CH + CH + q] = dv[q];
-                }
-                double2 w = make_double2(1.0, 0.0);
-                for (int k = 0; k < P; k++) {
-                    sPw[lane * P + k] = w;
-                    w = cmul(w, base);
+                    cfma(q_[q], v, pq);
                 }
             }
-            __syncwarp();
+            if (IFD) cfma(d_[q], sSt[s * 2 * CH + CH + q], pd);
+        }
+    };
+    int g = 0, j = 0;  // next source: j-th of range g
+    int tot = 0;
+    for (int e = 0; e < nrg; e++) tot += rgs[e].y - rgs[e].x;
+    for (int base = 0; base < tot; base += kPowSrc) {
+        const int n = min(kPowSrc, tot - base);
+        // this lane's source
+        int e = g, o = j + sl;
+        while (e < nrg - 1 && o >= rgs[e].y - rgs[e].x) {
+            o -= rgs[e].y - rgs[e].x;
+            e++;
+        }
+        const int js = rgs[e].x + o;
+        // where the next chunk begins
+        j += n;
+        while (g < nrg - 1 && j >= rgs[g].y - rgs[g].x) {
+            j -= rgs[g].y - rgs[g].x;
+            g++;
+        }
+        __syncwarp();
+        if (sl < n) {
+            const double2 x = src[js];
+            const double zx = x.x - c.x, zy = x.y - c.y;
+            double2 w1, f;  // the power base and the dipoles' factor
+            double lz = 0.0;
+            if (P2L) {
+                const double zz = zx * zx + zy * zy, iz = rcp_any(zz);
+                f = make_double2(-zx * iz, zy * iz);  // -1 / z0
+                w1 = make_double2(-f.x * r, -f.y * r);
+                if (IFC) lz = half_ln_any(zz);
+            } else {
+                const double ri = 1.0 / r;
+                f = make_double2(ri, 0.0);
+                w1 = make_double2(zx * ri, zy * ri);
+            }
+            if (t == 0) {
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int k = lane + 32 * h;
-                if (k >= P) break;
-                const double ik = k > 0 ? -1.0 / k : 0.0;
-                for (int s = 0; s < n; s++) {
-                    const double2 pk = sPw[s * P + k];
-                    // P2M: the dipole term takes z^(k-1); P2L takes w^k
-                    const double2 pd = P2L ? pk : (k > 0 ? sPw[s * P + k - 1] : make_double2(0.0, 0.0));
-                    const double lz = P2L ? sLz[s] : 0.0;
-#pragma unroll
-                    for (int q = 0; q < CH; q++) {
-                        const double2 qv = sSt[s * 2 * CH + q], dv = sSt[s * 2 * CH + CH + q];
-                        if (k == 0)
-                            acc[h][q] = cadd(acc[h][q], P2L ? cscal(qv, lz) : qv);
-                        else
-                            cfma(acc[h][q], qv, cscal(pk, ik));
-                        cfma(acc[h][q], dv, pd);
+                for (int q = 0; q < CH; q++) {
+                    if (IFC) sSt[sl * 2 * CH + q] = str_d2(chg[(size_t)js * ndc + c0 + q]);
+                    if (IFD) {
+                        const double2 dv = str_d2(dip[(size_t)js * ndc + c0 + q]);
+                        sSt[sl * 2 * CH + CH + q] = P2L ? cmul(dv, f) : cscal(dv, f.x);
                     }
                 }
             }
+            const double2 w2 = cmul(w1, w1), w4 = cmul(w2, w2);
+            double2 w = t == 0 ? make_double2(1.0, 0.0) : (t == 1 ? w1 : (t == 2 ? w2 : cmul(w2, w1)));
+            // (P2L: the place of b^0 holds log|z0|, the charges' factor)
+            double2 *pw = sPw + sl * row + t;
+            pw[0] = (P2L && t == 0) ? make_double2(lz, 0.0) : w;
+            for (int k = t + 4; k < P; k += 4) {
+                w = cmul(w, w4);
+                sPw[sl * row + k] = w;
+            }
+        }
+        __syncwarp();
+        if (lane < P)
+            for (int s = 0; s < n; s++) {
+                const double2 pk = sPw[s * row + lane];
+                const double2 pd = P2L && lane == 0 ? make_double2(1.0, 0.0) : pk;
+                add(Q[0], D[0], pk, pd, s);
+            }
+        if (left)
+            for (int s = grp; s < n; s += ngrp) {
+                const double2 pk = sPw[s * row + kl];
+                add(Q[1], D[1], pk, pk, s);
+            }
+    }
+    if (NL) {
+        // the parts of the coefficients above 31, to lanes 0 .. NL - 1
+#pragma unroll
+        for (int q = 0; q < CH; q++) {
+            double2 q1 = Q[1][q], d1 = D[1][q];
+            double2 qs = q1, ds = d1;
+            for (int u = 1; u < ngrp; u++) {
+                const int from = min(31, lane + u * NL);
+                if (IFC) {
+                    qs.x += __shfl_sync(0xffffffffu, q1.x, from);
+                    qs.y += __shfl_sync(0xffffffffu, q1.y, from);
+                }
+                if (IFD) {
+                    ds.x += __shfl_sync(0xffffffffu, d1.x, from);
+                    ds.y += __shfl_sync(0xffffffffu, d1.y, from);
+                }
+            }
+            Q[1][q] = qs;
+            D[1][q] = ds;
+        }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int k = lane + 32 * h;
+        const double ik = k > 0 ? -1.0 / k : 1.0;
+#pragma unroll
+        for (int q = 0; q < CH; q++) {
+            double2 d = D[h][q];
+            if (!P2L && IFD) {  // D_(k-1): the lane below's (lane 31's for k = 32)
+                const double2 lo = make_double2(__shfl_up_sync(0xffffffffu, d.x, 1),
+                                                __shfl_up_sync(0xffffffffu, d.y, 1));
+                const double2 d31 = make_double2(__shfl_sync(0xffffffffu, D[0][q].x, 31),
+                                                 __shfl_sync(0xffffffffu, D[0][q].y, 31));
+                d = lane > 0 ? lo : (h == 1 ? d31 : make_double2(0.0, 0.0));
+            }
+            double2 v = make_double2(0.0, 0.0);
+            if (IFC) v = cscal(Q[h][q], ik);
+            if (IFD) v = cadd(v, d);
+            out[h][q] = v;
         }
     }
 }
 
-template <int CH>
+// ids / nids (optional): the leaves with sources (only those are visited).
+template <int CH, int KIND, bool LAPR>
 __global__ void __launch_bounds__(kPowWarps * 32) p2m_warp_kernel(
-    int lo, int hi, int p, const int *__restrict__ nchild, const double2 *__restrict__ centers,
+    int lo, int hi, const int *__restrict__ ids, const int *__restrict__ nids, int p,
+    const int *__restrict__ nchild, const double2 *__restrict__ centers,
     const int *__restrict__ level, const double *__restrict__ bs, const int2 *__restrict__ sse,
     const double2 *__restrict__ src, const double2 *__restrict__ chg,
-    const double2 *__restrict__ dip, int ifc, int ifd, int ndc, int c0,
-    double2 *__restrict__ mp) {
+    const double2 *__restrict__ dip, int ndc, int c0, double2 *__restrict__ mp) {
     extern __shared__ double2 pow_smem[];
     const int P = p + 1, stride = P * ndc;
     const int lane = lane_id(), wib = threadIdx.x >> 5;
-    double2 *sPw = pow_smem + (size_t)wib * kPowSrc * (P + 2 * CH);
-    double2 *sSt = sPw + kPowSrc * P;
-    double *sLz = reinterpret_cast<double *>(pow_smem + (size_t)kPowWarps * kPowSrc * (P + 2 * CH)) +
-                  wib * kPowSrc;
-    for (int b = lo + warp_global(); b < hi; b += warp_count()) {
+    double2 *sPw = pow_smem + (size_t)wib * kPowSrc * (pow_row(p) + 2 * CH);
+    double2 *sSt = sPw + kPowSrc * pow_row(p);
+    const int k0 = ids ? 0 : lo, k1 = ids ? *nids : hi;
+    for (int kb = k0 + warp_global(); kb < k1; kb += warp_count()) {
+        const int b = ids ? ids[kb] : kb;
         if (nchild[b] != 0) continue;
         const int2 rg = sse[b];
         if (rg.y <= rg.x) continue;
         double2 acc[2][CH];
-#pragma unroll
-        for (int h = 0; h < 2; h++)
-#pragma unroll
-            for (int q = 0; q < CH; q++) acc[h][q] = make_double2(0.0, 0.0);
-        pow_warp_box<CH, false, double2>(b, p, lane, sPw, sSt, sLz, centers[b], bs[level[b]], &rg, 1, src,
-                                chg, dip, ifc, ifd, ndc, c0, acc);
+        pow_warp_box<CH, false, double2, KIND, LAPR>(p, lane, sPw, sSt, centers[b], bs[level[b]], &rg,
+                                                     1, src, chg, dip, ndc, c0, acc);
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             const int k = lane + 32 * h;
@@ -1812,25 +1932,21 @@ __global__ void __launch_bounds__(kPowWarps * 32) p2m_warp32_kernel(
 }
 
 // S: the strengths' type (FP64, or the mixed mode's FP32 copies).
-// ids / off (optional): the boxes with list-4 entries and evaluation
-// points in box order, entries ids[off[lo] .. off[hi]) (only those are
-// visited).
-template <int CH, class S>
+// ids / nids (optional): the boxes with list-4 entries and evaluation points
+// (only those are visited).
+template <int CH, class S, int KIND, bool LAPR>
 __global__ void __launch_bounds__(kPowWarps * 32) p2l_warp_kernel(
     int lo, int hi, const int *__restrict__ ids, const int *__restrict__ nids, int p,
     EvalCounts ec, const int *__restrict__ nlist4,
     const int *__restrict__ list4, const double2 *__restrict__ centers,
     const int *__restrict__ level, const double *__restrict__ bs,
     const double2 *__restrict__ src, const S *__restrict__ chg,
-    const S *__restrict__ dip, int ifc, int ifd, int ndc, int c0,
-    double2 *__restrict__ loc) {
+    const S *__restrict__ dip, int ndc, int c0, double2 *__restrict__ loc) {
     extern __shared__ double2 pow_smem[];
     const int P = p + 1, stride = P * ndc;
     const int lane = lane_id(), wib = threadIdx.x >> 5;
-    double2 *sPw = pow_smem + (size_t)wib * kPowSrc * (P + 2 * CH);
-    double2 *sSt = sPw + kPowSrc * P;
-    double *sLz = reinterpret_cast<double *>(pow_smem + (size_t)kPowWarps * kPowSrc * (P + 2 * CH)) +
-                  wib * kPowSrc;
+    double2 *sPw = pow_smem + (size_t)wib * kPowSrc * (pow_row(p) + 2 * CH);
+    double2 *sSt = sPw + kPowSrc * pow_row(p);
     const int k0 = ids ? 0 : lo, k1 = ids ? *nids : hi;
     for (int kb = k0 + warp_global(); kb < k1; kb += warp_count()) {
         const int b = ids ? ids[kb] : kb;
@@ -1839,12 +1955,8 @@ __global__ void __launch_bounds__(kPowWarps * 32) p2l_warp_kernel(
         int2 rgs[kMaxList4];
         for (int e = 0; e < n4; e++) rgs[e] = ec.sse[list4[kMaxList4 * b + e]];
         double2 acc[2][CH];
-#pragma unroll
-        for (int h = 0; h < 2; h++)
-#pragma unroll
-            for (int q = 0; q < CH; q++) acc[h][q] = make_double2(0.0, 0.0);
-        pow_warp_box<CH, true, S>(b, p, lane, sPw, sSt, sLz, centers[b], bs[level[b]], rgs, n4,
-                                  src, chg, dip, ifc, ifd, ndc, c0, acc);
+        pow_warp_box<CH, true, S, KIND, LAPR>(p, lane, sPw, sSt, centers[b], bs[level[b]], rgs, n4,
+                                              src, chg, dip, ndc, c0, acc);
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             const int k = lane + 32 * h;
@@ -1856,6 +1968,20 @@ __global__ void __launch_bounds__(kPowWarps * 32) p2l_warp_kernel(
             }
         }
     }
+}
+
+// Calls f(std::integral_constant kind, std::bool_constant lapr) for the
+// strengths present.
+template <class F>
+inline void pow_kinds(const CauchyProblem &P, F f) {
+    typedef std::integral_constant<int, 1> C;
+    typedef std::integral_constant<int, 2> Dp;
+    typedef std::integral_constant<int, 3> CD;
+    if (!P.ifcharge) f(Dp{}, std::false_type{});
+    else if (P.ifdipole && P.real_charge) f(CD{}, std::true_type{});
+    else if (P.ifdipole) f(CD{}, std::false_type{});
+    else if (P.real_charge) f(C{}, std::true_type{});
+    else f(C{}, std::false_type{});
 }
 
 inline int pow_grid(int nbox) {
@@ -1898,11 +2024,13 @@ void upward_chunk(const Tree &T, const CauchyProblem &P, int c0,
                 launch(p2m_warp32_kernel<CH, double2, false>, P.dipstr);
         } else if (warpk) {
             const size_t sm = pow_warp_smem(p, CH);
-            raise_smem_limit(p2m_warp_kernel<CH>, (int)sm);
-            p2m_warp_kernel<CH><<<pow_grid(nb - lo), kPowWarps * 32, sm, s>>>(
-                lo, nb, p, T.nchild.get(), T.centers.get(), T.level.get(), bs,
-                T.srcse.get(), P.src, P.charge, P.dipstr, P.ifcharge, P.ifdipole,
-                P.ndc, c0, mp);
+            pow_kinds(P, [&](auto kind, auto lapr) {
+                auto kern = p2m_warp_kernel<CH, decltype(kind)::value, decltype(lapr)::value>;
+                raise_smem_limit(kern, sm);
+                kern<<<pow_grid(nb - lo), kPowWarps * 32, sm, s>>>(
+                    lo, nb, P.p2m_ids, P.p2m_cnt, p, T.nchild.get(), T.centers.get(), T.level.get(),
+                    bs, T.srcse.get(), P.src, P.charge, P.dipstr, P.ndc, c0, mp);
+            });
         } else
             p2m_coef_kernel<CH><<<blocks(nb - lo), 256, 0, s>>>(
                 lo, nb, p, T.nchild.get(), T.centers.get(), T.level.get(), bs,
@@ -1917,7 +2045,11 @@ void upward_chunk(const Tree &T, const CauchyProblem &P, int c0,
         const int64_t nt = (int64_t)(hi - lo) * CH * 4;
         const int *ids = P.m2m_ids ? P.m2m_ids + lo : nullptr;
         const int *nid = P.m2m_ids ? P.m2m_cnt + l : nullptr;
-        if (p + 1 <= 20)
+        if (shift_matrix(P, nt))
+            m2m_coef_kernel<CH><<<blocks(4 * (hi - lo)), 256, 0, s>>>(
+                lo, hi, p, ids, nid, T.nchild.get(), T.child.get(), T.srcse.get(), A, P.ndc,
+                c0, mp);
+        else if (p + 1 <= 20)
             m2m_pascal_kernel<20><<<pascal_grid(nt), 128, 0, s>>>(
                 lo, hi, p, ids, nid, T.nchild.get(), T.child.get(), T.srcse.get(),
                 P.ndc, c0, CH, mp);
@@ -1925,14 +2057,10 @@ void upward_chunk(const Tree &T, const CauchyProblem &P, int c0,
             m2m_pascal_kernel<32><<<pascal_grid(nt), 128, 0, s>>>(
                 lo, hi, p, ids, nid, T.nchild.get(), T.child.get(), T.srcse.get(),
                 P.ndc, c0, CH, mp);
-        else if (p + 1 <= 40)
+        else
             m2m_pascal_kernel<40><<<pascal_grid(nt), 128, 0, s>>>(
                 lo, hi, p, ids, nid, T.nchild.get(), T.child.get(), T.srcse.get(),
                 P.ndc, c0, CH, mp);
-        else
-            m2m_coef_kernel<CH><<<blocks(hi - lo), 256, 0, s>>>(
-                lo, hi, p, T.nchild.get(), T.child.get(), T.srcse.get(), A, P.ndc,
-                c0, mp);
         FMM_CHECK_LAUNCH();
     }
     prof_mark("m2m", s);
@@ -1976,21 +2104,23 @@ void downward_chunk(const Tree &T, const CauchyProblem &P, int c0,
     const bool warpk = p + 1 <= 40;
     if (L >= 2) {
         const int lo = T.lstart[2];
-        if (warpk && P.mixed && (P.charge32 || !P.ifcharge) && (P.dipstr32 || !P.ifdipole)) {
-            // the FP32 copies of the strengths (the FP64 ones may be absent)
+        // (in the mixed mode from the FP32 copies of the strengths, since the
+        // FP64 ones may be absent)
+        const bool s32 = P.mixed && (P.charge32 || !P.ifcharge) && (P.dipstr32 || !P.ifdipole);
+        if (warpk) {
             const size_t sm = pow_warp_smem(p, CH);
-            raise_smem_limit(p2l_warp_kernel<CH, float2>, (int)sm);
-            p2l_warp_kernel<CH, float2><<<pow_grid(nb - lo), kPowWarps * 32, sm, s>>>(
-                lo, nb, P.p2l_ids, P.p2l_cnt, p, ec, T.nlist4.get(), T.list4.get(), T.centers.get(),
-                T.level.get(), bs, P.src, P.charge32, P.dipstr32, P.ifcharge,
-                P.ifdipole, P.ndc, c0, loc);
-        } else if (warpk) {
-            const size_t sm = pow_warp_smem(p, CH);
-            raise_smem_limit(p2l_warp_kernel<CH, double2>, (int)sm);
-            p2l_warp_kernel<CH, double2><<<pow_grid(nb - lo), kPowWarps * 32, sm, s>>>(
-                lo, nb, P.p2l_ids, P.p2l_cnt, p, ec, T.nlist4.get(), T.list4.get(), T.centers.get(),
-                T.level.get(), bs, P.src, P.charge, P.dipstr, P.ifcharge,
-                P.ifdipole, P.ndc, c0, loc);
+            pow_kinds(P, [&](auto kind, auto lapr) {
+                constexpr int K = decltype(kind)::value;
+                constexpr bool R = decltype(lapr)::value;
+                auto launch = [&](auto kern, const auto *chg, const auto *dip) {
+                    raise_smem_limit(kern, sm);
+                    kern<<<pow_grid(nb - lo), kPowWarps * 32, sm, s>>>(
+                        lo, nb, P.p2l_ids, P.p2l_cnt, p, ec, T.nlist4.get(), T.list4.get(),
+                        T.centers.get(), T.level.get(), bs, P.src, chg, dip, P.ndc, c0, loc);
+                };
+                if (s32) launch(p2l_warp_kernel<CH, float2, K, R>, P.charge32, P.dipstr32);
+                else launch(p2l_warp_kernel<CH, double2, K, R>, P.charge, P.dipstr);
+            });
         } else
             p2l_coef_kernel<CH><<<blocks(nb - lo), 256, 0, s>>>(
                 lo, nb, p, ec, T.nlist4.get(), T.list4.get(), T.centers.get(),
@@ -2006,7 +2136,10 @@ void downward_chunk(const Tree &T, const CauchyProblem &P, int c0,
         const int64_t nt = (int64_t)(hi - lo) * CH;
         const int *ids = P.l2l_ids ? P.l2l_ids + lo : nullptr;
         const int *nid = P.l2l_ids ? P.l2l_cnt + l + 1 : nullptr;
-        if (p + 1 <= 20)
+        if (shift_matrix(P, nt))
+            l2l_coef_kernel<CH><<<blocks(hi - lo), 256, 0, s>>>(
+                lo, hi, p, ec, ids, nid, T.parent.get(), T.child.get(), A, P.ndc, c0, loc, loc32);
+        else if (p + 1 <= 20)
             l2l_pascal_kernel<20><<<pascal_grid(nt), 128, 0, s>>>(
                 lo, hi, p, ec, ids, nid, T.parent.get(), T.child.get(), P.ndc, c0,
                 CH, loc, loc32);
@@ -2014,13 +2147,10 @@ void downward_chunk(const Tree &T, const CauchyProblem &P, int c0,
             l2l_pascal_kernel<32><<<pascal_grid(nt), 128, 0, s>>>(
                 lo, hi, p, ec, ids, nid, T.parent.get(), T.child.get(), P.ndc, c0,
                 CH, loc, loc32);
-        else if (p + 1 <= 40)
+        else
             l2l_pascal_kernel<40><<<pascal_grid(nt), 128, 0, s>>>(
                 lo, hi, p, ec, ids, nid, T.parent.get(), T.child.get(), P.ndc, c0,
                 CH, loc, loc32);
-        else
-            l2l_coef_kernel<CH><<<blocks(hi - lo), 256, 0, s>>>(
-                lo, hi, p, ec, T.parent.get(), T.child.get(), A, P.ndc, c0, loc);
         FMM_CHECK_LAUNCH();
     }
     prof_mark("l2l", s);
@@ -2222,20 +2352,17 @@ void cauchy_fmm(const Tree &T, const CauchyProblem &P0, cudaStream_t s) {
         const EvalCounts ec{T.srcse.get(), T.trgse.get(), P.sset.pgh, P.tset.pgh};
         LevelStarts ls{};
         for (int l = 0; l <= T.nlevels; l++) ls.v[l] = T.lstart[l];
-        const bool mixed = P.mixed;
         make_box_lists(T, ls, [=] __device__(int b) -> unsigned {
             const bool src = count(sse, b) > 0, pts = ec.npts(b) > 0, leaf = nchp[b] == 0;
-            return (!leaf && src ? 1u : 0u) | (pts ? 2u : 0u) | (mixed && leaf && src ? 4u : 0u) |
+            return (!leaf && src ? 1u : 0u) | (pts ? 2u : 0u) | (leaf && src ? 4u : 0u) |
                    (n4p[b] > 0 && pts ? 8u : 0u);
         }, lists, s);
         P.m2m_ids = lists.ids[0].get();
         P.l2l_ids = lists.ids[1].get();
         P.m2m_cnt = lists.count(0, 0);
         P.l2l_cnt = lists.count(1, 0);
-        if (mixed) {
-            P.p2m_ids = lists.ids[2].get();
-            P.p2m_cnt = lists.count(2, 0);
-        }
+        P.p2m_ids = lists.ids[2].get();
+        P.p2m_cnt = lists.count(2, 0);
         P.p2l_ids = lists.ids[3].get();
         P.p2l_cnt = lists.count(3, 0);
     }

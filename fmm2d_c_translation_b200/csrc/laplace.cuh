@@ -83,7 +83,7 @@ struct CauchyProblem {
     M2LCache *m2l_cache = nullptr;    // planning kept across evaluations (plans)
     // boxes visited by the Pascal M2M (parents with sources) and L2L (boxes
     // with evaluation points): level l's at ids + lstart[l], cnt[l] of them;
-    // by the mixed mode's P2M (leaves with sources) and the P2L (boxes with
+    // by the P2M (leaves with sources) and the P2L (boxes with
     // list-4 entries and evaluation points): ids, *cnt of them (set by
     // cauchy_fmm; the order within a level is arbitrary)
     const int *m2m_ids = nullptr, *m2m_cnt = nullptr;

@@ -68,4 +68,13 @@ __device__ __forceinline__ double half_ln_pos(double x) {
     return fma(q, u, fma((double)e, 0.34657359027997265471, c.y));
 }
 
+// The same for any number, outside the inner loops.
+__device__ __forceinline__ bool is_normal_pos(double x) { return x >= 2.3e-308 && x <= 1e307; }
+__device__ __forceinline__ double rcp_any(double x) {
+    return is_normal_pos(x) ? rcp_pos(x) : 1.0 / x;
+}
+__device__ __forceinline__ double half_ln_any(double x) {
+    return is_normal_pos(x) ? half_ln_pos(x) : 0.5 * log(x);
+}
+
 }  // namespace fmm2d
