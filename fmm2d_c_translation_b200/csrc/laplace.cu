@@ -212,6 +212,15 @@ template <class T2, class T> __device__ __forceinline__ T2 zscal(T2 a, T s) {
     r.y = a.y * s;
     return r;
 }
+// a b + c: in FP64 four fused operations (the FP32 passes keep the rounding of
+// a product and a sum)
+__device__ __forceinline__ float2 zmadd(float2 a, float2 b, float2 c) {
+    const float2 m = make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+    return make_float2(m.x + c.x, m.y + c.y);
+}
+__device__ __forceinline__ double2 zmadd(double2 a, double2 b, double2 c) {
+    return make_double2(fma(a.x, b.x, fma(-a.y, b.y, c.x)), fma(a.x, b.y, fma(a.y, b.x, c.y)));
+}
 template <class T2> __device__ __forceinline__ T2 zadd(T2 a, T2 b) {
     T2 r;
     r.x = a.x + b.x;
@@ -560,20 +569,29 @@ __device__ __forceinline__ void far_field_box(int b, int ntb, int2 tr, int2 sr0,
             const double r = fa.bs[fa.level[jb]];
             const double zx = x.x - cj.x, zy = x.y - cj.y;
             const double zz = zx * zx + zy * zy;
-            const R2 zi = mk2<R2>(zx / zz, -zy / zz);         // 1/z
-            const R2 w = mk2<R2>(r * zx / zz, -r * zy / zz);  // r/z
-            const R lz = (R)0.5 * Real<MIXED>::log_((R)zz);
+            R2 zi, w;  // 1/z, r/z
+            R lz;
+            if constexpr (MIXED) {
+                zi = mk2<R2>(zx / zz, -zy / zz);
+                w = mk2<R2>(r * zx / zz, -r * zy / zz);
+                lz = (R)0.5 * Real<MIXED>::log_((R)zz);
+            } else {
+                const double iz = rcp_any(zz);
+                zi = mk2<R2>(zx * iz, -zy * iz);
+                w = zscal(zi, r);
+                lz = half_ln_any(zz);
+            }
             const R rinv = (R)(1.0 / r);
 #pragma unroll
             for (int q = 0; q < CH; q++) {
                 R2 q0 = s_mp[p * CH + q], q1 = mk2<R2>(0.0, 0.0), q2 = mk2<R2>(0.0, 0.0);
                 for (int m = p - 1; m >= 1; m--) {
-                    if (PGH >= 3) q2 = zadd(zmul(q2, w), q1);
-                    if (PGH >= 2) q1 = zadd(zmul(q1, w), q0);
-                    q0 = zadd(zmul(q0, w), s_mp[m * CH + q]);
+                    if (PGH >= 3) q2 = zmadd(q2, w, q1);
+                    if (PGH >= 2) q1 = zmadd(q1, w, q0);
+                    q0 = zmadd(q0, w, s_mp[m * CH + q]);
                 }
-                if (PGH >= 3) q2 = zadd(zmul(q2, w), q1);
-                if (PGH >= 2) q1 = zadd(zmul(q1, w), q0);
+                if (PGH >= 3) q2 = zmadd(q2, w, q1);
+                if (PGH >= 2) q1 = zmadd(q1, w, q0);
                 q0 = zmul(q0, w);
                 const R2 M0 = s_mp[q];
                 po[q] = zadd(po[q], zadd(zscal(M0, lz), q0));
@@ -599,9 +617,9 @@ __device__ __forceinline__ void far_field_box(int b, int ntb, int2 tr, int2 sr0,
             for (int q = 0; q < CH; q++) {
                 R2 q0 = s_loc[p * CH + q], q1 = mk2<R2>(0.0, 0.0), q2 = mk2<R2>(0.0, 0.0);
                 for (int m = p - 1; m >= 0; m--) {
-                    if (PGH >= 3) q2 = zadd(zmul(q2, z), q1);
-                    if (PGH >= 2) q1 = zadd(zmul(q1, z), q0);
-                    q0 = zadd(zmul(q0, z), s_loc[m * CH + q]);
+                    if (PGH >= 3) q2 = zmadd(q2, z, q1);
+                    if (PGH >= 2) q1 = zmadd(q1, z, q0);
+                    q0 = zmadd(q0, z, s_loc[m * CH + q]);
                 }
                 po[q] = zadd(po[q], q0);
                 if (PGH >= 2) gr[q] = zadd(gr[q], zscal(q1, rinv));
