@@ -727,13 +727,62 @@ __device__ __forceinline__ void p2p_pair(const typename PosT<MIXED>::T &x,
     }
 }
 
-// Strength slots per warp of p2p_kernel: the staged strengths, or the
-// 32 lanes' group sums (3 CH values each) when those are more.
-template <int CH, bool IFC, bool IFD>
+// A warp's staged strengths: the charges of kP2PStage sources, then their
+// dipoles.  The two real charges of a complex-Laplace density share one
+// complex slot, and in FP32 two slots are read as one 16-byte word: a pair
+// reads 3 (FP64: 4) words of shared memory instead of 5, whose wavefronts
+// bound the FP64 form (LSU 65 %, FP64 pipe 45 % busy).
+template <int CH, bool IFC, bool IFD, bool LAPR, class R2>
+struct Strengths {
+    static constexpr bool kPair = LAPR && CH == 2;  // charges of a source in one slot
+    static constexpr int kC = IFC ? (kPair ? 1 : CH) : 0, kD = IFD ? CH : 0;
+    static constexpr int kSlots = kP2PStage * (kC + kD);
+    static __device__ __forceinline__ void stage(R2 *s, int i, const R2 *chg, const R2 *dip,
+                                                 size_t o) {
+        if (IFC && kPair) {
+            s[i] = mk2<R2>(chg[o].x, chg[o + 1].x);
+        } else if (IFC) {
+#pragma unroll
+            for (int q = 0; q < CH; q++) s[i * CH + q] = chg[o + q];
+        }
+        if (IFD)
+#pragma unroll
+            for (int q = 0; q < CH; q++) s[kP2PStage * kC + i * CH + q] = dip[o + q];
+    }
+    // CH consecutive slots (s 16-byte aligned, i a multiple of CH)
+    static __device__ __forceinline__ void slots(const double2 *s, int i, double2 *v) {
+#pragma unroll
+        for (int q = 0; q < CH; q++) v[q] = s[i + q];
+    }
+    static __device__ __forceinline__ void slots(const float2 *s, int i, float2 *v) {
+        if (CH == 2) {
+            const float4 w = *reinterpret_cast<const float4 *>(s + i);
+            v[0] = make_float2(w.x, w.y);
+            v[CH - 1] = make_float2(w.z, w.w);
+        } else {
+#pragma unroll
+            for (int q = 0; q < CH; q++) v[q] = s[i + q];
+        }
+    }
+    // source i's strengths as p2p_pair takes them
+    static __device__ __forceinline__ void load(const R2 *s, int i, R2 *v) {
+        if (IFC && kPair) {
+            const R2 c = s[i];
+            v[0] = mk2<R2>(c.x, 0.0);
+            v[CH - 1] = mk2<R2>(c.y, 0.0);
+        } else if (IFC) {
+            slots(s, i * CH, v);
+        }
+        if (IFD) slots(s + kP2PStage * kC, i * CH, v + (IFC ? CH : 0));
+    }
+};
+
+// Slots per warp of p2p_kernel: the staged strengths, or the 32 lanes' group
+// sums (3 CH values each) when those are more.
+template <int CH, bool IFC, bool IFD, bool LAPR>
 constexpr int p2p_str_slots() {
-    return kP2PStage * ((IFC ? CH : 0) + (IFD ? CH : 0)) > 32 * 3 * CH
-               ? kP2PStage * ((IFC ? CH : 0) + (IFD ? CH : 0))
-               : 32 * 3 * CH;
+    constexpr int k = Strengths<CH, IFC, IFD, LAPR, double2>::kSlots;
+    return k > 32 * 3 * CH ? k : 32 * 3 * CH;
 }
 
 template <int CH, int PGH, bool IFC, bool IFD, bool MIXED, bool LAPR>
@@ -750,11 +799,11 @@ __global__ void __launch_bounds__(kP2PWarps * 32) p2p_kernel(
     typedef typename Real<MIXED>::T R;
     typedef typename Real<MIXED>::T2 R2;
     typedef typename PosT<MIXED>::T PT;
-    constexpr int kStr = (IFC ? CH : 0) + (IFD ? CH : 0);
-    constexpr int kRed = 3 * CH;
+    typedef Strengths<CH, IFC, IFD, LAPR, R2> Str;
+    constexpr int kNS = (IFC ? CH : 0) + (IFD ? CH : 0), kRed = 3 * CH;
     // the strengths' slots double as the 32 lanes' group sums (kRed values
     // each), so they hold the larger of the two
-    constexpr int kStrSlots = p2p_str_slots<CH, IFC, IFD>();
+    constexpr int kStrSlots = p2p_str_slots<CH, IFC, IFD, LAPR>();
     constexpr int kWarpBytes = kP2PStage * 16 + kStrSlots * (int)sizeof(R2);
     extern __shared__ __align__(16) unsigned char p2p_smem[];
     const int lane = lane_id(), wib = threadIdx.x >> 5;
@@ -830,18 +879,22 @@ __global__ void __launch_bounds__(kP2PWarps * 32) p2p_kernel(
                                   __shfl_sync(0xffffffffu, jofs, e);
                     if (i >= nst) continue;
                     s_pos[i] = src[k];
-#pragma unroll
-                    for (int q = 0; q < CH; q++) {
-                        if (IFC) s_str[i * kStr + q] = chg[(size_t)k * ndc + c0 + q];
-                        if (IFD) s_str[i * kStr + (IFC ? CH : 0) + q] = dip[(size_t)k * ndc + c0 + q];
-                    }
+                    Str::stage(s_str, i, chg, dip, (size_t)k * ndc + c0);
                 }
                 __syncwarp();
                 if (act) {
 #pragma unroll 4
-                    for (int kk = g; kk < nst; kk += G)
-                        p2p_pair<CH, PGH, IFC, IFD, MIXED, LAPR, true>(x, s_pos[kk], s_str + kk * kStr,
-                                                                 th2, po, gr, he);
+                    for (int kk = g; kk < nst; kk += G) {
+                        // (unpacked FP64 strengths are read where they lie)
+                        R2 st[kNS];
+                        const R2 *sp = s_str + kk * kNS;
+                        if (MIXED || IFC) {
+                            Str::load(s_str, kk, st);
+                            sp = st;
+                        }
+                        p2p_pair<CH, PGH, IFC, IFD, MIXED, LAPR, true>(x, s_pos[kk], sp, th2, po,
+                                                                       gr, he);
+                    }
                 }
             }
             // sum the lane groups
@@ -895,11 +948,12 @@ template <bool MIXED> struct FlatItems { static constexpr int value = MIXED ? 96
 template <int CH, int PGH>
 constexpr int flat_outputs() { return CH * (1 + (PGH >= 2 ? 1 : 0) + (PGH >= 3 ? 1 : 0)); }
 
-template <int CH, int PGH, bool IFC, bool IFD, bool MIXED>
+template <int CH, int PGH, bool IFC, bool IFD, bool MIXED, bool LAPR>
 constexpr size_t p2p_flat_warp_bytes() {
-    return (size_t)kP2PStage * (16 + ((IFC ? CH : 0) + (IFD ? CH : 0)) * sizeof(typename Real<MIXED>::T2)) +
+    typedef typename Real<MIXED>::T2 R2;
+    return (size_t)kP2PStage * 16 + Strengths<CH, IFC, IFD, LAPR, R2>::kSlots * sizeof(R2) +
            32 * 16 + (size_t)FlatItems<MIXED>::value * flat_outputs<CH, PGH>() *
-                          sizeof(typename Real<MIXED>::T2);
+                          sizeof(R2);
 }
 
 template <int CH, int PGH, bool IFC, bool IFD, bool MIXED, bool LAPR>
@@ -916,15 +970,16 @@ __global__ void __launch_bounds__(kP2PWarps * 32) p2p_flat_kernel(
     typedef typename Real<MIXED>::T R;
     typedef typename Real<MIXED>::T2 R2;
     typedef typename PosT<MIXED>::T PT;
-    constexpr int kStr = (IFC ? CH : 0) + (IFD ? CH : 0);
+    typedef Strengths<CH, IFC, IFD, LAPR, R2> Str;
+    constexpr int kNS = (IFC ? CH : 0) + (IFD ? CH : 0);
     constexpr int kNo = flat_outputs<CH, PGH>();
     constexpr int kItems = FlatItems<MIXED>::value;
-    constexpr size_t kWarpBytes = p2p_flat_warp_bytes<CH, PGH, IFC, IFD, MIXED>();
+    constexpr size_t kWarpBytes = p2p_flat_warp_bytes<CH, PGH, IFC, IFD, MIXED, LAPR>();
     extern __shared__ __align__(16) unsigned char p2p_smem[];
     const int lane = lane_id(), wib = threadIdx.x >> 5;
     PT *s_pos = reinterpret_cast<PT *>(p2p_smem + (size_t)wib * kWarpBytes);
     R2 *s_str = reinterpret_cast<R2 *>(s_pos + kP2PStage);
-    PT *s_tgt = reinterpret_cast<PT *>(s_str + kP2PStage * kStr);
+    PT *s_tgt = reinterpret_cast<PT *>(s_str + Str::kSlots);
     R2 *part = reinterpret_cast<R2 *>(s_tgt + 32);
     const R th2 = MIXED ? (R)fmax(th2d, 1.1754943508222875e-38) : (R)th2d;
     for (int b = lo + warp_global(); b < hi; b += warp_count()) {
@@ -988,11 +1043,7 @@ __global__ void __launch_bounds__(kP2PWarps * 32) p2p_flat_kernel(
                                   __shfl_sync(0xffffffffu, jofs, e);
                     if (i >= nst) continue;
                     s_pos[i] = src[k];
-#pragma unroll
-                    for (int q = 0; q < CH; q++) {
-                        if (IFC) s_str[i * kStr + q] = chg[(size_t)k * ndc + c0 + q];
-                        if (IFD) s_str[i * kStr + (IFC ? CH : 0) + q] = dip[(size_t)k * ndc + c0 + q];
-                    }
+                    Str::stage(s_str, i, chg, dip, (size_t)k * ndc + c0);
                 }
                 __syncwarp();
                 const int sb = (nst + B - 1) / B;
@@ -1004,9 +1055,12 @@ __global__ void __launch_bounds__(kP2PWarps * 32) p2p_flat_kernel(
                     for (int q = 0; q < CH; q++) apo[q] = agr[q] = ahe[q] = mk2<R2>(0.0, 0.0);
                     const int j0 = blk * sb, j1 = min(nst, j0 + sb);
 #pragma unroll 4
-                    for (int kk = j0; kk < j1; kk++)
-                        p2p_pair<CH, PGH, IFC, IFD, MIXED, LAPR, false>(x, s_pos[kk], s_str + kk * kStr,
-                                                                 th2, apo, agr, ahe);
+                    for (int kk = j0; kk < j1; kk++) {
+                        R2 st[kNS];
+                        Str::load(s_str, kk, st);
+                        p2p_pair<CH, PGH, IFC, IFD, MIXED, LAPR, false>(x, s_pos[kk], st, th2, apo, agr,
+                                                                 ahe);
+                    }
                     R2 *pp = part + (size_t)i * kNo;
 #pragma unroll
                     for (int q = 0; q < CH; q++) {
@@ -1048,10 +1102,10 @@ __global__ void __launch_bounds__(kP2PWarps * 32) p2p_flat_kernel(
     }
 }
 
-template <int CH, bool IFC, bool IFD, bool MIXED>
+template <int CH, bool IFC, bool IFD, bool MIXED, bool LAPR>
 constexpr size_t p2p_smem_bytes() {
     return (size_t)kP2PWarps * ((size_t)kP2PStage * 16 +
-                                (size_t)p2p_str_slots<CH, IFC, IFD>() * sizeof(typename Real<MIXED>::T2));
+                                (size_t)p2p_str_slots<CH, IFC, IFD, LAPR>() * sizeof(typename Real<MIXED>::T2));
 }
 
 int grid_for(int nwarps) {
@@ -1088,14 +1142,14 @@ void launch_p2p_t(const Tree &T, const CauchyProblem &P, int c0, double th2,
     do {                                                                        \
         if (flat) {                                                             \
             constexpr size_t sm =                                               \
-                kP2PWarps * p2p_flat_warp_bytes<CH, PGH, IFC, IFD, MIXED>();    \
+                kP2PWarps * p2p_flat_warp_bytes<CH, PGH, IFC, IFD, MIXED, LAPR>();    \
             auto kern = p2p_flat_kernel<CH, PGH, IFC, IFD, MIXED, LAPR>;        \
             raise_smem_limit(kern, sm);                                         \
             kern<<<g, kP2PWarps * 32, sm, s>>>(lo, hi, n1, l1, nc, leaves, sse, \
                                               spos, chg, dip, P.sset, P.tset,   \
                                               spos, tpos, P.ndc, c0, th2);      \
         } else {                                                                \
-            constexpr size_t sm = p2p_smem_bytes<CH, IFC, IFD, MIXED>();        \
+            constexpr size_t sm = p2p_smem_bytes<CH, IFC, IFD, MIXED, LAPR>();        \
             auto kern = p2p_kernel<CH, PGH, IFC, IFD, MIXED, LAPR>;             \
             raise_smem_limit(kern, sm);                                         \
             kern<<<g, kP2PWarps * 32, sm, s>>>(lo, hi, n1, l1, nc, leaves, sse, \
