@@ -30,6 +30,7 @@
 #include <mutex>
 #include <stdlib.h>
 #include <string.h>
+#include <type_traits>
 #include <vector>
 
 namespace fmm2d {
@@ -525,27 +526,30 @@ __global__ void __launch_bounds__(kFp32Tile) m2l_fp32_kernel(
 }
 
 // The leading NR rows (local coefficients) of the same sums, which the
-// tensor-core forms recompute in FP32 (see the end of m2l_fp32): one thread
-// per (box, row), so the 27 slots' matrices of the rows fit into shared
-// memory at once and a thread's chain is its row's terms alone; every
-// accumulator adds the same terms in the same order as m2l_fp32_kernel's.
-// Bound by the latency of the source rows' loads.  (With a thread per box and
-// the matrices staged slot by slot, a tile took 79 us whatever it held.)
-constexpr int kRowsTile = 32;
+// tensor-core form leaves to FP32 (see the end of m2l_fp32): one thread per
+// (box, row), so the 27 slots' matrices of the rows fit into shared memory at
+// once and a thread's chain is its row's terms alone; every accumulator adds
+// the same terms in the same order as m2l_fp32_kernel's.  Bound by the latency
+// of the source rows' loads, which are issued one slot ahead.  Runs in blocks
+// of m2l_tc_kernel's launch beside its tiles.  (A thread per box with the
+// matrices staged slot by slot took 79 us for a tile, whatever it held.)
+constexpr int rows_tile(int nr) { return 128 / nr; }  // boxes per block of 128 threads
+constexpr int kRowsP1 = 20;
 
-template <int P1, int CH, int NR>
-__global__ void __launch_bounds__(kRowsTile * NR) m2l_rows_kernel(
-    SegTable seg, const int *__restrict__ boxes, const int *__restrict__ slots,
-    const double *__restrict__ bs, int ndc, int c0, int p, const float2 *__restrict__ Tall,
-    const float2 *__restrict__ mp32, double2 *__restrict__ loc, int ntiles) {
-    __shared__ __align__(16) float2 sT[kSlots * NR * P1];
-    __shared__ int s_tb[257];
-    for (int e = threadIdx.x; e <= seg.nseg && e < 257; e += blockDim.x) s_tb[e] = seg.tile_base[e];
+template <int CH, int NR>
+__device__ __forceinline__ void m2l_rows(const SegTable &seg, const int *s_tb, float2 *sT,
+                                         const int *__restrict__ boxes,
+                                         const int *__restrict__ slots,
+                                         const double *__restrict__ bs, int ndc, int c0, int p,
+                                         const float2 *__restrict__ Tall,
+                                         const float2 *__restrict__ mp32,
+                                         double2 *__restrict__ loc, int first, int step,
+                                         int ntiles) {
+    constexpr int P1 = kRowsP1, TILE = rows_tile(NR);
     const int stride = (p + 1) * ndc;
     const int row = threadIdx.x % NR, bx = threadIdx.x / NR;
     int cp_in = -1;
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        __syncthreads();
+    for (int tile = first; tile < ntiles; tile += step) {
         int lo = 0, hi = seg.nseg;
         while (hi - lo > 1) {
             const int mid = (lo + hi) >> 1;
@@ -553,27 +557,44 @@ __global__ void __launch_bounds__(kRowsTile * NR) m2l_rows_kernel(
         }
         const int cp = seg.cpos[lo];
         if (cp != cp_in) {
+            __syncthreads();
             const float2 *Tc = Tall + (size_t)cp * kSlots * P1 * P1;
             for (int e = threadIdx.x; e < kSlots * NR * P1; e += blockDim.x)
                 sT[e] = Tc[(size_t)(e / (NR * P1)) * P1 * P1 + e % (NR * P1)];
             cp_in = cp;
             __syncthreads();
         }
-        const int q = seg.start[lo] + (tile - s_tb[lo]) * kRowsTile + bx;
-        if (q >= seg.start[lo] + seg.count[lo] || row > p) continue;
-        float2 acc[CH], s0[CH];
+        const int q = seg.start[lo] + (tile - s_tb[lo]) * TILE + bx;
+        if (bx >= TILE || q >= seg.start[lo] + seg.count[lo] || row > p) continue;
+        const int *qs = slots + (size_t)q * kSlots;
+        int sb[kSlots];
+        unsigned mask = 0u;
 #pragma unroll
-        for (int c = 0; c < CH; c++) acc[c] = s0[c] = make_float2(0.f, 0.f);
-        for (int k = 0; k < kSlots; k++) {
-            const int sb = slots[(size_t)q * kSlots + k];
-            if (sb < 0) continue;
-            const float2 *M = mp32 + (size_t)sb * stride + c0;
-            float2 m[P1][CH];
+        for (int k = 0; k < kSlots; k++) sb[k] = qs[k];
+#pragma unroll
+        for (int k = 0; k < kSlots; k++)
+            if (sb[k] >= 0) mask |= 1u << k;
+        float2 m[P1][CH], n[P1][CH];
+        auto load = [&](int k) {
+            const float2 *M = mp32 + (size_t)qs[k] * stride + c0;
 #pragma unroll
             for (int j = 0; j < P1; j++)
 #pragma unroll
                 for (int c = 0; c < CH; c++)
-                    m[j][c] = j <= p ? M[(size_t)j * ndc + c] : make_float2(0.f, 0.f);
+                    n[j][c] = j <= p ? M[(size_t)j * ndc + c] : make_float2(0.f, 0.f);
+        };
+        float2 acc[CH], s0[CH];
+#pragma unroll
+        for (int c = 0; c < CH; c++) acc[c] = s0[c] = make_float2(0.f, 0.f);
+        if (mask) load(__ffs(mask) - 1);
+        while (mask) {
+            const int k = __ffs(mask) - 1;
+            mask &= mask - 1;
+#pragma unroll
+            for (int j = 0; j < P1; j++)
+#pragma unroll
+                for (int c = 0; c < CH; c++) m[j][c] = n[j][c];
+            if (mask) load(__ffs(mask) - 1);
             const float2 *t0 = sT + (k * NR + row) * P1;
 #pragma unroll
             for (int c = 0; c < CH; c++) {
@@ -679,22 +700,6 @@ void launch_fp32(const M2LWork &w, const Tree &T, const CauchyProblem &P, const 
     }
 }
 
-template <int P1, int NR>
-void launch_rows(const M2LWork &w, const Tree &T, const CauchyProblem &P, const float2 *Tab,
-                 const float2 *mp32, double2 *loc, cudaStream_t s) {
-    const int ntiles = w.ntiles(kRowsTile);
-    const int blocks = std::max(1, std::min(ntiles, kNumSM * 16));
-    for (int c0 = 0; c0 < P.ndc;) {
-        const int ch = P.ndc - c0 >= 2 ? 2 : 1;
-        auto kern = ch == 2 ? m2l_rows_kernel<P1, 2, NR> : m2l_rows_kernel<P1, 1, NR>;
-        kern<<<blocks, kRowsTile * NR, 0, s>>>(w.seg(kRowsTile), w.boxes.get(), w.slots.get(),
-                                               T.d_boxsize.get(), P.ndc, c0, P.p, Tab, mp32, loc,
-                                               ntiles);
-        FMM_CHECK_LAUNCH();
-        c0 += ch;
-    }
-}
-
 // ---------------------------------------------------------------------------
 // M2L of the mixed mode on the 5th-generation tensor cores (tcgen05, kind
 // tf32, operands in shared memory, accumulator in tensor memory).
@@ -733,31 +738,71 @@ __device__ __forceinline__ bool tc_wait(uint32_t mbar, uint32_t parity) {
 // `rows` rows
 __host__ __device__ __forceinline__ int tc_off(int row, int k, int rows) { return tc_fidx(row, k, rows) << 2; }
 
-template <int CH, int HALF>
-__global__ void __launch_bounds__(kTcRows, 1) m2l_tc_kernel(
-    SegTable seg, const int *__restrict__ boxes, const int *__restrict__ slots,
-    const double *__restrict__ bs, int ndc, int c0, int p,
-    const float *__restrict__ Bimg, const float2 *__restrict__ T0,
-    const float2 *__restrict__ mp32, double2 *__restrict__ loc, int ntiles,
-    int *__restrict__ err) {
+// The slots of a tile are pipelined D deep: the rows' source multipoles are
+// loaded D slots ahead into registers, a slot's matrix comes by one bulk copy D
+// slots ahead into one of 2 D buffers, and the operand rows have D buffers, so
+// that with D = 2 storing one slot's rows overlaps the MMAs of the slot before.
+// D = 2 (one block per SM) runs while every tile has an SM of its own and the
+// chain of its 27 slots is what takes the time; with more tiles three blocks of
+// D = 1 per SM overlap one another instead.  (One buffer, filled by all threads
+// after the previous slot's MMAs, took 2.8 us per slot: 76 us for a single
+// tile.)
+//
+// NR > 0: the rows below NR are left to m2l_rows, which runs in the blocks
+// from ntcb on; NR = 0: row 0 (L_0, whose terms cancel across the slots) is
+// summed in FP32 beside the MMAs.
+template <int HALF, int D>
+constexpr size_t tc_smem_bytes() {
+    return (size_t)D * (2 * kTcRows * 2 * HALF + 2 * 2 * 4 * HALF * HALF) * sizeof(float);
+}
+
+struct TcArgs {
+    SegTable seg, rseg;  // tiles of the rows' operand, of m2l_rows
+    const int *boxes, *slots;
+    const double *bs;
+    int ndc, c0, p, ntiles, ntcb, nrtiles;
+    const float *Bimg;
+    const float2 *T0, *Trows, *mp32;
+    double2 *loc;
+    int *err;
+};
+
+template <int CH, int HALF, int NR, int D>
+__global__ void __launch_bounds__(kTcRows, D == 1 ? 3 : 1) m2l_tc_kernel(const TcArgs A) {
+    constexpr int kABufs = D, kBBufs = 2 * D;
     constexpr int KP = 2 * HALF;  // [Re 0..HALF-1 | Im 0..HALF-1]
+    constexpr int kAFloats = 2 * kTcRows * KP, kBFloats = 2 * KP * KP;
     extern __shared__ __align__(1024) unsigned char tc_smem[];
-    float *sAhi = reinterpret_cast<float *>(tc_smem);
-    float *sAlo = sAhi + kTcRows * KP;
-    float *sBhi = sAlo + kTcRows * KP;  // followed by the lo image
-    __shared__ __align__(8) uint64_t s_mbar;
+    float *sA = reinterpret_cast<float *>(tc_smem);       // [buffer][hi, lo]
+    float *sB = sA + kABufs * kAFloats;                 // [buffer][hi, lo]
+    constexpr int TPT = kTcRows / CH;
+    __shared__ __align__(8) uint64_t s_mbar[kABufs + kBBufs];
     __shared__ uint32_t s_tmem;
     __shared__ int s_tb[257];
     __shared__ unsigned s_mask;
-    __shared__ float2 s_t0[kSlots * (kTcMaxKP / 2)];
+    __shared__ int s_qs[TPT * kSlots];
+    __shared__ float2 s_t0[NR > 0 ? 1 : kSlots * (kTcMaxKP / 2)];
     const int tid = threadIdx.x, warp = tid >> 5;
+    if constexpr (NR > 0) {
+        if ((int)blockIdx.x >= A.ntcb) {
+            for (int e = tid; e <= A.rseg.nseg && e < 257; e += blockDim.x)
+                s_tb[e] = A.rseg.tile_base[e];
+            __syncthreads();
+            m2l_rows<CH, NR>(A.rseg, s_tb, reinterpret_cast<float2 *>(tc_smem), A.boxes, A.slots,
+                             A.bs, A.ndc, A.c0, A.p, A.Trows, A.mp32, A.loc,
+                             (int)blockIdx.x - A.ntcb, (int)gridDim.x - A.ntcb, A.nrtiles);
+            return;
+        }
+    }
+    const SegTable &seg = A.seg;
     for (int e = tid; e <= seg.nseg && e < 257; e += blockDim.x) s_tb[e] = seg.tile_base[e];
-    if (tid == 0) s_mask = 0u;
-    const uint32_t mbar = smem_u32(&s_mbar);
     if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mbar), "r"(1) : "memory");
+        s_mask = 0u;
+        for (int i = 0; i < kABufs + kBBufs; i++) mbar_init(smem_u32(&s_mbar[i]), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    auto a_bar = [&](int i) { return smem_u32(&s_mbar[i]); };
+    auto b_bar = [&](int i) { return smem_u32(&s_mbar[kABufs + i]); };
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                          smem_u32(&s_tmem)),
@@ -768,18 +813,16 @@ __global__ void __launch_bounds__(kTcRows, 1) m2l_tc_kernel(
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = s_tmem;
-    const int TPT = kTcRows / CH;
-    const int P = p + 1, stride = P * ndc;
-    const int nB4 = (2 * KP * KP) / 4;  // float4s of the two B images
-    const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(KP >> 3) << 17) |
-                           (8u << 24);
-    const uint32_t aLBO = (kTcRows / 8) * 128, bLBO = (KP / 8) * 128, SBO = 128;
-    const uint32_t aHi = smem_u32(sAhi), aLo = smem_u32(sAlo);
-    const uint32_t bHi = smem_u32(sBhi), bLo = bHi + KP * KP * 4;
-    uint32_t ncommit = 0;
+    const int P = A.p + 1, stride = P * A.ndc;
+    constexpr uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(KP >> 3) << 17) |
+                               (8u << 24);
+    constexpr uint32_t aLBO = (kTcRows / 8) * 128, bLBO = (KP / 8) * 128, SBO = 128;
+    // uses of every buffer so far (thread-uniform; B's by thread 0)
+    uint32_t na[kABufs] = {}, nb_issued[kBBufs] = {}, nb_done[kBBufs] = {};
+    int last = -1;  // operand buffer of the last commit
     bool failed = false;
     int cp_loaded = -1;
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    for (int tile = blockIdx.x; tile < A.ntiles; tile += NR > 0 ? A.ntcb : (int)gridDim.x) {
         int lo = 0, hi = seg.nseg;
         while (hi - lo > 1) {
             const int mid = (lo + hi) >> 1;
@@ -787,20 +830,24 @@ __global__ void __launch_bounds__(kTcRows, 1) m2l_tc_kernel(
         }
         const int sg = lo;
         const int qend = seg.start[sg] + seg.count[sg];
-        const int q = seg.start[sg] + (tile - s_tb[sg]) * TPT + tid / CH;
-        const int c = c0 + tid % CH;
-        const bool valid = q < qend;
+        const int q0 = seg.start[sg] + (tile - s_tb[sg]) * TPT;
+        const int nbox = min(TPT, qend - q0);
+        const int bx = tid / CH, q = q0 + bx, c = A.c0 + tid % CH;
+        const bool valid = bx < nbox;
         const int cp = seg.cpos[sg];
-        // the source of every slot for this row, and the tile's slot mask
-        const int *qslots = slots + (size_t)(valid ? q : 0) * kSlots;
+        // the sources of the tile's slots, and the mask of slots in use
         unsigned mymask = 0u;
-#pragma unroll
-        for (int k = 0; k < kSlots; k++)
-            if (valid && qslots[k] >= 0) mymask |= 1u << k;
-        if (mymask) atomicOr(&s_mask, mymask);
-        if (cp != cp_loaded) {  // row 0 of this position's 27 matrices
+        for (int e = tid; e < nbox * kSlots; e += kTcRows) {
+            const int sb = A.slots[(size_t)q0 * kSlots + e];
+            s_qs[e] = sb;
+            if (sb >= 0) mymask |= 1u << (e % kSlots);
+        }
+        mymask = __reduce_or_sync(0xffffffffu, mymask);
+        if ((tid & 31) == 0 && mymask) atomicOr(&s_mask, mymask);
+        if (NR == 0 && cp != cp_loaded) {  // row 0 of this position's 27 matrices
             for (int e = tid; e < kSlots * P; e += blockDim.x)
-                s_t0[(e / P) * (kTcMaxKP / 2) + e % P] = T0[((size_t)cp * kSlots + e / P) * P + e % P];
+                s_t0[(e / P) * (kTcMaxKP / 2) + e % P] =
+                    A.T0[((size_t)cp * kSlots + e / P) * P + e % P];
         }
         cp_loaded = cp;
         __syncthreads();
@@ -809,34 +856,46 @@ __global__ void __launch_bounds__(kTcRows, 1) m2l_tc_kernel(
         if (tid == 0) s_mask = 0u;
         float l0x = 0.f, l0y = 0.f;  // row 0 (L_0) on the CUDA cores
         float s0x = 0.f, s0y = 0.f;
-        // registers holding the next slot's row and matrix part
-        float2 mrow[HALF];
-        float4 breg[(2 * KP * KP / 4 + kTcRows - 1) / kTcRows];
-        auto prefetch = [&](int k) {
-            const int sb = valid ? qslots[k] : -1;
-            const float2 *M = mp32 + (size_t)(sb >= 0 ? sb : 0) * stride + c;
+        // source rows of the coming D slots
+        float2 m0[HALF], m1[D == 2 ? HALF : 1];
+        auto load = [&](int k, float2 *m) {
+            const int sb = valid && k >= 0 ? s_qs[bx * kSlots + k] : -1;
+            const float2 *M = A.mp32 + (size_t)(sb >= 0 ? sb : 0) * stride + c;
 #pragma unroll
             for (int j = 0; j < HALF; j++)
-                mrow[j] = (sb >= 0 && j < P) ? M[(size_t)j * ndc] : make_float2(0.f, 0.f);
-            const float4 *src = reinterpret_cast<const float4 *>(
-                Bimg + ((size_t)cp * kSlots + k) * 2 * KP * KP);
-#pragma unroll
-            for (int u = 0; u < (int)(sizeof(breg) / sizeof(float4)); u++) {
-                const int e = tid + u * kTcRows;
-                breg[u] = e < nB4 ? src[e] : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
+                m[j] = (sb >= 0 && j < P) ? M[(size_t)j * A.ndc] : make_float2(0.f, 0.f);
         };
-        bool issued = false;
-        if (mask) prefetch(__ffs(mask) - 1);
-        while (mask) {
+        // a slot's matrix (hi and lo images) into B buffer `buf`
+        auto fetch = [&](int k, int buf) {
+            if (tid != 0 || k < 0) return;
+            mbar_arrive_expect_tx(b_bar(buf), kBFloats * sizeof(float));
+            bulk_g2s(smem_u32(sB + buf * kBFloats),
+                     A.Bimg + ((size_t)cp * kSlots + k) * kBFloats, kBFloats * sizeof(float),
+                     b_bar(buf));
+            nb_issued[buf]++;
+        };
+        // slots in order: k0 now, k1 (and with D = 2 k2) next
+        auto pop = [&]() {
+            if (!mask) return -1;
             const int k = __ffs(mask) - 1;
             mask &= mask - 1;
-            // the previous slot's MMAs read the operand buffers
-            if (ncommit > 0 && !tc_wait(mbar, (ncommit - 1) & 1)) failed = true;
-            if (__syncthreads_or(failed)) {
-                failed = true;
-                break;
-            }
+            return k;
+        };
+        int k0 = pop(), k1 = pop();
+        // (every MMA of the tile before has completed: the buffers are free)
+        fetch(k0, 0);
+        load(k0, m0);
+        if (D == 2) {
+            fetch(k1, 1);
+            load(k1, m1);
+        }
+        bool issued = false;
+        for (int i = 0; k0 >= 0; i++) {
+            const int ab = i & (kABufs - 1), bb = i & (kBBufs - 1);
+            // the MMAs of slot i - D read this operand buffer (and B buffer
+            // i + D)
+            if (i >= D && !tc_wait(a_bar(ab), (na[ab] - 1) & 1)) failed = true;
+            float *hi_ = sA + ab * kAFloats, *lo_ = hi_ + kTcRows * KP;
             // A row `tid`: [Re M_0..HALF-1 | Im M_0..HALF-1] (zero beyond p),
             // split into TF32 hi / lo
 #pragma unroll
@@ -846,62 +905,79 @@ __global__ void __launch_bounds__(kTcRows, 1) m2l_tc_kernel(
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
                     const int kk = kc + u;
-                    const float v = kk < HALF ? mrow[kk].x : mrow[kk - HALF].y;
+                    const float v = kk < HALF ? m0[kk].x : m0[kk - HALF].y;
                     const float h = tc_tf32(v);
                     ph[u] = h;
                     pl[u] = tc_tf32(v - h);
                 }
                 const int off = tc_off(tid, kc, kTcRows) >> 2;
-                *reinterpret_cast<float4 *>(sAhi + off) = vh;
-                *reinterpret_cast<float4 *>(sAlo + off) = vl;
-            }
-            {
-                float4 *dst = reinterpret_cast<float4 *>(sBhi);
-#pragma unroll
-                for (int u = 0; u < (int)(sizeof(breg) / sizeof(float4)); u++) {
-                    const int e = tid + u * kTcRows;
-                    if (e < nB4) dst[e] = breg[u];
-                }
+                *reinterpret_cast<float4 *>(hi_ + off) = vh;
+                *reinterpret_cast<float4 *>(lo_ + off) = vl;
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncthreads();
-            if (tid == 0) {
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                for (int ks = 0; ks < KP / 8; ks++) {
-                    const uint32_t ao = 2 * ks * aLBO, bo = 2 * ks * bLBO;
-                    tc_mma(tmem, tc_sdesc(aHi + ao, aLBO, SBO), tc_sdesc(bHi + bo, bLBO, SBO),
-                           idesc, (issued || ks > 0) ? 1u : 0u);
-                    tc_mma(tmem, tc_sdesc(aHi + ao, aLBO, SBO), tc_sdesc(bLo + bo, bLBO, SBO),
-                           idesc, 1u);
-                    tc_mma(tmem, tc_sdesc(aLo + ao, aLBO, SBO), tc_sdesc(bHi + bo, bLBO, SBO),
-                           idesc, 1u);
-                }
-                tc_commit(mbar);
+            if (__syncthreads_or(failed)) {
+                failed = true;
+                break;
             }
-            ncommit++;
+            const int k2 = pop(), kn = D == 2 ? k2 : k1;  // kn: D slots on
+            fetch(kn, (i + D) & (kBBufs - 1));  // (was slot i - D's)
+            if (tid == 0) {
+                if (!tc_wait(b_bar(bb), (nb_issued[bb] - 1) & 1)) {
+                    failed = true;
+                } else {
+                    nb_done[bb] = nb_issued[bb];
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint32_t aHi = smem_u32(hi_), aLo = smem_u32(lo_);
+                    const uint32_t bHi = smem_u32(sB + bb * kBFloats), bLo = bHi + KP * KP * 4;
+                    for (int ks = 0; ks < KP / 8; ks++) {
+                        const uint32_t ao = 2 * ks * aLBO, bo = 2 * ks * bLBO;
+                        tc_mma(tmem, tc_sdesc(aHi + ao, aLBO, SBO), tc_sdesc(bHi + bo, bLBO, SBO),
+                               idesc, (issued || ks > 0) ? 1u : 0u);
+                        tc_mma(tmem, tc_sdesc(aHi + ao, aLBO, SBO), tc_sdesc(bLo + bo, bLBO, SBO),
+                               idesc, 1u);
+                        tc_mma(tmem, tc_sdesc(aLo + ao, aLBO, SBO), tc_sdesc(bHi + bo, bLBO, SBO),
+                               idesc, 1u);
+                    }
+                    tc_commit(a_bar(ab));
+                }
+            }
+            na[ab]++;
+            last = ab;
             issued = true;
-            // row 0 on the CUDA cores while the MMAs run, then the next slot
-            if (valid && qslots[k] >= 0) {
-                const float2 *t0 = s_t0 + k * (kTcMaxKP / 2);
+            if (NR == 0 && valid && s_qs[bx * kSlots + k0] >= 0) {
+                // row 0 on the CUDA cores while the MMAs run
+                const float2 *t0 = s_t0 + (NR > 0 ? 0 : k0 * (kTcMaxKP / 2));
 #pragma unroll
                 for (int j = 0; j < HALF; j++) {
                     if (j < P) {
-                        const float2 t = t0[j], m = mrow[j];
+                        const float2 t = t0[j], m = m0[j];
                         l0x = fmaf(t.x, m.x, fmaf(-t.y, m.y, l0x));
                         l0y = fmaf(t.x, m.y, fmaf(t.y, m.x, l0y));
                     }
                 }
-                s0x += mrow[0].x;
-                s0y += mrow[0].y;
+                s0x += m0[0].x;
+                s0y += m0[0].y;
             }
-            if (mask) prefetch(__ffs(mask) - 1);
+            if (D == 2) {
+#pragma unroll
+                for (int j = 0; j < HALF; j++) m0[j] = m1[D == 2 ? j : 0];
+                load(kn, m1);
+            } else {
+                load(kn, m0);
+            }
+            k0 = k1;
+            k1 = k2;
         }
-        if (failed) break;
+        if (__syncthreads_or(failed)) {
+            failed = true;
+            break;
+        }
         float d[KP];
 #pragma unroll
         for (int i = 0; i < KP; i++) d[i] = 0.f;
         if (issued) {
-            if (!tc_wait(mbar, (ncommit - 1) & 1)) failed = true;
+            // (a commit covers every MMA issued before it)
+            if (!tc_wait(a_bar(last), (na[last] - 1) & 1)) failed = true;
             if (__syncthreads_or(failed)) {
                 failed = true;
                 break;
@@ -918,21 +994,20 @@ __global__ void __launch_bounds__(kTcRows, 1) m2l_tc_kernel(
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         }
         if (valid) {
-            const int b = boxes[q];
-            const double lr = log(bs[seg.level[sg]]);
+            const int b = A.boxes[q];
+            const double lr = NR > 0 ? 0.0 : log(A.bs[seg.level[sg]]);
 #pragma unroll
             for (int i = 0; i < HALF; i++) {
-                if (i < P) {
-                    double re, im;
-                    if (i == 0) {
-                        re = (double)l0x + lr * s0x;
-                        im = (double)l0y + lr * s0y;
-                    } else {
-                        re = d[i];
-                        im = d[HALF + i];
-                    }
-                    loc[(size_t)b * stride + (size_t)i * ndc + c] = make_double2(re, im);
+                if (i < NR || i >= P) continue;
+                double re, im;
+                if (i == 0) {
+                    re = (double)l0x + lr * s0x;
+                    im = (double)l0y + lr * s0y;
+                } else {
+                    re = d[i];
+                    im = d[HALF + i];
                 }
+                A.loc[(size_t)b * stride + (size_t)i * A.ndc + c] = make_double2(re, im);
             }
         }
         // the next tile's MMAs overwrite the accumulator
@@ -940,9 +1015,14 @@ __global__ void __launch_bounds__(kTcRows, 1) m2l_tc_kernel(
         __syncthreads();
     }
     if (failed) {
-        if (tid == 0) atomicExch(err, 1);
-        // let MMAs still in flight finish before the memory is released
-        if (ncommit > 0) tc_wait(mbar, (ncommit - 1) & 1);
+        if (tid == 0) {
+            atomicExch(A.err, 1);
+            // let the copies and MMAs still in flight finish before the
+            // memory is released
+            for (int i = 0; i < kBBufs; i++)
+                if (nb_issued[i] != nb_done[i]) tc_wait(b_bar(i), (nb_issued[i] - 1) & 1);
+        }
+        if (last >= 0 && na[last] > 0) tc_wait(a_bar(last), (na[last] - 1) & 1);
     }
     __syncthreads();
     if (warp == 0) {
@@ -950,6 +1030,20 @@ __global__ void __launch_bounds__(kTcRows, 1) m2l_tc_kernel(
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(64)
                      : "memory");
     }
+}
+
+// m2l_rows alone: with more tiles than SMs its blocks would wait for the shared
+// memory of the tensor-core form's.
+template <int CH, int NR>
+__global__ void __launch_bounds__(kTcRows) m2l_rows_kernel(const TcArgs A) {
+    extern __shared__ __align__(16) unsigned char rows_smem[];
+    __shared__ int s_tb[257];
+    for (int e = threadIdx.x; e <= A.rseg.nseg && e < 257; e += blockDim.x)
+        s_tb[e] = A.rseg.tile_base[e];
+    __syncthreads();
+    m2l_rows<CH, NR>(A.rseg, s_tb, reinterpret_cast<float2 *>(rows_smem), A.boxes, A.slots, A.bs,
+                     A.ndc, A.c0, A.p, A.Trows, A.mp32, A.loc, (int)blockIdx.x, (int)gridDim.x,
+                     A.nrtiles);
 }
 
 // B images per (child position, slot): the real form of T (rows = outputs
@@ -1376,14 +1470,15 @@ bool m2l_fp32(const Tree &T, const CauchyProblem &P, const double2 *mp, double2 
     const uint64_t done =
         (simt || tile_only) ? 0 : m2l_window_fp32(T, P, mp32p, loc, errp, s);
     const int wtile = simt ? kFp32Tile : kTcRows / CH;
-    const bool rows = !simt && m2l_exact_rows(p);
+    const bool hess = std::max(P.sset.n > 0 ? P.sset.pgh : 0, P.tset.n > 0 ? P.tset.pgh : 0) >= 3;
+    const int nrows = simt || !m2l_exact_rows(p) ? 0 : (hess ? kM2LExactRowsHess : kM2LExactRows);
     bool ok = false;
     // (tiles of the tensor-core form, of its single remaining channels and
     // of the leading rows from one plan)
-    const auto wp = m2l_cached<M2LWork>(cache, m2l_key(3, wtile, done), ok, [&](M2LWork &x) {
+    const auto wp = m2l_cached<M2LWork>(cache, m2l_key(3, wtile + 1000 * nrows, done), ok, [&](M2LWork &x) {
         std::vector<int> tiles{wtile};
         if (!simt && CH == 2 && P.ndc % 2 != 0) tiles.push_back(kTcRows);
-        if (rows) tiles.push_back(kRowsTile);
+        if (nrows) tiles.push_back(rows_tile(nrows));
         return m2l_work(T, P, tiles, s, x, done);
     });
     if (!ok) return false;
@@ -1399,47 +1494,81 @@ bool m2l_fp32(const Tree &T, const CauchyProblem &P, const double2 *mp, double2 
         const int KP = 2 * HALF;
         const float2 *tab0 = nullptr;
         const float *tab = tc_tables(p, KP, s, &tab0);
-        const size_t smem = (size_t)(2 * kTcRows * KP + 2 * KP * KP) * sizeof(float);
-        auto launch = [&](auto kern, int tile, int c0) {
-            raise_smem_limit(kern, (int)smem);
-            const int ntiles = w.ntiles(tile);
-            const int blocks = std::max(1, std::min(ntiles, kNumSM * 4));
-            kern<<<blocks, kTcRows, smem, s>>>(w.seg(tile), w.boxes.get(), w.slots.get(),
-                                               T.d_boxsize.get(), P.ndc, c0, p, tab, tab0,
-                                               mp32p, loc, ntiles, errp);
+        // A TF32 x 3 product is accurate to about 2^-22, four times an FP32
+        // product.  Measured on 10^5 uniform charges at eps 1e-6 (order 18),
+        // the gradient at the sources then has a relative error of 1.6e-6
+        // with the tensor-core forms against 2.0e-7 with the FP32 CUDA-core
+        // form.  From order kM2LExactFrom on, the leading kM2LExactRows local
+        // coefficients -- L_0 .. L_3, which carry most of the gradient at a
+        // leaf's points -- are therefore summed in FP32 on the CUDA cores: on
+        // the window levels from the windows (m2l_window.cu), on the other
+        // levels by m2l_rows.
+        auto launch = [&](auto deep, size_t deep_smem, auto wide, size_t wide_smem, auto rows,
+                          int tile, int nr, int c0) {
+            TcArgs a;
+            a.seg = w.seg(tile);
+            a.rseg = nr ? w.seg(rows_tile(nr)) : a.seg;
+            a.boxes = w.boxes.get();
+            a.slots = w.slots.get();
+            a.bs = T.d_boxsize.get();
+            a.ndc = P.ndc;
+            a.c0 = c0;
+            a.p = p;
+            a.ntiles = w.ntiles(tile);
+            const bool own = a.ntiles <= kNumSM;  // an SM for every tile
+            a.ntcb = std::max(1, std::min(a.ntiles, kNumSM * 3));
+            a.nrtiles = nr ? w.ntiles(rows_tile(nr)) : 0;
+            a.Bimg = tab;
+            a.T0 = tab0;
+            a.Trows = nr ? fp32_tables(p, kRowsP1, s) : nullptr;
+            a.mp32 = mp32p;
+            a.loc = loc;
+            a.err = errp;
+            // one launch while every tile has an SM, else the rows apart
+            const bool apart = nr && a.ntiles + a.nrtiles > kNumSM;
+            const int blocks = a.ntcb + (apart ? 0 : a.nrtiles);
+            if (own) {
+                raise_smem_limit(deep, deep_smem);
+                deep<<<blocks, kTcRows, deep_smem, s>>>(a);
+            } else {
+                raise_smem_limit(wide, wide_smem);
+                wide<<<blocks, kTcRows, wide_smem, s>>>(a);
+            }
             FMM_CHECK_LAUNCH();
+            if (apart) {
+                const size_t sm = (size_t)kSlots * nr * kRowsP1 * sizeof(float2);
+                rows<<<std::min(a.nrtiles, kNumSM * 8), kTcRows, sm, s>>>(a);
+                FMM_CHECK_LAUNCH();
+            }
+        };
+        auto form = [&](auto ch, auto half, auto nr, auto rows, int tile, int c0) {
+            constexpr int C = decltype(ch)::value, H = decltype(half)::value,
+                          N = decltype(nr)::value;
+            launch(m2l_tc_kernel<C, H, N, 2>, tc_smem_bytes<H, 2>(), m2l_tc_kernel<C, H, N, 1>,
+                   tc_smem_bytes<H, 1>(), rows, tile, N, c0);
+        };
+        auto one = [&](auto ch, int tile, int c0) {
+            constexpr int C = decltype(ch)::value;
+            constexpr std::integral_constant<int, 0> none{};
+            constexpr std::integral_constant<int, kM2LExactRows> nr{};
+            constexpr std::integral_constant<int, kM2LExactRowsHess> nrh{};
+            constexpr std::integral_constant<int, 12> h12{};
+            constexpr std::integral_constant<int, 20> h20{};
+            auto rows = m2l_rows_kernel<C, kM2LExactRows>;
+            if (HALF == 12) form(ch, h12, none, rows, tile, c0);
+            else if (nrows == kM2LExactRowsHess)
+                form(ch, h20, nrh, m2l_rows_kernel<C, kM2LExactRowsHess>, tile, c0);
+            else if (nrows) form(ch, h20, nr, rows, tile, c0);
+            else form(ch, h20, none, rows, tile, c0);
         };
         int c0 = 0;
-        if (CH == 2) {
-            for (; P.ndc - c0 >= 2; c0 += 2) {
-                if (HALF == 12) launch(m2l_tc_kernel<2, 12>, wtile, c0);
-                else launch(m2l_tc_kernel<2, 20>, wtile, c0);
-            }
-        }
+        if (CH == 2)
+            for (; P.ndc - c0 >= 2; c0 += 2) one(std::integral_constant<int, 2>{}, wtile, c0);
         // remaining single channels, one channel per row
-        for (; c0 < P.ndc; c0++) {
-            if (HALF == 12) launch(m2l_tc_kernel<1, 12>, kTcRows, c0);
-            else launch(m2l_tc_kernel<1, 20>, kTcRows, c0);
-        }
+        for (; c0 < P.ndc; c0++) one(std::integral_constant<int, 1>{}, kTcRows, c0);
     }
     if (!deferred && read_scalar(errp, s) != 0)
         throw FmmError(4, "tensor-core M2L: a wait for an MMA or operand barrier timed out");
-    // A TF32 x 3 product is accurate to about 2^-22, four times an FP32
-    // product.  Measured on 10^5 uniform charges at eps 1e-6 (order 18),
-    // the gradient at the sources then has a relative error of 1.6e-6 with
-    // the tensor-core forms against 2.0e-7 with the FP32 CUDA-core form.
-    // From order kM2LExactFrom on, the leading kM2LExactRows local
-    // coefficients -- L_0 .. L_3, which carry most of the gradient at a
-    // leaf's points -- are therefore recomputed in FP32 on the CUDA cores:
-    // on the window levels from the windows (m2l_window.cu), on the other
-    // levels here with the slot tables.
-    if (rows && w.ntarg > 0) {
-        const bool hess = std::max(P.sset.n > 0 ? P.sset.pgh : 0, P.tset.n > 0 ? P.tset.pgh : 0) >= 3;
-        if (hess)
-            launch_rows<20, kM2LExactRowsHess>(w, T, P, fp32_tables(p, 20, s), mp32p, loc, s);
-        else
-            launch_rows<20, kM2LExactRows>(w, T, P, fp32_tables(p, 20, s), mp32p, loc, s);
-    }
     return true;
 }
 
