@@ -6,8 +6,8 @@
 // depending on the one before: about seven per level, most of them a few
 // microseconds of dependent loads.  As launches, with a host synchronisation
 // per level for the counts, they took 1.08 ms on 4e5 clustered points (12
-// levels; here 0.49), 0.87 ms on 5e4 (0.33), 2.76 ms on the 8e6 points of a
-// boundary curve (18 levels; 2.50, bound by the colleagues' loads).  Here they
+// levels; here 0.43), 0.87 ms on 5e4 (0.35), 2.76 ms on the 8e6 points of a
+// boundary curve (18 levels; 2.10, bound by the colleagues' loads).  Here they
 // are
 // phases of one kernel with a grid-wide barrier between them; counts stay on
 // the device, and one status read at the end gives the host the new level
@@ -33,8 +33,10 @@ struct LrOut {
     int lstart[kRefLevels], lend[kRefLevels];
 };
 
-constexpr int kLrThreads = 256;
-constexpr int kLrBlocks = kNumSM * 4;
+// One block of 1024 threads per SM: a quarter of the arrivals at each of the
+// grid barriers (four blocks of 256: 2.48 ms on the boundary curve's points).
+constexpr int kLrThreads = 1024;
+constexpr int kLrBlocks = kNumSM;
 
 struct LrArgs {
     LrSet a, b;
@@ -209,7 +211,7 @@ struct LrMap {
     }
 };
 
-__global__ void __launch_bounds__(kLrThreads, 4) tree_lr_kernel(LrArgs A) {
+__global__ void __launch_bounds__(kLrThreads, 1) tree_lr_kernel(LrArgs A) {
     namespace cg = cooperative_groups;
     cg::grid_group grid = cg::this_grid();
     __shared__ LrMap M;
