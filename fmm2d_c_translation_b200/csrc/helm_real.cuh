@@ -363,23 +363,67 @@ __global__ void __launch_bounds__(256) helm_p2l_real_kernel(
 }
 
 // ---------------------------------------------------------------------------
-// M2P + L2P: one thread per point (0.80 -> 0.46 ms at 2e6 points, zk 200; 0.49
-// -> 0.21 ms at 2,001 points with Hessians, where the serial recurrence bounds
-// it).
+// M2P + L2P.  G lanes (a power of two) share a point: they deal its list-3
+// expansions among them, the last one adds the local expansion, and their sums
+// are added by halving.  G = 1 unless the points leave the chip idle
+// (far_lanes): the recurrences are serial, and a few thousand points are a few
+// warps per SM.  The coefficients of the orders around n move through a window
+// of registers, loaded one order ahead: with derivatives an order takes ten
+// coefficients, of which two are new.
+// Bound by the recurrences' latency: 0.80 ms with the general kernels, 0.47
+// here at 2e6 points, zk 200; 1e5 clustered points 0.44 -> 0.21 ms, 2,001
+// points with Hessians 0.21 -> 0.033 ms (one lane per point, coefficients
+// loaded where they are used, a launch per point set).
 // ---------------------------------------------------------------------------
 struct AccR {
     double2 p, u, v, u2, v2;
 };
 
 // One expansion's coefficients with the real derivative factors
-// a_n = (n >= 0 ? z2 : z1), b_n = (n >= 1 ? z1 : z2).
+// a_n = (n >= 0 ? z2 : z1), b_n = (n >= 1 ? z1 : z2).  The window holds
+// P[j] = C(n + j - H), M[j] = C(-n + j - H); up() and down() move n by one.
+template <int PGH, bool UP>
 struct CoefR {
+    static constexpr int H = PGH - 1, K = 2 * H + 1;
     const double2 *c0;
     int p, nd;
     double z1, z2;
+    double2 P[K], M[K], np, nm;
     __device__ __forceinline__ double2 at(int n) const {
         return (n < -p || n > p) ? make_double2(0.0, 0.0) : c0[(long long)n * nd];
     }
+    __device__ __forceinline__ void ahead(int n) {  // what the step from n brings in
+        np = at(UP ? n + 1 + H : n - 1 - H);
+        nm = at(UP ? -n - 1 - H : -n + 1 + H);
+    }
+    __device__ __forceinline__ CoefR(const double2 *c, int p_, int nd_, double za, double zb, int n)
+        : c0(c), p(p_), nd(nd_), z1(za), z2(zb) {
+#pragma unroll
+        for (int j = 0; j < K; j++) {
+            P[j] = at(n + j - H);
+            M[j] = at(-n + j - H);
+        }
+        ahead(n);
+    }
+    // to order n (from n - 1, or n + 1 downwards)
+    __device__ __forceinline__ void step(int n) {
+        constexpr bool pl = UP;  // P moves towards lower indexes
+#pragma unroll
+        for (int j = 0; j + 1 < K; j++) {
+            if (pl) {
+                P[j] = P[j + 1];
+                M[K - 1 - j] = M[K - 2 - j];
+            } else {
+                P[K - 1 - j] = P[K - 2 - j];
+                M[j] = M[j + 1];
+            }
+        }
+        P[pl ? K - 1 : 0] = np;
+        M[pl ? 0 : K - 1] = nm;
+        ahead(n);
+    }
+    __device__ __forceinline__ double2 pos(int d) const { return P[H + d]; }  // C(n + d)
+    __device__ __forceinline__ double2 neg(int d) const { return M[H + d]; }  // C(-n + d)
 };
 
 // Adds the order +n / -n terms (n >= 0) with the angular factor w^n = wn and
@@ -392,17 +436,18 @@ __device__ __forceinline__ void radial_add(double2 &a, double2 g, double b) {
 }
 __device__ __forceinline__ void radial_add(double2 &a, double2 g, double2 b) { cfma(a, g, b); }
 
-template <int PGH, class B>
-__device__ __forceinline__ void acc_real(AccR &A, const CoefR &C, int n, double2 wn, B b) {
+template <int PGH, bool UP, class B>
+__device__ __forceinline__ void acc_real(AccR &A, const CoefR<PGH, UP> &C, int n, double2 wn, B b) {
+    constexpr int d1 = PGH >= 2 ? 1 : 0, d2 = PGH >= 3 ? 2 : 0;  // (inside the window)
     if (n == 0) {
-        radial_add(A.p, C.at(0), b);
+        radial_add(A.p, C.pos(0), b);
         if (PGH >= 2) {
-            radial_add(A.u, cscal(C.at(1), C.z2), b);
-            radial_add(A.v, cscal(C.at(-1), C.z2), b);
+            radial_add(A.u, cscal(C.pos(d1), C.z2), b);
+            radial_add(A.v, cscal(C.pos(-d1), C.z2), b);
         }
         if (PGH >= 3) {
-            radial_add(A.u2, cscal(C.at(2), C.z2 * C.z2), b);
-            radial_add(A.v2, cscal(C.at(-2), C.z2 * C.z2), b);
+            radial_add(A.u2, cscal(C.pos(d2), C.z2 * C.z2), b);
+            radial_add(A.v2, cscal(C.pos(-d2), C.z2 * C.z2), b);
         }
         return;
     }
@@ -413,37 +458,52 @@ __device__ __forceinline__ void acc_real(AccR &A, const CoefR &C, int n, double2
         radial_add(S, g, b);
     };
     {
-        double2 g = cmul(C.at(n), wn);
-        cfma(g, C.at(-n), wm);
+        double2 g = cmul(C.pos(0), wn);
+        cfma(g, C.neg(0), wm);
         radial_add(A.p, g, b);
     }
     if (PGH >= 2) {
-        two(A.u, C.at(n + 1), C.z2, C.at(-n + 1), C.z1);
-        two(A.v, C.at(n - 1), C.z1, C.at(-n - 1), C.z2);
+        two(A.u, C.pos(d1), C.z2, C.neg(d1), C.z1);
+        two(A.v, C.pos(-d1), C.z1, C.neg(-d1), C.z2);
     }
     if (PGH >= 3) {
         const double s1 = C.z1 * C.z1, s2 = C.z2 * C.z2, s12 = C.z1 * C.z2;
         // a_-n a_-n+1: z1 z1, or z1 z2 at n = 1; b_n b_n-1 likewise
         const double f = n == 1 ? s12 : s1;
-        two(A.u2, C.at(n + 2), s2, C.at(-n + 2), f);
-        two(A.v2, C.at(n - 2), f, C.at(-n - 2), s2);
+        two(A.u2, C.pos(d2), s2, C.neg(d2), f);
+        two(A.v2, C.pos(-d2), f, C.neg(-d2), s2);
     }
+}
+
+// Lanes per point: as many (up to 8) as keep the threads of all points within
+// what the chip holds at once of this kernel (16 warps per SM).
+inline int far_lanes(long long points) {
+    int g = 1;
+    while (g < 8 && points * g * 2 <= (long long)kNumSM * 16 * 32) g *= 2;
+    return g;
 }
 
 template <int PGH>
 __global__ void __launch_bounds__(128) helm_far_real_kernel(
-    int n, const double2 *__restrict__ pos, const int *__restrict__ leaf,
-    const int *__restrict__ level, const double2 *__restrict__ centers,
-    const int *__restrict__ nlist3, const int *__restrict__ list3, const HLevel *__restrict__ lv,
-    int nlevels, const double2 *__restrict__ mp, const double2 *__restrict__ loc, int nd,
-    double k, int lmin, double2 *__restrict__ pot, double2 *__restrict__ grad,
-    double2 *__restrict__ hess) {
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        const int b = leaf[t];
+    HFarSet s0, HFarSet s1, int g0, const int *__restrict__ level,
+    const double2 *__restrict__ centers, const int *__restrict__ nlist3,
+    const int *__restrict__ list3, const HLevel *__restrict__ lv, int nlevels,
+    const double2 *__restrict__ mp, const double2 *__restrict__ loc, int nd, int G, double k,
+    int lmin) {
+    const bool second = blockIdx.x >= g0;
+    const HFarSet X = second ? s1 : s0;
+    const long long n = (long long)X.n * G;
+    const int blk = blockIdx.x - (second ? g0 : 0), nblk = second ? gridDim.x - g0 : g0;
+    const int lane = threadIdx.x & 31, sub = lane & (G - 1);
+    const unsigned mask = (G == 1 ? 1u : (1u << G) - 1u) << (lane - sub);
+    for (long long i = (long long)blk * blockDim.x + threadIdx.x; i < n;
+         i += (long long)nblk * blockDim.x) {
+        const int t = (int)(i / G);
+        const int b = X.leaf[t];
         const int l = level[b];
-        if (l < lmin) continue;
+        if (l < lmin) continue;  // (uniform over a point's lanes)
         const HLevel L = lv[l];
-        const double2 x = pos[t];
+        const double2 x = X.pos[t];
         for (int c = 0; c < nd; c++) {
             AccR A;
             A.p = A.u = A.v = A.u2 = A.v2 = make_double2(0.0, 0.0);
@@ -453,22 +513,24 @@ __global__ void __launch_bounds__(128) helm_far_real_kernel(
                 const HLevel L3 = lv[l + 1];
                 const double rs = L3.rs, rs2 = rs * rs;
                 const int N = L3.p + PGH - 1;
-                for (int e = 0; e < nl3; e++) {
+                for (int e = sub; e < nl3; e += G) {
                     const int jb = list3[b * 20 + e];
                     const double2 cc = centers[jb];
                     const double dx = x.x - cc.x, dy = x.y - cc.y;
                     const double rr = sqrt(dx * dx + dy * dy), rinv = 1.0 / rr;
                     const double2 w = make_double2(dx * rinv, dy * rinv);
                     const double xx = k * rr, s = xx * xx;
+                    CoefR<PGH, true> C(coef0(mp, L3, jb, nd) + c, L3.p, nd, 0.5 * k / rs,
+                                       0.5 * k * rs, 0);
                     double2 h0, g;
                     if (s < hb::kSMax) hb::hankel01_sq(s, 1.0 / s, h0, g);
                     else hankel01_far(s, h0, g);
                     const double zr = 2.0 * rs * rinv / k;
-                    const CoefR C{coef0(mp, L3, jb, nd) + c, L3.p, nd, 0.5 * k / rs, 0.5 * k * rs};
-                    acc_real<PGH>(A, C, 0, w, h0);
+                    acc_real(A, C, 0, w, h0);
                     double2 hm1 = h0, hc = cscal(g, xx * rs), wn = w;
                     for (int m = 1; m <= N; m++) {
-                        acc_real<PGH>(A, C, m, wn, hc);
+                        C.step(m);
+                        acc_real(A, C, m, wn, hc);
                         const double f = zr * (double)m;
                         const double2 hn = make_double2(fma(f, hc.x, -rs2 * hm1.x),
                                                         fma(f, hc.y, -rs2 * hm1.y));
@@ -479,13 +541,12 @@ __global__ void __launch_bounds__(128) helm_far_real_kernel(
                 }
             }
             // L2P of the leaf's own local expansion
-            if (l >= 2 && L.flag) {
+            if (l >= 2 && L.flag && sub == G - 1) {
                 const double rs = L.rs, rs2 = rs * rs;
                 const double2 cc = centers[b];
                 const double dx = x.x - cc.x, dy = x.y - cc.y;
                 const double rr = sqrt(dx * dx + dy * dy);
                 const double2 w = rr > 0.0 ? make_double2(dx / rr, dy / rr) : make_double2(1.0, 0.0);
-                const CoefR C{coef0(loc, L, b, nd) + c, L.p, nd, 0.5 * k * rs, 0.5 * k / rs};
                 const int N = L.p + PGH - 1;
                 const double xx = k * rr, h = 0.5 * xx / rs;
                 double ja, jb;  // j_m, j_{m+1}
@@ -497,30 +558,54 @@ __global__ void __launch_bounds__(128) helm_far_real_kernel(
                     ja = jm;
                 }
                 // (a sequence that starts below N: the orders above m + 1 are zero)
-                if (m + 1 <= N) acc_real<PGH>(A, C, m + 1, cpow_int(w, m + 1), jb);
+                const int top = min(m + 1, N);
+                CoefR<PGH, false> C(coef0(loc, L, b, nd) + c, L.p, nd, 0.5 * k * rs, 0.5 * k / rs,
+                                    top);
+                if (m + 1 <= N) {
+                    acc_real(A, C, m + 1, cpow_int(w, m + 1), jb);
+                    C.step(m);
+                }
                 double2 wn = cpow_int(w, m);
                 const double2 wc = cconj(w);
                 for (; m >= 1; m--) {
-                    acc_real<PGH>(A, C, m, wn, ja);
+                    acc_real(A, C, m, wn, ja);
                     const double jm = fma((double)m * hi, ja, -rs2 * jb);
                     jb = ja;
                     ja = jm;
                     wn = cmul(wn, wc);
+                    C.step(m - 1);
                 }
-                acc_real<PGH>(A, C, 0, wn, ja);
+                acc_real(A, C, 0, wn, ja);
             }
+            for (int o = 1; o < G; o <<= 1) {
+                auto sum = [&](double2 &z) {
+                    z.x += __shfl_xor_sync(mask, z.x, o);
+                    z.y += __shfl_xor_sync(mask, z.y, o);
+                };
+                sum(A.p);
+                if (PGH >= 2) {
+                    sum(A.u);
+                    sum(A.v);
+                }
+                if (PGH >= 3) {
+                    sum(A.u2);
+                    sum(A.v2);
+                }
+            }
+            if (sub != 0) continue;
             // i / 4
             auto i4 = [](double2 z) { return make_double2(-0.25 * z.y, 0.25 * z.x); };
-            pot[(long long)t * nd + c] = i4(A.p);
+            X.pot[(long long)t * nd + c] = i4(A.p);
             if (PGH >= 2) {
-                grad[((long long)t * 2 + 0) * nd + c] = i4(csub(A.u, A.v));
-                grad[((long long)t * 2 + 1) * nd + c] = i4(hk::cmuli(cadd(A.u, A.v)));
+                X.grad[((long long)t * 2 + 0) * nd + c] = i4(csub(A.u, A.v));
+                X.grad[((long long)t * 2 + 1) * nd + c] = i4(hk::cmuli(cadd(A.u, A.v)));
             }
             if (PGH >= 3) {
                 const double2 sm = cadd(A.u2, A.v2), kp = cscal(A.p, 0.5 * k * k);
-                hess[((long long)t * 3 + 0) * nd + c] = i4(csub(sm, kp));
-                hess[((long long)t * 3 + 1) * nd + c] = i4(hk::cmuli(csub(A.u2, A.v2)));
-                hess[((long long)t * 3 + 2) * nd + c] = i4(make_double2(-sm.x - kp.x, -sm.y - kp.y));
+                X.hess[((long long)t * 3 + 0) * nd + c] = i4(csub(sm, kp));
+                X.hess[((long long)t * 3 + 1) * nd + c] = i4(hk::cmuli(csub(A.u2, A.v2)));
+                X.hess[((long long)t * 3 + 2) * nd + c] =
+                    i4(make_double2(-sm.x - kp.x, -sm.y - kp.y));
             }
         }
     }

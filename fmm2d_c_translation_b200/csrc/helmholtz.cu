@@ -934,16 +934,31 @@ __device__ __forceinline__ void acc_terms(Acc &a, const Coefs &C, const DScale &
     }
 }
 
+// One point set of an evaluation.  Sources and targets that want the same
+// outputs go in one launch, the first g0 blocks taking the first set: a call
+// of a few thousand points fills a fraction of the chip with each.
+struct HFarSet {
+    int n = 0;
+    const double2 *pos = nullptr;
+    const int *leaf = nullptr;
+    double2 *pot = nullptr, *grad = nullptr, *hess = nullptr;
+};
+
 template <int PGH>
 __global__ void __launch_bounds__(128) helm_far_kernel(
-    int n, const double2 *__restrict__ pos, const int *__restrict__ leaf,
-    const int *__restrict__ level, const double2 *__restrict__ centers,
-    const int *__restrict__ nlist3, const int *__restrict__ list3, const HLevel *__restrict__ lv,
-    int nlevels, const double2 *__restrict__ mp, const double2 *__restrict__ loc, int nd,
-    double2 zk, int lmax, double2 *__restrict__ pot, double2 *__restrict__ grad,
-    double2 *__restrict__ hess) {
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        const int b = leaf[t];
+    HFarSet s0, HFarSet s1, int g0, const int *__restrict__ level,
+    const double2 *__restrict__ centers, const int *__restrict__ nlist3,
+    const int *__restrict__ list3, const HLevel *__restrict__ lv, int nlevels,
+    const double2 *__restrict__ mp, const double2 *__restrict__ loc, int nd, double2 zk,
+    int lmax) {
+    const bool second = blockIdx.x >= g0;
+    const HFarSet X = second ? s1 : s0;
+    const int n = X.n, blk = blockIdx.x - (second ? g0 : 0),
+              nblk = second ? gridDim.x - g0 : g0;
+    const double2 *__restrict__ pos = X.pos;
+    double2 *__restrict__ pot = X.pot, *__restrict__ grad = X.grad, *__restrict__ hess = X.hess;
+    for (int t = blk * blockDim.x + threadIdx.x; t < n; t += nblk * blockDim.x) {
+        const int b = X.leaf[t];
         const int l = level[b];
         if (l >= lmax) continue;
         const double2 x = pos[t];
@@ -1294,14 +1309,14 @@ constexpr size_t helm_p2p_flat_warp_bytes() {
 
 // KIND 0: any wavenumber; 1, 2, 3: a positive real one with charges, dipoles,
 // both (pair_add_real).
+// Both point sets in one launch when they want the same outputs (nsets 2).
 template <int PGH, int KIND>
 __global__ void __launch_bounds__(kHfWarps * 32) helm_p2p_flat_kernel(
-    int nb, const int *__restrict__ nchild, const int2 *__restrict__ tse,
-    const double2 *__restrict__ pos, const int *__restrict__ nlist1,
-    const int *__restrict__ list1, const int2 *__restrict__ sse, const double2 *__restrict__ src,
-    const double2 *__restrict__ charge, const double2 *__restrict__ dipstr,
-    const double2 *__restrict__ dipvec, int ifc, int ifd, double2 zk, double thresh,
-    double2 *__restrict__ pot, double2 *__restrict__ grad, double2 *__restrict__ hess) {
+    int nb, int nsets, HPointSet set0, HPointSet set1, const int *__restrict__ nchild,
+    const int *__restrict__ nlist1, const int *__restrict__ list1, const int2 *__restrict__ sse,
+    const double2 *__restrict__ src, const double2 *__restrict__ charge,
+    const double2 *__restrict__ dipstr, const double2 *__restrict__ dipvec, int ifc, int ifd,
+    double2 zk, double thresh) {
     constexpr int NO = hf_outs<PGH>();
     extern __shared__ __align__(16) unsigned char hf_smem[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -1313,9 +1328,11 @@ __global__ void __launch_bounds__(kHfWarps * 32) helm_p2p_flat_kernel(
     const double k2 = zk.x * zk.x, thresh2 = thresh * thresh;
     const double2 zero = make_double2(0.0, 0.0);
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (int b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; b < nb; b += nwarps) {
+    for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nb * nsets; w += nwarps) {
+        const bool second = w >= nb;
+        const int b = second ? w - nb : w;
         if (nchild[b] != 0) continue;
-        const int2 tr = tse[b];
+        const int2 tr = (second ? set1 : set0).se[b];
         const int ntot = tr.y - tr.x;
         const int n1 = nlist1[b];
         if (ntot <= 0 || n1 == 0) continue;
@@ -1339,7 +1356,7 @@ __global__ void __launch_bounds__(kHfWarps * 32) helm_p2p_flat_kernel(
         for (int t0 = 0; t0 < ntot; t0 += T0) {
             const int T = min(T0, ntot - t0);
             __syncwarp();
-            if (lane < T) s_tgt[lane] = pos[tr.x + t0 + lane];
+            if (lane < T) s_tgt[lane] = (second ? set1 : set0).pos[tr.x + t0 + lane];
             int B = 1, best = 1 << 30;
             for (int bb = 1; bb * T <= kHfItems; bb++) {
                 const int cost = ((T * bb + 31) >> 5) * ((ns_eff + bb - 1) / bb);
@@ -1416,7 +1433,10 @@ __global__ void __launch_bounds__(kHfWarps * 32) helm_p2p_flat_kernel(
                 }
             }
             if (KIND != 0) tot.scale(make_double2(0.0, 0.25));  // i / 4
-            if (lane < T) store_add<PGH>(tot, (long long)(tr.x + t0 + lane), 1, 0, pot, grad, hess);
+            if (lane < T)
+                store_add<PGH>(tot, (long long)(tr.x + t0 + lane), 1, 0,
+                               (second ? set1 : set0).pot, (second ? set1 : set0).grad,
+                               (second ? set1 : set0).hess);
         }
     }
 }
@@ -1969,52 +1989,65 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
     prof_mark("h_l2l", s);
     // ---- M2P + L2P, then P2P, per point set ----
     const double thresh = hk::cabs_(zk) * T.boxsize[0] * std::ldexp(1.0, -51);
-    for (int set = 0; set < 2; set++) {
-        const HPointSet &X = set == 0 ? P.sset : P.tset;
-        if (X.pgh <= 0 || X.n <= 0) continue;
-        DevBuf<int> leaf(X.n, s);
-        helm_leaf_of_kernel<<<grid_for(nb, 256), 256, 0, s>>>(nb, T.nchild.get(), X.se, leaf.get());
-        FMM_CHECK_LAUNCH();
-        const unsigned g = grid_for(X.n, 128);
-#define HFAR(KERN, PG, K_, LV_)                                                            \
-    KERN<PG><<<g, 128, 0, s>>>(X.n, X.pos, leaf.get(), T.level.get(), T.centers.get(),     \
-                               T.nlist3.get(), T.list3.get(), d_lv.get(), nl, mp.get(),    \
-                               loc.get(), nd, K_, LV_, X.pot, X.grad, X.hess)
-#define HFARP(KERN, K_, LV_)                     \
-    do {                                         \
-        if (X.pgh == 1) HFAR(KERN, 1, K_, LV_);  \
-        else if (X.pgh == 2) HFAR(KERN, 2, K_, LV_); \
-        else HFAR(KERN, 3, K_, LV_);             \
-        FMM_CHECK_LAUNCH();                      \
+    HPointSet sets[2];
+    int nsets = 0;
+    if (P.sset.pgh > 0 && P.sset.n > 0) sets[nsets++] = P.sset;
+    if (P.tset.pgh > 0 && P.tset.n > 0) sets[nsets++] = P.tset;
+    const int together = nsets == 2 && sets[0].pgh == sets[1].pgh ? 2 : 1;
+    for (int first = 0; first < nsets; first += together) {
+        const HPointSet &X = sets[first];
+        const int64_t np = (int64_t)X.n + (together == 2 ? sets[1].n : 0);
+        DevBuf<int> leaf(np, s);
+        HFarSet f[2];
+        int64_t o = 0;
+        for (int i = 0; i < together; i++) {
+            const HPointSet &Y = sets[first + i];
+            f[i] = HFarSet{Y.n, Y.pos, leaf.get() + o, Y.pot, Y.grad, Y.hess};
+            helm_leaf_of_kernel<<<grid_for(nb, 256), 256, 0, s>>>(nb, T.nchild.get(), Y.se,
+                                                                  leaf.get() + o);
+            FMM_CHECK_LAUNCH();
+            o += Y.n;
+        }
+#define HFAR(KERN, PG, G_, ...)                                                              \
+    do {                                                                                     \
+        const unsigned g0 = grid_for((int64_t)f[0].n * (G_), 128);                           \
+        const unsigned g1 = together == 2 ? grid_for((int64_t)f[1].n * (G_), 128) : 0;       \
+        KERN<PG><<<g0 + g1, 128, 0, s>>>(f[0], f[1], (int)g0, T.level.get(), T.centers.get(), \
+                                         T.nlist3.get(), T.list3.get(), d_lv.get(), nl,      \
+                                         mp.get(), loc.get(), nd, __VA_ARGS__);              \
+    } while (0)
+#define HFARP(KERN, G_, ...)                               \
+    do {                                                   \
+        if (X.pgh == 1) HFAR(KERN, 1, G_, __VA_ARGS__);    \
+        else if (X.pgh == 2) HFAR(KERN, 2, G_, __VA_ARGS__); \
+        else HFAR(KERN, 3, G_, __VA_ARGS__);               \
+        FMM_CHECK_LAUNCH();                                \
     } while (0)
         // (every leaf takes exactly one of the two, which is the first
         // writer of its points' outputs)
-        if (lreal > 0) HFARP(helm_far_kernel, zk, lreal);
-        if (lreal <= nl) HFARP(helm_far_real_kernel, zk.x, lreal);
+        if (lreal > 0) HFARP(helm_far_kernel, 1, zk, lreal);
+        const int G = far_lanes(np);
+        if (lreal <= nl) HFARP(helm_far_real_kernel, G, G, zk.x, lreal);
 #undef HFARP
 #undef HFAR
-        prof_mark(set == 0 ? "h_eval_src" : "h_eval_trg", s);
+        prof_mark(first == 0 ? "h_eval_src" : "h_eval_trg", s);
         if (!P.ifnear) continue;
-#define HP2P(PG, RK)                                                                        \
-    helm_p2p_kernel<PG, RK><<<g, 128, 0, s>>>(X.n, X.pos, leaf.get(), T.nlist1.get(),       \
-                                              T.list1.get(), T.srcse.get(), P.src, P.charge, \
-                                              P.dipstr, P.dipvec, ifc, ifd, nd, zk, thresh,  \
-                                              X.pot, X.grad, X.hess)
+        // one warp per leaf (nd = 1; FMM2D_B200_HELM_P2P=point keeps a thread per point)
+        const char *pm = getenv("FMM2D_B200_HELM_P2P");
+        if (nd == 1 && !(pm && !strcmp(pm, "point"))) {
 #define HP2PF(PG, KD)                                                                        \
     do {                                                                                     \
         constexpr size_t sm = kHfWarps * helm_p2p_flat_warp_bytes<PG>();                     \
         auto kern = helm_p2p_flat_kernel<PG, KD>;                                            \
         raise_smem_limit((const void *)kern, sm);                                            \
-        const int gw = std::max(1, std::min((nb + kHfWarps - 1) / kHfWarps, kNumSM * 16));   \
-        kern<<<gw, kHfWarps * 32, sm, s>>>(nb, T.nchild.get(), X.se, X.pos, T.nlist1.get(),   \
-                                          T.list1.get(), T.srcse.get(), P.src, P.charge,      \
-                                          P.dipstr, P.dipvec, ifc, ifd, zk, thresh, X.pot,    \
-                                          X.grad, X.hess);                                    \
+        const int gw = std::max(1, std::min((nb * together + kHfWarps - 1) / kHfWarps,       \
+                                            kNumSM * 16));                                   \
+        kern<<<gw, kHfWarps * 32, sm, s>>>(nb, together, X, sets[first + together - 1],      \
+                                          T.nchild.get(), T.nlist1.get(), T.list1.get(),     \
+                                          T.srcse.get(), P.src, P.charge, P.dipstr, P.dipvec, \
+                                          ifc, ifd, zk, thresh);                             \
+        FMM_CHECK_LAUNCH();                                                                  \
     } while (0)
-        // one warp per leaf (nd = 1; FMM2D_B200_HELM_P2P=point keeps a thread per point)
-        const char *pm = getenv("FMM2D_B200_HELM_P2P");
-        const bool flat = nd == 1 && !(pm && !strcmp(pm, "point"));
-        if (flat) {
 #define HP2PK(KD)                          \
     do {                                   \
         if (X.pgh == 1) HP2PF(1, KD);      \
@@ -2030,19 +2063,30 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
                 else HP2PK(1);
             }
 #undef HP2PK
-        } else if (realk) {
-            if (X.pgh == 1) HP2P(1, true);
-            else if (X.pgh == 2) HP2P(2, true);
-            else HP2P(3, true);
-        } else {
-            if (X.pgh == 1) HP2P(1, false);
-            else if (X.pgh == 2) HP2P(2, false);
-            else HP2P(3, false);
-        }
-#undef HP2P
 #undef HP2PF
-        FMM_CHECK_LAUNCH();
-        prof_mark(set == 0 ? "h_p2p_src" : "h_p2p_trg", s);
+        } else {
+            for (int i = 0; i < together; i++) {
+                const HPointSet &Y = sets[first + i];
+                const unsigned g = grid_for(Y.n, 128);
+#define HP2P(PG, RK)                                                                        \
+    helm_p2p_kernel<PG, RK><<<g, 128, 0, s>>>(Y.n, Y.pos, f[i].leaf, T.nlist1.get(),        \
+                                              T.list1.get(), T.srcse.get(), P.src, P.charge, \
+                                              P.dipstr, P.dipvec, ifc, ifd, nd, zk, thresh,  \
+                                              Y.pot, Y.grad, Y.hess)
+                if (realk) {
+                    if (Y.pgh == 1) HP2P(1, true);
+                    else if (Y.pgh == 2) HP2P(2, true);
+                    else HP2P(3, true);
+                } else {
+                    if (Y.pgh == 1) HP2P(1, false);
+                    else if (Y.pgh == 2) HP2P(2, false);
+                    else HP2P(3, false);
+                }
+#undef HP2P
+                FMM_CHECK_LAUNCH();
+            }
+        }
+        prof_mark(first == 0 ? "h_p2p_src" : "h_p2p_trg", s);
     }
 }
 
