@@ -658,36 +658,60 @@ __global__ void __launch_bounds__(256) helm_m2l_kernel(
 // rs^|i| (pw[|i|]) scales the sum; the host takes it where those powers
 // stay far inside the FP64 range.  Otherwise the weight is applied per
 // term, from the case split above.
+//
+// All levels go in one launch (per form): a level is a few blocks at the top
+// of the tree and near the leaves of an adaptive one, and its chain of 27
+// slots of 2p + 1 steps took 20 to 30 us per level, two to three launches each
+// (1e5 clustered points, 10 levels: 0.97 ms).  A level's slots are dealt to
+// nslice slices of blocks so that no block's chain is longer than an even share
+// of the whole work (slices_for); a slice writes its own partial sums, added in
+// slice order by helm_m2l_sum_kernel.
 constexpr int kHTile = 4;  // boxes per tile (8 measured slower: registers)
 constexpr int kHGroups = 8;
-struct HTiles {
+constexpr int kHJobs = 32;  // levels per launch
+struct HJob {
     int tb[5];     // tiles of the level's four segments: [tb[c], tb[c + 1])
     int start[4];  // first target of each segment
     int count[4];  // targets of each segment
+    int l, p, G;   // level, order, tiles per block
+    int blk0, nblk, nslice;  // first block, blocks per slice, slices
+    int nq;                  // targets of the level
+    long long part0;         // its partial sums: [slice][target][(2p + 1) nd]
+    long long sum0;          // its outputs among those of the split levels
+    long long off, ncoef;    // its block of the expansions
+    const double2 *T;
+    const double *pw;
+};
+struct HJobs {
+    int n = 0;
+    HJob j[kHJobs];
 };
 
-template <bool SC, bool SPLIT>
+template <bool SC>
 __global__ void __launch_bounds__(128, 5) helm_m2l_tile_kernel(
-    HTiles lt, const int *__restrict__ boxes, const int *__restrict__ slots,
-    const int2 *__restrict__ dxy, int nd, const HLevel *__restrict__ lv, int l,
-    const double2 *__restrict__ T, const double *__restrict__ pw,
-    const double2 *__restrict__ zero, const double2 *__restrict__ mp,
-    double2 *__restrict__ loc, double2 *__restrict__ part) {
+    const __grid_constant__ HJobs jobs, const int *__restrict__ boxes,
+    const int *__restrict__ slots, const int2 *__restrict__ dxy, int nd,
+    const HLevel *__restrict__ lv, const double2 *__restrict__ zero,
+    const double2 *__restrict__ mp, double2 *__restrict__ loc, double2 *__restrict__ part) {
     constexpr int R = kHTile;
     __shared__ int s_src[kHGroups][R][27];
     __shared__ int s_trg[kHGroups][R];
     __shared__ int s_q[kHGroups][R];
     __shared__ int s_cp[kHGroups];
-    const HLevel L = lv[l];
+    int ji = 0;
+    while (ji + 1 < jobs.n && (int)blockIdx.x >= jobs.j[ji + 1].blk0) ji++;
+    const HJob &lt = jobs.j[ji];
+    const HLevel L = lv[lt.l];
+    const double2 *__restrict__ T = lt.T;
+    const double *__restrict__ pw = lt.pw;
     const int p = L.p, tw = 4 * p + 1, wn = (p + 1) * nd;  // a thread per two outputs
-    const int G = wn <= (int)blockDim.x ? min(kHGroups, (int)blockDim.x / wn) : 1;
-    const int ntiles = lt.tb[4] - lt.tb[0];
-    // slots [k0, k1) of slice blockIdx.y; with several slices each writes
-    // its own partial sums (part: [slice][level target][(2p + 1) nd])
-    const int k0 = SPLIT ? blockIdx.y * 27 / gridDim.y : 0;
-    const int k1 = SPLIT ? (blockIdx.y + 1) * 27 / gridDim.y : 27;
-    for (int base = blockIdx.x * G; base < ntiles; base += gridDim.x * G) {
-        __syncthreads();  // the previous pass's reads of the shared tables are done
+    const int G = lt.G, ntiles = lt.tb[4] - lt.tb[0];
+    const int rel = blockIdx.x - lt.blk0, slice = rel / lt.nblk;
+    const bool split = lt.nslice > 1;
+    // slots [k0, k1) of this slice
+    const int k0 = slice * 27 / lt.nslice, k1 = (slice + 1) * 27 / lt.nslice;
+    const int base = (rel - slice * lt.nblk) * G;
+    {
         for (int e = threadIdx.x; e < G * R * 27; e += blockDim.x) {
             const int g = e / (R * 27), r = (e / 27) % R, k = e % 27;
             const int tile = base + g;
@@ -769,9 +793,9 @@ __global__ void __launch_bounds__(128, 5) helm_m2l_tile_kernel(
                 if (s_trg[g][r] < 0) continue;
                 const double2 v0 = SC ? cscal(acc0[r], sc0) : acc0[r];
                 const double2 v1 = SC ? cscal(acc1[r], sc1) : acc1[r];
-                if (SPLIT) {  // this slice's partial sums, added in order by helm_m2l_sum_kernel
-                    const int nq = lt.start[3] + lt.count[3] - lt.start[0];
-                    double2 *op = part + ((size_t)blockIdx.y * nq + s_q[g][r]) * (2 * p + 1) * nd +
+                if (split) {
+                    double2 *op = part + lt.part0 +
+                                  ((size_t)slice * lt.nq + s_q[g][r]) * (2 * p + 1) * nd +
                                   (size_t)(i0 + p) * nd + c;
                     op[0] = v0;
                     if (two) op[nd] = v1;
@@ -786,32 +810,58 @@ __global__ void __launch_bounds__(128, 5) helm_m2l_tile_kernel(
 }
 
 // Sum of the slices' partial M2L sums of helm_m2l_tile_kernel, in slice
-// order, into the local expansions of the level's targets.
+// order, into the local expansions of the split levels' targets.
 __global__ void __launch_bounds__(256) helm_m2l_sum_kernel(
-    int nq, int wf, int nslice, const double2 *__restrict__ part, const int *__restrict__ boxes,
-    int q_lo, const HLevel *__restrict__ lv, int l, int nd, double2 *__restrict__ loc) {
-    const HLevel L = lv[l];
-    const long long n = (long long)nq * wf;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
+    const __grid_constant__ HJobs jobs, long long total, const double2 *__restrict__ part,
+    const int *__restrict__ boxes, const HLevel *__restrict__ lv, int nd,
+    double2 *__restrict__ loc) {
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
          t += (long long)gridDim.x * blockDim.x) {
-        const int q = (int)(t / wf), o = (int)(t - (long long)q * wf);
+        int ji = 0;
+        for (int i = 1; i < jobs.n; i++)
+            if (jobs.j[i].nslice > 1 && jobs.j[i].sum0 <= t) ji = i;
+        if (jobs.j[ji].nslice <= 1) continue;
+        const HJob &J = jobs.j[ji];
+        const HLevel L = lv[J.l];
+        const int wf = (2 * L.p + 1) * nd;
+        const long long n = (long long)J.nq * wf, u = t - J.sum0;
+        const int q = (int)(u / wf), o = (int)(u - (long long)q * wf);
         double2 acc = make_double2(0.0, 0.0);
-        for (int y = 0; y < nslice; y++) acc = cadd(acc, part[(size_t)y * n + t]);
-        double2 *op = coef0(loc, L, boxes[q_lo + q], nd) - (long long)L.p * nd + o;
+#pragma unroll 4
+        for (int y = 0; y < J.nslice; y++) acc = cadd(acc, part[J.part0 + y * n + u]);
+        double2 *op = coef0(loc, L, boxes[J.start[0] + q], nd) - (long long)L.p * nd + o;
         *op = cadd(*op, acc);
     }
 }
 
-// Scaled multipoles of the level-l boxes for the scaled M2L form:
+// Scaled multipoles of the jobs' levels for the scaled M2L form:
 // out = mp * rs^|j| for coefficient j (pw[|j|]).
-__global__ void __launch_bounds__(256) helm_scale_mp_kernel(
-    long long off, long long n, int p, int nd, const double *__restrict__ pw,
-    const double2 *__restrict__ mp, double2 *__restrict__ out) {
-    const int wn = (2 * p + 1) * nd;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
+__global__ void __launch_bounds__(256) helm_scale_mp_kernel(const __grid_constant__ HJobs jobs,
+                                                            long long total, int nd,
+                                                            const double2 *__restrict__ mp,
+                                                            double2 *__restrict__ out) {
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
          t += (long long)gridDim.x * blockDim.x) {
-        const int j = (int)(t % wn) / nd - p;
-        out[off + t] = cscal(mp[off + t], pw[abs(j)]);
+        long long u = t;
+        int ji = 0;
+        while (u >= jobs.j[ji].ncoef) u -= jobs.j[ji++].ncoef;
+        const HJob &J = jobs.j[ji];
+        const int j = (int)(u % ((2 * J.p + 1) * nd)) / nd - J.p;
+        out[J.off + u] = cscal(mp[J.off + u], J.pw[abs(j)]);
+    }
+}
+
+// Slices of the jobs' levels: a block's chain is its slots' 2p + 1 steps each,
+// and the chip runs kNumSM * 5 blocks at once; a chain longer than an even
+// share of all the steps (or than 240 steps, about 10 us, when there is less
+// work than that) is cut.
+void slices_for(HJobs &J) {
+    double steps = 0.0;
+    for (int i = 0; i < J.n; i++) steps += (double)J.j[i].nblk * 27 * (2 * J.j[i].p + 1);
+    const double share = std::max(240.0, steps / (kNumSM * 5));
+    for (int i = 0; i < J.n; i++) {
+        const double chain = 27.0 * (2 * J.j[i].p + 1);
+        J.j[i].nslice = std::max(1, std::min(27, (int)std::ceil(chain / share)));
     }
 }
 
@@ -1851,6 +1901,7 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
     if (tc) FMM_CUDA(cudaMemsetAsync(tc_err.get(), 0, sizeof(int), s));
     bool tc_used = false;
     std::vector<char> tc_lev(nl + 1, 0);
+    std::vector<HJob> jobs[2];  // levels of the tile form: unscaled, scaled
     const bool hf_on = !(getenv("FMM2D_B200_HELM_HF") && !strcmp(getenv("FMM2D_B200_HELM_HF"), "0"));
     for (int l = 2; l <= nl; l++) {
         if (!hl[l].flag) continue;
@@ -1878,7 +1929,7 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
         }
         if (tiled) {
             if (spl.ntiles == 0) continue;
-            HTiles ht;
+            HJob ht;
             const int g0 = 4 * (l - 2);
             for (int c = 0; c <= 4; c++) ht.tb[c] = spl.tile_base[g0 + c];
             for (int c = 0; c < 4; c++) {
@@ -1887,43 +1938,20 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
             }
             const int ntl = ht.tb[4] - ht.tb[0];
             if (ntl == 0) continue;
-            // 128 threads at most: groups of wn threads (two outputs
-            // each), one tile per group
+            // 128 threads: groups of wn threads (two outputs each), one tile
+            // per group
             const int wn = (hl[l].p + 1) * nd;
-            const int G = wn <= 128 ? std::min(kHGroups, 128 / wn) : 1;
-            const int threads = std::min(128, (G * wn + 31) / 32 * 32);
-            const int nblk = (ntl + G - 1) / G;
-            // levels with fewer blocks than SMs (few boxes, high
-            // orders) split the 27 slots over slices of blocks
-            const int nslice = nblk < kNumSM ? std::min(27, std::max(2, 2 * kNumSM / nblk)) : 1;
-            const dim3 grid(std::min(nblk, kNumSM * 64), nslice);
-            const int q_lo = ht.start[0], nq = ht.start[3] + ht.count[3] - q_lo;
-            const int wf = (2 * hl[l].p + 1) * nd;
-            DevBuf<double2> part(nslice > 1 ? (size_t)nslice * nq * wf : 0, s);
-            const double *pw = d_rt.get() + lt[l].m2l_pw;
-            if (lt[l].sc_ok) {
-                if (!mps.get()) mps.alloc(std::max<long long>(off, 1), s);
-                const long long n = (long long)(T.lend[l] - T.lstart[l]) * (2 * hl[l].p + 1) * nd;
-                helm_scale_mp_kernel<<<grid_for(n, 256), 256, 0, s>>>(hl[l].off, n, hl[l].p, nd,
-                                                                      pw, mp.get(), mps.get());
-                FMM_CHECK_LAUNCH();
-#define HM2L(SC_, SPLIT_, TAB_, MP_)                                                       \
-    helm_m2l_tile_kernel<SC_, SPLIT_><<<grid, threads, 0, s>>>(                            \
-        ht, spl.boxes, spl.slots, spl.dxy, nd, d_lv.get(), l, TAB_, pw, zero.get(), MP_, \
-        loc.get(), part.get())
-                if (nslice > 1) HM2L(true, true, d_ct.get() + lt[l].m2l_sc, mps.get());
-                else HM2L(true, false, d_ct.get() + lt[l].m2l_sc, mps.get());
-            } else {
-                if (nslice > 1) HM2L(false, true, d_ct.get() + lt[l].m2l, mp.get());
-                else HM2L(false, false, d_ct.get() + lt[l].m2l, mp.get());
-#undef HM2L
-            }
-            FMM_CHECK_LAUNCH();
-            if (nslice > 1) {
-                helm_m2l_sum_kernel<<<grid_for((int64_t)nq * wf, 256), 256, 0, s>>>(
-                    nq, wf, nslice, part.get(), spl.boxes, q_lo, d_lv.get(), l, nd, loc.get());
-                FMM_CHECK_LAUNCH();
-            }
+            ht.l = l;
+            ht.p = hl[l].p;
+            ht.G = wn <= 128 ? std::min(kHGroups, 128 / wn) : 1;
+            ht.nblk = (ntl + ht.G - 1) / ht.G;
+            ht.nq = ht.start[3] + ht.count[3] - ht.start[0];
+            ht.off = hl[l].off;
+            ht.ncoef = (long long)(T.lend[l] - T.lstart[l]) * (2 * hl[l].p + 1) * nd;
+            const bool sc = lt[l].sc_ok;
+            ht.T = d_ct.get() + (sc ? lt[l].m2l_sc : lt[l].m2l);
+            ht.pw = d_rt.get() + lt[l].m2l_pw;
+            jobs[sc].push_back(ht);
             continue;
         }
         const int lo = T.lstart[l], hi = T.lend[l];
@@ -1934,6 +1962,47 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
             d_rt.get() + lt[l].m2l_pw, mp.get(), loc.get());
         FMM_CHECK_LAUNCH();
     }
+    for (int sc = 0; sc < 2; sc++)
+        for (size_t first = 0; first < jobs[sc].size(); first += kHJobs) {
+            HJobs J;
+            J.n = (int)std::min<size_t>(kHJobs, jobs[sc].size() - first);
+            for (int i = 0; i < J.n; i++) J.j[i] = jobs[sc][first + i];
+            slices_for(J);
+            long long blocks = 0, part_n = 0, sum_n = 0, mp_n = 0;
+            for (int i = 0; i < J.n; i++) {
+                HJob &h = J.j[i];
+                const long long out = (long long)h.nq * (2 * h.p + 1) * nd;
+                h.blk0 = (int)blocks;
+                h.part0 = part_n;
+                h.sum0 = sum_n;
+                blocks += (long long)h.nblk * h.nslice;
+                if (h.nslice > 1) {
+                    part_n += out * h.nslice;
+                    sum_n += out;
+                }
+                mp_n += h.ncoef;
+            }
+            DevBuf<double2> part(part_n, s);
+            if (sc) {
+                if (!mps.get()) mps.alloc(std::max<long long>(off, 1), s);
+                helm_scale_mp_kernel<<<grid_for(mp_n, 256), 256, 0, s>>>(J, mp_n, nd, mp.get(),
+                                                                         mps.get());
+                FMM_CHECK_LAUNCH();
+                helm_m2l_tile_kernel<true><<<(unsigned)blocks, 128, 0, s>>>(
+                    J, spl.boxes, spl.slots, spl.dxy, nd, d_lv.get(), zero.get(), mps.get(),
+                    loc.get(), part.get());
+            } else {
+                helm_m2l_tile_kernel<false><<<(unsigned)blocks, 128, 0, s>>>(
+                    J, spl.boxes, spl.slots, spl.dxy, nd, d_lv.get(), zero.get(), mp.get(),
+                    loc.get(), part.get());
+            }
+            FMM_CHECK_LAUNCH();
+            if (sum_n > 0) {
+                helm_m2l_sum_kernel<<<grid_for(sum_n, 256), 256, 0, s>>>(
+                    J, sum_n, part.get(), spl.boxes, d_lv.get(), nd, loc.get());
+                FMM_CHECK_LAUNCH();
+            }
+        }
     prof_mark("h_m2l", s);
     if (profiling_enabled()) {
         // F_M2L = 8 sum_l pairs_l (2 p_l + 1)^2 nd, and the part on the tensor cores
