@@ -1303,6 +1303,7 @@ __device__ __forceinline__ void store_add(const Acc &a, long long t, int nd, int
 }
 
 #include "helm_real.cuh"
+#include "helm_tables.cuh"
 
 // P2P over list 1 for one point set (the outputs already hold the far field).
 template <int PGH, bool REALK>
@@ -1547,78 +1548,15 @@ unsigned grid_for(int64_t work, int block) {
     return (unsigned)g;
 }
 
-// The per-level translation tables (host).
-// T(m), m = -N..N, for the shift from center1 to center2 = center1 + d:
-// T(0) = B_0, T(m) = zmul^m B_m, T(-m) = (-1)^m zinv^m B_m with
-// zmul = e^{-i (atan2(d) - pi)} and B the scaled J (M2M, L2L) or H (M2L)
-// sequence of k |d| (h2dmpmp / h2dlocloc / h2dmploc, helmrouts2d.c:736-1042).
-void shift_table(double2 zk, double dx, double dy, int N, double rs1, bool hankel,
-                 double2 *T) {
-    const double r = std::sqrt(dx * dx + dy * dy);
-    const double pi = 4.0 * std::atan(1.0);
-    const double th = ((dx == 0.0 && dy == 0.0) ? 0.0 : std::atan2(dy, dx)) - pi;
-    const double2 z = cscal(zk, r);
-    std::vector<double2> B(N + 4);
-    if (hankel)
-        helm_hvec(N + 1, z, rs1, B.data());
-    else
-        helm_jvec(N + 3, z, rs1, B.data());
-    const double2 zmul = make_double2(std::cos(th), -std::sin(th));
-    const double2 zinv = make_double2(zmul.x, -zmul.y);
-    double2 *T0 = T + N;
-    T0[0] = B[0];
-    double2 t1 = zmul, t2 = make_double2(-zinv.x, -zinv.y);
-    for (int j = 1; j <= N; j++) {
-        T0[j] = cmul(t1, B[j]);
-        T0[-j] = cmul(t2, B[j]);
-        t1 = cmul(t1, zmul);
-        t2 = cscal(cmul(t2, zinv), -1.0);
-    }
-}
-
-}  // namespace
-
-namespace {
-
-// Host translation tables of one evaluation.  Layout per level: M2M
-// [4][2N+1] + S + pw, L2L likewise, M2L [49][4p+1] + pw (+ the scaled M2L
-// table where it applies).
-struct LevTab {
-    size_t m2m = 0, m2m_s = 0, m2m_pw = 0, l2l = 0, l2l_s = 0, l2l_pw = 0, m2l = 0, m2l_pw = 0;
-    size_t m2l_sc = 0;   // M2L table of the scaled form, T_q rs^-|q|
-    // folded M2M and L2L: child 0's table T_q r^|q| and the factors of the
-    // input and output orders
-    size_t m2m_f = 0, m2m_in = 0, m2m_out = 0, l2l_f = 0, l2l_in = 0, l2l_out = 0;
-    bool m2m_ok = false, l2l_ok = false;
-    bool sc_ok = false;  // the scaled form applies on this level
-    double m2l_max = 0;  // largest |T_q| of the M2L table (tensor-core form's scale)
+// Places of a level's tables (HTabLev) and what the host decides by.
+struct LevTab : HTabLev {
+    bool m2m_ok = false, l2l_ok = false;  // the folded shifts apply
+    bool sc_ok = false;   // the scaled M2L form applies
+    double m2l_max = 0;   // bound of |T_q| of the M2L table (tensor-core form's scale)
 };
-struct HTables {
-    std::vector<LevTab> lt;
-    std::vector<double2> ct;  // complex tables
-    std::vector<double> rt;   // real tables
-};
-using HTabKey = std::tuple<double, double, double, double, int>;  // zk, eps, root box, depth
 
-// The last kHTabCache table sets, shared by the threads of the process.
-constexpr size_t kHTabCache = 16;
-std::mutex g_htab_mu;
-std::vector<std::pair<HTabKey, std::shared_ptr<HTables>>> g_htab;
-
-std::shared_ptr<HTables> htables_find(const HTabKey &k) {
-    std::lock_guard<std::mutex> lock(g_htab_mu);
-    for (auto &e : g_htab)
-        if (e.first == k) return e.second;
-    return nullptr;
-}
-
-void htables_store(const HTabKey &k, const std::shared_ptr<HTables> &t) {
-    std::lock_guard<std::mutex> lock(g_htab_mu);
-    for (auto &e : g_htab)
-        if (e.first == k) return;
-    if (g_htab.size() >= kHTabCache) g_htab.erase(g_htab.begin());
-    g_htab.emplace_back(k, t);
-}
+// The seven lengths of list-2 offsets, in box sides squared.
+constexpr int kM2LLengths[7] = {4, 5, 8, 9, 10, 13, 18};
 
 }  // namespace
 
@@ -1652,148 +1590,97 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
     DevBuf<double2> mp(std::max<long long>(off, 1), s), loc(std::max<long long>(off, 1), s);
     mp.zero(s);
     loc.zero(s);
-    // ---- translation tables (kept for calls with the same zk, eps, root
-    // box and depth, which fix every level's order, scale and offsets) ----
-    const HTabKey tkey{zk.x, zk.y, P.eps, T.boxsize[0], nl};
-    std::shared_ptr<HTables> tabs = htables_find(tkey);
-    if (!tabs) {
-        tabs = std::make_shared<HTables>();
-        std::vector<LevTab> &lt = tabs->lt;
-        std::vector<double2> &ct = tabs->ct;
-        std::vector<double> &rt = tabs->rt;
-        lt.resize(nl + 1);
-        auto powtab = [&](double r, int n) {
-            const size_t o = rt.size();
-            double v = 1.0;
-            for (int e = 0; e <= n; e++) {
-                rt.push_back(v);
-                v *= r;
+    // ---- translation tables ----
+    // Folded shifts: boxes per block so that a level gives every SM a few
+    // blocks; levels whose staging does not fit into shared memory (orders
+    // above about 120) keep the general kernels
+    auto fold_range = [&](int n) {
+        return std::max(4, std::min(kShRange, (n + kNumSM * 8 - 1) / (kNumSM * 8)));
+    };
+    auto fold_smem = [&](int n1, int n2, int per) {
+        return ((size_t)2 * (n1 + n2) + 1 + (size_t)shift_units(2 * n2 + 1) * (2 * n1 + 1) * per) *
+               sizeof(double2);
+    };
+    constexpr size_t kFoldSmem = 200 * 1024;
+    // whether scale r^N stays inside 1e+-220
+    auto in_range = [](double r, int N) {
+        return r > 0.0 && N * std::fabs(std::log10(r)) <= 220.0;
+    };
+    std::vector<LevTab> lt(nl + 1);
+    long long ct_n = 0, rt_n = 0;
+    auto place = [](long long &n, long long len) {
+        const long long o = n;
+        n += len;
+        return o;
+    };
+    std::vector<double2> hv;
+    for (int l = 2; l <= nl; l++) {
+        const HLevel &L = hl[l], &C = hl[std::min(l + 1, nl)];
+        LevTab &t = lt[l];
+        t.p = L.p;
+        t.pc = C.p;
+        t.Nm = t.Nl = C.p + L.p;
+        t.N2 = 2 * L.p;
+        t.bs = T.boxsize[l];
+        t.hb = l < nl ? T.boxsize[l + 1] / 2.0 : 0.0;
+        t.rl = L.rs;
+        t.rc = C.rs;
+        t.m2m = t.m2m_f = t.l2l = t.l2l_f = t.m2l_sc = -1;
+        t.m2m_s = t.m2m_pw = t.m2m_in = t.m2m_out = -1;
+        t.l2l_s = t.l2l_pw = t.l2l_in = t.l2l_out = -1;
+        if (l < nl) {
+            const long long len = 2 * t.Nm + 1;
+            t.m2m_ok = in_range(C.rs, t.Nm) && fold_smem(C.p, L.p, 4) <= kFoldSmem;
+            t.l2l_ok = in_range(L.rs, t.Nl) && fold_smem(L.p, C.p, 1) <= kFoldSmem;
+            if (t.m2m_ok) {
+                t.m2m_f = place(ct_n, len);
+                t.m2m_in = place(rt_n, C.p + 1);
+                t.m2m_out = place(rt_n, L.p + 1);
+            } else {
+                t.m2m = place(ct_n, 4 * len);
+                t.m2m_s = place(rt_n, L.p + 1);
+                t.m2m_pw = place(rt_n, 2 * C.p + 1);
             }
-            return o;
-        };
-        // The folded form of the shift whose child-0 table (2N + 1 entries)
-        // is at ct[tab] and whose output factors S are at rt[sf]: table
-        // T_q r^|q|, input order j times r^(sign |j|), output order i times
-        // S_i r^(-sign |i|); false where a power leaves 1e+-220.
-        auto folded = [&](size_t tab, size_t sf, int N, int n1, int n2, double r, int sign,
-                          size_t &o_tab, size_t &o_in, size_t &o_out) {
-            if (!(r > 0.0) || N * std::fabs(std::log10(r)) > 220.0) return false;
-            std::vector<double> pw(N + 1);
-            pw[0] = 1.0;
-            for (int e = 1; e <= N; e++) pw[e] = pw[e - 1] * r;
-            o_tab = ct.size();
-            for (int q = -N; q <= N; q++) ct.push_back(cscal(ct[tab + q + N], pw[std::abs(q)]));
-            o_in = rt.size();
-            for (int j = 0; j <= n1; j++) rt.push_back(sign > 0 ? pw[j] : 1.0 / pw[j]);
-            o_out = rt.size();
-            for (int i = 0; i <= n2; i++)
-                rt.push_back(rt[sf + i] * (sign > 0 ? 1.0 / pw[i] : pw[i]));
-            return true;
-        };
-        for (int l = 2; l <= nl; l++) {
-            const HLevel &L = hl[l];
-            if (l + 1 <= nl) {
-                const HLevel &C = hl[l + 1];
-                const double hb = T.boxsize[l + 1] / 2.0;
-                // M2M: child (scale r1) -> parent (scale r2), d = parent - child
-                {
-                    const int n1 = C.p, n2 = L.p, N = n1 + n2;
-                    lt[l].m2m = ct.size();
-                    ct.resize(ct.size() + (size_t)4 * (2 * N + 1));
-                    for (int cs = 0; cs < 4; cs++) {
-                        const double sx = (cs & 1) ? 1.0 : -1.0, sy = (cs & 2) ? 1.0 : -1.0;
-                        shift_table(zk, -sx * hb, -sy * hb, N, C.rs, false,
-                                    ct.data() + lt[l].m2m + (size_t)cs * (2 * N + 1));
-                    }
-                    lt[l].m2m_s = rt.size();
-                    double f = 1.0;
-                    for (int i = 0; i <= n2; i++) {
-                        rt.push_back(f);
-                        f = f * C.rs / L.rs;
-                    }
-                    lt[l].m2m_pw = powtab(C.rs, 2 * n1);
-                    lt[l].m2m_ok = folded(lt[l].m2m, lt[l].m2m_s, N, n1, n2, C.rs, 1, lt[l].m2m_f,
-                                          lt[l].m2m_in, lt[l].m2m_out);
-                }
-                // L2L: parent (scale r1) -> child (scale r2), d = child - parent
-                {
-                    const int n1 = L.p, n2 = C.p, N = n1 + n2;
-                    lt[l].l2l = ct.size();
-                    ct.resize(ct.size() + (size_t)4 * (2 * N + 1));
-                    for (int cs = 0; cs < 4; cs++) {
-                        const double sx = (cs & 1) ? 1.0 : -1.0, sy = (cs & 2) ? 1.0 : -1.0;
-                        shift_table(zk, sx * hb, sy * hb, N, L.rs, false,
-                                    ct.data() + lt[l].l2l + (size_t)cs * (2 * N + 1));
-                    }
-                    lt[l].l2l_s = rt.size();
-                    double f = 1.0;
-                    for (int i = 0; i <= n2; i++) {
-                        rt.push_back(f);
-                        f = f * C.rs / L.rs;
-                    }
-                    lt[l].l2l_pw = powtab(L.rs, 2 * n2);
-                    lt[l].l2l_ok = folded(lt[l].l2l, lt[l].l2l_s, N, n1, n2, L.rs, -1, lt[l].l2l_f,
-                                          lt[l].l2l_in, lt[l].l2l_out);
-                }
-            }
-            // M2L: d = target - source = (ix, iy) * boxsize
-            {
-                const int p = L.p, N = 2 * p;
-                lt[l].m2l = ct.size();
-                ct.resize(ct.size() + (size_t)49 * (2 * N + 1), make_double2(0.0, 0.0));
-                for (int iy = -3; iy <= 3; iy++)
-                    for (int ix = -3; ix <= 3; ix++) {
-                        if (std::abs(ix) <= 1 && std::abs(iy) <= 1) continue;
-                        shift_table(zk, ix * T.boxsize[l], iy * T.boxsize[l], N, L.rs, true,
-                                    ct.data() + lt[l].m2l + (size_t)((iy + 3) * 7 + (ix + 3)) * (2 * N + 1));
-                    }
-                lt[l].m2l_pw = powtab(L.rs, 2 * p);
-                {
-                    double mx = 0.0;
-                    const size_t n = (size_t)49 * (2 * N + 1);
-                    for (size_t e = 0; e < n; e++) {
-                        const double2 v = ct[lt[l].m2l + e];
-                        mx = std::max(mx, std::max(std::fabs(v.x), std::fabs(v.y)));
-                    }
-                    lt[l].m2l_max = mx;
-                }
-                // the scaled form where rs^(2p) and the scaled entries stay
-                // inside 1e-250 .. 1e250
-                if (L.rs > 0.0 && 2.0 * p * std::fabs(std::log10(L.rs)) < 250.0) {
-                    const size_t n = (size_t)49 * (2 * N + 1), o = ct.size();
-                    ct.resize(o + n);
-                    bool fine = true;
-                    std::vector<double> f(N + 1);  // rs^-q
-                    f[0] = 1.0;
-                    for (int q = 1; q <= N; q++) f[q] = f[q - 1] / L.rs;
-                    for (size_t e = 0; e < n; e++) {
-                        const int q = (int)(e % (2 * N + 1)) - N;
-                        const double2 v = cscal(ct[lt[l].m2l + e], f[std::abs(q)]);
-                        if (!(std::fabs(v.x) <= 1e250 && std::fabs(v.y) <= 1e250)) fine = false;
-                        ct[o + e] = v;
-                    }
-                    if (fine) {
-                        lt[l].m2l_sc = o;
-                        lt[l].sc_ok = true;
-                    } else {
-                        ct.resize(o);
-                    }
-                }
+            if (t.l2l_ok) {
+                t.l2l_f = place(ct_n, len);
+                t.l2l_in = place(rt_n, L.p + 1);
+                t.l2l_out = place(rt_n, C.p + 1);
+            } else {
+                t.l2l = place(ct_n, 4 * len);
+                t.l2l_s = place(rt_n, C.p + 1);
+                t.l2l_pw = place(rt_n, 2 * C.p + 1);
             }
         }
-        htables_store(tkey, tabs);
+        const long long len = 2 * t.N2 + 1;
+        t.m2l = place(ct_n, 49 * len);
+        t.m2l_pw = place(rt_n, 2 * L.p + 1);
+        // the scaled M2L form where rs^(2p) and the scaled entries stay inside
+        // 1e-250 .. 1e250; |H_q(k r)| falls with r for a real k, so the
+        // shortest offset has the largest entries
+        const bool scale = L.rs > 0.0 && 2.0 * L.p * std::fabs(std::log10(L.rs)) < 250.0;
+        bool fine = true;
+        hv.resize(t.N2 + 2);
+        for (int i = 0; i < (zk.y == 0.0 && zk.x > 0.0 ? 1 : 7); i++) {
+            helm_hvec(t.N2, cscal(zk, std::sqrt((double)kM2LLengths[i]) * t.bs), L.rs, hv.data());
+            double f = 1.0;  // rs^-q
+            for (int q = 0; q <= t.N2; q++, f /= L.rs) {
+                const double a = hk::cabs_(hv[q]);
+                t.m2l_max = std::max(t.m2l_max, a);
+                if (!(a <= 1e250) || (scale && !(a * f <= 1e250))) fine = false;
+            }
+        }
+        t.sc_ok = scale && fine;
+        if (t.sc_ok) t.m2l_sc = place(ct_n, 49 * len);
     }
-    const std::vector<LevTab> &lt = tabs->lt;
-    const std::vector<double2> &ct = tabs->ct;
-    const std::vector<double> &rt = tabs->rt;
-    DevBuf<double2> d_ct(std::max<size_t>(ct.size(), 1), s);
-    DevBuf<double> d_rt(std::max<size_t>(rt.size(), 1), s);
-    if (!ct.empty())
-        FMM_CUDA(cudaMemcpyAsync(d_ct.get(), ct.data(), ct.size() * sizeof(double2),
-                                 cudaMemcpyHostToDevice, s));
-    if (!rt.empty())
-        FMM_CUDA(cudaMemcpyAsync(d_rt.get(), rt.data(), rt.size() * sizeof(double),
-                                 cudaMemcpyHostToDevice, s));
+    DevBuf<double2> d_ct(std::max<long long>(ct_n, 1), s);
+    DevBuf<double> d_rt(std::max<long long>(rt_n, 1), s);
+    for (int l = 2; l <= nl; l += kTabLevels) {
+        const int n = std::min(kTabLevels, nl + 1 - l);
+        HTabLevs tl;
+        for (int i = 0; i < n; i++) tl.l[i] = lt[l + i];
+        helm_tables_kernel<<<10 * n, 128, 0, s>>>(tl, zk, d_ct.get(), d_rt.get());
+        FMM_CHECK_LAUNCH();
+    }
     prof_mark("h_tables", s);
     const int nb = T.nboxes;
     const int ifc = P.ifcharge, ifd = P.ifdipole;
@@ -1847,22 +1734,11 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
     FMM_CHECK_LAUNCH();
     prof_mark("h_p2m_p2l", s);
     // ---- M2M, upward (parents at levels nl-1 .. 2) ----
-    // Folded shifts: boxes per block so that a level gives every SM a few
-    // blocks; levels whose staging does not fit into shared memory (orders
-    // above about 120) keep the general kernels
-    auto fold_range = [&](int n) {
-        return std::max(4, std::min(kShRange, (n + kNumSM * 8 - 1) / (kNumSM * 8)));
-    };
-    auto fold_smem = [&](int n1, int n2, int per) {
-        return ((size_t)2 * (n1 + n2) + 1 + (size_t)shift_units(2 * n2 + 1) * (2 * n1 + 1) * per) *
-               sizeof(double2);
-    };
-    constexpr size_t kFoldSmem = 200 * 1024;
     for (int l = nl - 1; l >= 2; l--) {
         if (!hl[l].flag) continue;
         const int lo = T.lstart[l], hi = T.lend[l];
         const size_t fsm = fold_smem(hl[l + 1].p, hl[l].p, 4);
-        if (lt[l].m2m_ok && fsm <= kFoldSmem) {
+        if (lt[l].m2m_ok) {
             const int range = fold_range(hi - lo);
             raise_smem_limit(helm_m2m_fold_kernel, fsm);
             helm_m2m_fold_kernel<<<(hi - lo + range - 1) / range, kShThreads, fsm, s>>>(
@@ -2039,7 +1915,7 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
     for (int l = 2; l <= nl - 1; l++) {
         if (!hl[l].flag) continue;
         const size_t fsm = fold_smem(hl[l].p, hl[l + 1].p, 1);
-        if (lt[l].l2l_ok && fsm <= kFoldSmem) {
+        if (lt[l].l2l_ok) {
             const int plo = T.lstart[l], phi = T.lend[l], range = fold_range(phi - plo);
             raise_smem_limit(helm_l2l_fold_kernel, fsm);
             helm_l2l_fold_kernel<<<(phi - plo + range - 1) / range, kShThreads, fsm, s>>>(
