@@ -810,6 +810,159 @@ __global__ void __launch_bounds__(128, 5) helm_m2l_tile_kernel(
     }
 }
 
+// The scaled form with the slot's operands in shared memory, for levels whose
+// tiles have a thread for every two outputs ((p + 1) nd <= 128): the sources of
+// the block's tiles ([tile][channel][j][box], so that a step reads one 64-byte
+// row, broadcast) and each tile's table row (even and odd entries apart, so
+// that neighbouring threads, whose entries are two apart, read neighbouring
+// words) come by asynchronous copies one slot ahead.  A step's 32 fused
+// operations then wait for shared memory instead of five dependent global
+// loads: 250 ns per step in a launch that does not fill the chip (2,001 points:
+// 62 -> 24 us for 0.02 GFLOP); M2L 0.55 -> 0.47 ms at 1e5 clustered points.
+constexpr int kHStageM = 128 * 2 * kHTile;   // sum over tiles and channels of (2p + 1) boxes <=
+constexpr int kHStageT = 4 * 128;            // sum over tiles of 4p + 2 <=
+constexpr size_t kHStageBytes = (size_t)2 * (kHStageM + kHStageT) * sizeof(double2);
+
+__device__ __forceinline__ void cp_async16(double2 *dst, const double2 *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src)
+                 : "memory");
+}
+
+__global__ void __launch_bounds__(128, 4) helm_m2l_stage_kernel(
+    const __grid_constant__ HJobs jobs, const int *__restrict__ boxes,
+    const int *__restrict__ slots, const int2 *__restrict__ dxy, int nd,
+    const HLevel *__restrict__ lv, const double2 *__restrict__ mp, double2 *__restrict__ loc,
+    double2 *__restrict__ part) {
+    constexpr int R = kHTile;
+    extern __shared__ __align__(16) double2 hst_sm[];
+    __shared__ int s_src[kHGroups][R][27];
+    __shared__ int s_trg[kHGroups][R];
+    __shared__ int s_q[kHGroups][R];
+    __shared__ int s_cp[kHGroups];
+    int ji = 0;
+    while (ji + 1 < jobs.n && (int)blockIdx.x >= jobs.j[ji + 1].blk0) ji++;
+    const HJob &lt = jobs.j[ji];
+    const HLevel L = lv[lt.l];
+    const double2 *__restrict__ T = lt.T;
+    const int p = L.p, w = 2 * p + 1, tw = 4 * p + 1, wn = (p + 1) * nd;
+    const int G = lt.G, ntiles = lt.tb[4] - lt.tb[0];
+    const int rel = blockIdx.x - lt.blk0, slice = rel / lt.nblk;
+    const int k0 = slice * 27 / lt.nslice, k1 = (slice + 1) * 27 / lt.nslice;
+    const int base = (rel - slice * lt.nblk) * G;
+    for (int e = threadIdx.x; e < G * R * 27; e += blockDim.x) {
+        const int g = e / (R * 27), r = (e / 27) % R, k = e % 27;
+        const int tile = base + g;
+        int v = -1, tb = -1, cp = 0;
+        if (tile < ntiles) {
+            const int t = lt.tb[0] + tile;
+            while (cp < 3 && t >= lt.tb[cp + 1]) cp++;
+            const int q = lt.start[cp] + (t - lt.tb[cp]) * R + r;
+            if (q < lt.start[cp] + lt.count[cp]) {
+                v = slots[(size_t)q * 27 + k];
+                tb = boxes[q];
+                if (k == 0) s_q[g][r] = q - lt.start[0];
+            }
+        }
+        s_src[g][r][k] = v;
+        if (k == 0) s_trg[g][r] = tb;
+        if (k == 0 && r == 0) s_cp[g] = cp;
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    // slot k's operands into buffer (k - k0) & 1
+    auto stage = [&](int k) {
+        double2 *sM = hst_sm + (size_t)((k - k0) & 1) * (kHStageM + kHStageT), *sT = sM + kHStageM;
+        for (int gr = wid; gr < G * R; gr += 4) {
+            const int g = gr / R, r = gr - g * R, sb = s_src[g][r][k];
+            const double2 *m = sb >= 0 ? coef0(mp, L, sb, nd) - (long long)p * nd : nullptr;
+            for (int e = lane; e < w * nd; e += 32) {
+                const int j = nd == 1 ? e : e / nd, c = e - j * nd;
+                double2 *d = sM + ((size_t)(g * nd + c) * w + j) * R + r;
+                if (m) cp_async16(d, m + e);
+                else *d = make_double2(0.0, 0.0);
+            }
+        }
+        for (int g = wid; g < G; g += 4) {
+            const int2 d = dxy[s_cp[g] * 27 + k];
+            const double2 *t = T + (size_t)((3 - d.y) * 7 + (3 - d.x)) * tw;
+            double2 *row = sT + (size_t)g * (tw + 1);
+            for (int e = lane; e < tw; e += 32)
+                cp_async16(row + (e >> 1) + (e & 1) * (2 * p + 1), t + e);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // this thread's outputs: orders i0 and i0 + 1 (the second absent for
+    // i0 = p) of channel c of tile g
+    const int u = threadIdx.x, g = u / wn, o = u - g * wn;
+    const bool act = g < G && s_trg[min(g, kHGroups - 1)][0] >= 0;
+    const int oo = o / nd, c = o - oo * nd, i0 = 2 * oo - p;
+    const bool two = i0 < p;
+    double2 acc0[R], acc1[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) acc0[r] = acc1[r] = make_double2(0.0, 0.0);
+    stage(k0);
+    for (int k = k0; k < k1; k++) {
+        if (k + 1 < k1) {
+            stage(k + 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        if (act) {
+            const double2 *sM = hst_sm + (size_t)((k - k0) & 1) * (kHStageM + kHStageT);
+            const double2 *m = sM + (size_t)(g * nd + c) * w * R;
+            // entries p + 2 oo' of T are even where p + ... - j is: step jj
+            // (j = jj - p) takes entry 2p + 2 oo - jj
+            const double2 *te = sM + kHStageM + (size_t)g * (tw + 1) + p + oo;
+            const double2 *to = te + 2 * p + 1;
+            double2 tb = two ? *to : make_double2(0.0, 0.0);
+            auto step = [&](double2 ta) {
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    const double2 v = m[r];
+                    acc0[r].x = fma(v.x, ta.x, acc0[r].x);
+                    acc0[r].x = fma(-v.y, ta.y, acc0[r].x);
+                    acc0[r].y = fma(v.x, ta.y, acc0[r].y);
+                    acc0[r].y = fma(v.y, ta.x, acc0[r].y);
+                    acc1[r].x = fma(v.x, tb.x, acc1[r].x);
+                    acc1[r].x = fma(-v.y, tb.y, acc1[r].x);
+                    acc1[r].y = fma(v.x, tb.y, acc1[r].y);
+                    acc1[r].y = fma(v.y, tb.x, acc1[r].y);
+                }
+                tb = ta;
+                m += R;
+            };
+            for (int jj = 0; jj < 2 * p; jj += 2) {
+                step(*te--);  // entry 2 (p + oo) - jj
+                step(*--to);  // the odd one below
+            }
+            step(*te);
+        }
+        __syncthreads();
+    }
+    if (!act) return;
+    const double *__restrict__ pw = lt.pw;
+    const double sc0 = pw[abs(i0)], sc1 = pw[min(abs(i0 + 1), p)];
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        if (s_trg[g][r] < 0) continue;
+        const double2 v0 = cscal(acc0[r], sc0), v1 = cscal(acc1[r], sc1);
+        if (lt.nslice > 1) {
+            double2 *op = part + lt.part0 + ((size_t)slice * lt.nq + s_q[g][r]) * w * nd +
+                          (size_t)(i0 + p) * nd + c;
+            op[0] = v0;
+            if (two) op[nd] = v1;
+        } else {
+            double2 *op = coef0(loc, L, s_trg[g][r], nd) + (long long)i0 * nd + c;
+            *op = cadd(*op, v0);
+            if (two) op[nd] = cadd(op[nd], v1);
+        }
+    }
+}
+
 // Sum of the slices' partial M2L sums of helm_m2l_tile_kernel, in slice
 // order, into the local expansions of the split levels' targets.
 __global__ void __launch_bounds__(256) helm_m2l_sum_kernel(
@@ -854,12 +1007,12 @@ __global__ void __launch_bounds__(256) helm_scale_mp_kernel(const __grid_constan
 
 // Slices of the jobs' levels: a block's chain is its slots' 2p + 1 steps each,
 // and the chip runs kNumSM * 5 blocks at once; a chain longer than an even
-// share of all the steps (or than 240 steps, about 10 us, when there is less
+// share of all the steps (or than 200 steps, about 10 us, when there is less
 // work than that) is cut.
 void slices_for(HJobs &J) {
     double steps = 0.0;
     for (int i = 0; i < J.n; i++) steps += (double)J.j[i].nblk * 27 * (2 * J.j[i].p + 1);
-    const double share = std::max(240.0, steps / (kNumSM * 5));
+    const double share = std::max(200.0, steps / (kNumSM * 5));
     for (int i = 0; i < J.n; i++) {
         const double chain = 27.0 * (2 * J.j[i].p + 1);
         J.j[i].nslice = std::max(1, std::min(27, (int)std::ceil(chain / share)));
@@ -1778,7 +1931,8 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
     if (tc) FMM_CUDA(cudaMemsetAsync(tc_err.get(), 0, sizeof(int), s));
     bool tc_used = false;
     std::vector<char> tc_lev(nl + 1, 0);
-    std::vector<HJob> jobs[2];  // levels of the tile form: unscaled, scaled
+    // levels of the tile form: unscaled, scaled, scaled with staged operands
+    std::vector<HJob> jobs[3];
     const bool hf_on = !(getenv("FMM2D_B200_HELM_HF") && !strcmp(getenv("FMM2D_B200_HELM_HF"), "0"));
     for (int l = 2; l <= nl; l++) {
         if (!hl[l].flag) continue;
@@ -1828,7 +1982,7 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
             const bool sc = lt[l].sc_ok;
             ht.T = d_ct.get() + (sc ? lt[l].m2l_sc : lt[l].m2l);
             ht.pw = d_rt.get() + lt[l].m2l_pw;
-            jobs[sc].push_back(ht);
+            jobs[!sc ? 0 : wn > 128 ? 1 : 2].push_back(ht);
             continue;
         }
         const int lo = T.lstart[l], hi = T.lend[l];
@@ -1839,7 +1993,7 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
             d_rt.get() + lt[l].m2l_pw, mp.get(), loc.get());
         FMM_CHECK_LAUNCH();
     }
-    for (int sc = 0; sc < 2; sc++)
+    for (int sc = 0; sc < 3; sc++)
         for (size_t first = 0; first < jobs[sc].size(); first += kHJobs) {
             HJobs J;
             J.n = (int)std::min<size_t>(kHJobs, jobs[sc].size() - first);
@@ -1865,9 +2019,16 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
                 helm_scale_mp_kernel<<<grid_for(mp_n, 256), 256, 0, s>>>(J, mp_n, nd, mp.get(),
                                                                          mps.get());
                 FMM_CHECK_LAUNCH();
-                helm_m2l_tile_kernel<true><<<(unsigned)blocks, 128, 0, s>>>(
-                    J, spl.boxes, spl.slots, spl.dxy, nd, d_lv.get(), zero.get(), mps.get(),
-                    loc.get(), part.get());
+                if (sc == 2) {
+                    raise_smem_limit((const void *)helm_m2l_stage_kernel, kHStageBytes);
+                    helm_m2l_stage_kernel<<<(unsigned)blocks, 128, kHStageBytes, s>>>(
+                        J, spl.boxes, spl.slots, spl.dxy, nd, d_lv.get(), mps.get(), loc.get(),
+                        part.get());
+                } else {
+                    helm_m2l_tile_kernel<true><<<(unsigned)blocks, 128, 0, s>>>(
+                        J, spl.boxes, spl.slots, spl.dxy, nd, d_lv.get(), zero.get(), mps.get(),
+                        loc.get(), part.get());
+                }
             } else {
                 helm_m2l_tile_kernel<false><<<(unsigned)blocks, 128, 0, s>>>(
                     J, spl.boxes, spl.slots, spl.dxy, nd, d_lv.get(), zero.get(), mp.get(),
