@@ -1514,10 +1514,12 @@ constexpr size_t helm_p2p_flat_warp_bytes() {
 
 // KIND 0: any wavenumber; 1, 2, 3: a positive real one with charges, dipoles,
 // both (pair_add_real).
-// Both point sets in one launch when they want the same outputs (nsets 2).
+// Both point sets in one launch when they want the same outputs (nsets 2).  A
+// leaf's targets are dealt to `parts` warps (a power of two) while the boxes
+// leave the chip idle: each then has fewer targets to the same sources.
 template <int PGH, int KIND>
 __global__ void __launch_bounds__(kHfWarps * 32) helm_p2p_flat_kernel(
-    int nb, int nsets, HPointSet set0, HPointSet set1, const int *__restrict__ nchild,
+    int nb, int nsets, int parts, HPointSet set0, HPointSet set1, const int *__restrict__ nchild,
     const int *__restrict__ nlist1, const int *__restrict__ list1, const int2 *__restrict__ sse,
     const double2 *__restrict__ src, const double2 *__restrict__ charge,
     const double2 *__restrict__ dipstr, const double2 *__restrict__ dipvec, int ifc, int ifd,
@@ -1533,11 +1535,18 @@ __global__ void __launch_bounds__(kHfWarps * 32) helm_p2p_flat_kernel(
     const double k2 = zk.x * zk.x, thresh2 = thresh * thresh;
     const double2 zero = make_double2(0.0, 0.0);
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nb * nsets; w += nwarps) {
-        const bool second = w >= nb;
-        const int b = second ? w - nb : w;
+    for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < nb * nsets * parts;
+         w += nwarps) {
+        const int bs = w / parts, part_i = w - bs * parts;
+        const bool second = bs >= nb;
+        const int b = second ? bs - nb : bs;
         if (nchild[b] != 0) continue;
-        const int2 tr = (second ? set1 : set0).se[b];
+        int2 tr = (second ? set1 : set0).se[b];
+        if (parts > 1) {
+            const int m = tr.y - tr.x;
+            tr = make_int2(tr.x + (int)((long long)m * part_i / parts),
+                           tr.x + (int)((long long)m * (part_i + 1) / parts));
+        }
         const int ntot = tr.y - tr.x;
         const int n1 = nlist1[b];
         if (ntot <= 0 || n1 == 0) continue;
@@ -2142,14 +2151,18 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
         // one warp per leaf (nd = 1; FMM2D_B200_HELM_P2P=point keeps a thread per point)
         const char *pm = getenv("FMM2D_B200_HELM_P2P");
         if (nd == 1 && !(pm && !strcmp(pm, "point"))) {
+            // warps per leaf: as many (up to 8) as the chip holds beside one
+            // another (16 warps per SM; 2,001 points: 0.077 -> 0.033 ms)
+            int parts = 1;
+            while (parts < 8 && (int64_t)nb * together * parts * 2 <= kNumSM * 16) parts *= 2;
 #define HP2PF(PG, KD)                                                                        \
     do {                                                                                     \
         constexpr size_t sm = kHfWarps * helm_p2p_flat_warp_bytes<PG>();                     \
         auto kern = helm_p2p_flat_kernel<PG, KD>;                                            \
         raise_smem_limit((const void *)kern, sm);                                            \
-        const int gw = std::max(1, std::min((nb * together + kHfWarps - 1) / kHfWarps,       \
+        const int gw = std::max(1, std::min((nb * together * parts + kHfWarps - 1) / kHfWarps, \
                                             kNumSM * 16));                                   \
-        kern<<<gw, kHfWarps * 32, sm, s>>>(nb, together, X, sets[first + together - 1],      \
+        kern<<<gw, kHfWarps * 32, sm, s>>>(nb, together, parts, X, sets[first + together - 1], \
                                           T.nchild.get(), T.nlist1.get(), T.list1.get(),     \
                                           T.srcse.get(), P.src, P.charge, P.dipstr, P.dipvec, \
                                           ifc, ifd, zk, thresh);                             \
