@@ -349,6 +349,14 @@ void laplace_evaluate(const FmmCall &c, const LapGeometry &G, bool on_dev, cudaS
     P.split = G.split;
     P.real_charge = lap;
     P.m2l_cache = m2l;
+    // the M2L's error flag comes with the call's last synchronisation instead
+    // of one of its own (about 15 us of a call of 300 to 10^5 points)
+    DevBuf<int> m2l_err;
+    if (sync && G.mixed && !m2l) {
+        m2l_err.alloc(1, s);
+        FMM_CUDA(cudaMemsetAsync(m2l_err.get(), 0, sizeof(int), s));
+        P.m2l_err = m2l_err.get();
+    }
     if (mixed) {
         P.charge32 = chg32.get();
         P.dipstr32 = dip32.get();
@@ -487,7 +495,12 @@ void laplace_evaluate(const FmmCall &c, const LapGeometry &G, bool on_dev, cudaS
     }
     // (the outputs, copied to host arrays where the caller's are, are
     // complete when the call returns)
-    if (sync) FMM_CUDA(cudaStreamSynchronize(s));
+    if (m2l_err.get()) {
+        if (read_scalar(m2l_err.get(), s) != 0)
+            throw FmmError(4, "tensor-core M2L: a wait for an MMA or operand barrier timed out");
+    } else if (sync) {
+        FMM_CUDA(cudaStreamSynchronize(s));
+    }
     prof_mark("scatter_d2h", s);
 }
 

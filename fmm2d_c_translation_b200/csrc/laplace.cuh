@@ -81,6 +81,9 @@ struct CauchyProblem {
     const float4 *trg_hl = nullptr;
     double *timeinfo = nullptr;       // 8 phase times (s), optional
     M2LCache *m2l_cache = nullptr;    // planning kept across evaluations (plans)
+    // device flag, zero on entry, that takes the M2L's bounded-wait error for
+    // the caller to read with the results (null: read at the end of the M2L)
+    int *m2l_err = nullptr;
     // boxes visited by the Pascal M2M (parents with sources) and L2L (boxes
     // with evaluation points): level l's at ids + lstart[l], cnt[l] of them;
     // by the P2M (leaves with sources) and the P2L (boxes with

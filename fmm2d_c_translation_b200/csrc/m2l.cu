@@ -1464,9 +1464,9 @@ bool m2l_fp32(const Tree &T, const CauchyProblem &P, const double2 *mp, double2 
     M2LCache *cache = P.m2l_cache;
     const bool deferred = cache && cache->deferred;
     DevBuf<int> err_own;
-    if (!deferred) err_own.alloc(1, s);
-    int *errp = deferred ? cache->err : err_own.get();
-    FMM_CUDA(cudaMemsetAsync(errp, 0, sizeof(int), s));
+    if (!deferred && !P.m2l_err) err_own.alloc(1, s);
+    int *errp = deferred ? cache->err : P.m2l_err ? P.m2l_err : err_own.get();
+    if (errp != P.m2l_err) FMM_CUDA(cudaMemsetAsync(errp, 0, sizeof(int), s));
     const uint64_t done =
         (simt || tile_only) ? 0 : m2l_window_fp32(T, P, mp32p, loc, errp, s);
     const int wtile = simt ? kFp32Tile : kTcRows / CH;
@@ -1567,7 +1567,7 @@ bool m2l_fp32(const Tree &T, const CauchyProblem &P, const double2 *mp, double2 
         // remaining single channels, one channel per row
         for (; c0 < P.ndc; c0++) one(std::integral_constant<int, 1>{}, kTcRows, c0);
     }
-    if (!deferred && read_scalar(errp, s) != 0)
+    if (errp == err_own.get() && read_scalar(errp, s) != 0)
         throw FmmError(4, "tensor-core M2L: a wait for an MMA or operand barrier timed out");
     return true;
 }
