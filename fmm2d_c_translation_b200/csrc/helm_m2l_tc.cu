@@ -29,13 +29,19 @@
 // Pipeline (one block per SM, persistent over the level's tiles): the K
 // dimension of each slot is cut into chunks of 16, and every (slot, chunk)
 // step stages A (128 x 16, hi and lo: gathered with cp.async from
-// operand-ready rows built once per level) and Bop (N x 16, hi and lo: a
-// contiguous block of the per-level images, also cp.async) into one of
-// kHtStages shared-memory stages.  Warps 0-3 (one thread per A row) fill
-// the stages, keeping kHtLag groups of copies in flight; warp 8 issues
+// operand-ready rows built once per level) and Bop (N x 16, hi and lo: one bulk
+// copy of a contiguous block of the per-level images) into one of kHtStages
+// shared-memory stages.  Warps 0-3 fill the stages, keeping kHtLag groups of
+// copies in flight; four lanes share an A row, whose chunk (hi and lo) is one
+// 128-byte line, so that a copy instruction touches 8 lines instead of 32.
+// Bound by the producers (issuing the copies, the proxy fence and the hand-over
+// are about half of the 1,300 cycles of a step) and by what every SM reads from
+// L2, 26 KB per step; 2.6 -> 2.3 ms for the levels of 2e6 points at order
+// 19.  Warp 12 issues
 // 3 x 2 MMAs per step and commits the stage back.  Each slot accumulates
-// in a fresh tensor-memory tile (two alternate), and warps 4-7 add every
-// slot's tile to FP64 sums in shared memory: the FP32 accumulation then
+// in a fresh tensor-memory tile (two alternate), and warps 4-11 (two per lane
+// quarter, half of the columns each) add every
+// slot's tile to FP64 sums in registers: the FP32 accumulation then
 // spans one slot's K chunks (a few tens of MMAs) instead of all 27 slots,
 // whose hundreds of FP32 roundings measured 4e-6 relative in the
 // potential.  (A caller whose products are small beside the result -- the
@@ -58,10 +64,11 @@ namespace fmm2d {
 namespace {
 
 constexpr int kHtRows = 128;
-constexpr int kHtStages = 4;
-constexpr int kHtLag = 2;
-constexpr int kHtEpi0 = 4;             // warps 4-7 read the accumulators
-constexpr int kHtThreads = 9 * 32;     // warp 8 issues the MMAs
+constexpr int kHtStages = 7;
+constexpr int kHtLag = 3;
+constexpr int kHtEpi0 = 4;             // warps 4-11 read the accumulators
+constexpr int kHtEpiWarps = 8;
+constexpr int kHtThreads = 13 * 32;    // warp 12 issues the MMAs
 constexpr int kHtTmemCols = 256;       // two accumulators of up to 128 columns
 constexpr uint64_t kHtWaitNs = 2000000000ull;
 constexpr int kHtSlots = 27;
@@ -75,7 +82,7 @@ struct HtArgs {
     const int *slots;  // [plan row][27] source box, -1 when none
     int lstart;        // first box of the level
     int nd, tpt, W;    // channels, target boxes per tile, 2p + 1
-    const float *arow;  // [level box][nd][hi KP | lo KP]
+    const float *arow;  // [level box][nd][K chunk][hi 16 | lo 16]
     const float *bimg;  // [cp][slot][chunk][hi NP x 16 | lo NP x 16], operand layout
     double2 *locl;      // the level's local expansions, [level box][2p + 1][nd]
     double oscale;      // 1 / (scale of Bop)
@@ -116,12 +123,10 @@ __global__ void __launch_bounds__(kHtThreads, 1) slot_gemm_tc_kernel(HtArgs A) {
     constexpr uint32_t IDESC = tc_idesc_tf32(kHtRows, NP);
     static_assert(KP % 16 == 0 && NP % 16 == 0 && NP <= 128, "operand shape");
     extern __shared__ __align__(1024) unsigned char ht_smem[];
-    // FP64 sums of the slots' partial products, column-major [NP][128] (the
-    // epilogue thread of row r owns column entries c * 128 + r)
-    double *sSum = reinterpret_cast<double *>(ht_smem + (size_t)kHtStages * STAGE);
     // barriers: [0, S) stage full, [S, 2S) stage free, 2S + a accumulator a
-    // full, 2S + 2 + a accumulator a free, 2S + 4 final
-    __shared__ __align__(8) uint64_t s_bar[2 * kHtStages + 5];
+    // full, 2S + 2 + a accumulator a free, 2S + 4 final, 2S + 5 + s the
+    // stage's matrix block landed
+    __shared__ __align__(8) uint64_t s_bar[3 * kHtStages + 5];
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
     volatile int *abort_flag = &s_abort;
@@ -132,10 +137,11 @@ __global__ void __launch_bounds__(kHtThreads, 1) slot_gemm_tc_kernel(HtArgs A) {
         for (int i = 0; i < kHtStages; i++) {
             mbar_init(HBAR(i), kHtRows);
             mbar_init(HBAR(kHtStages + i), 1);
+            mbar_init(HBAR(2 * kHtStages + 5 + i), 1);  // (with the bulk copy's bytes)
         }
         for (int a = 0; a < 2; a++) {
             mbar_init(HBAR(2 * kHtStages + a), 1);
-            mbar_init(HBAR(2 * kHtStages + 2 + a), kHtRows);
+            mbar_init(HBAR(2 * kHtStages + 2 + a), kHtEpiWarps * 32);
         }
         mbar_init(HBAR(2 * kHtStages + 4), 1);
         s_abort = 0;
@@ -165,47 +171,67 @@ __global__ void __launch_bounds__(kHtThreads, 1) slot_gemm_tc_kernel(HtArgs A) {
 
     if (warp < kHtEpi0) {
         // ------------------------------------------------------- producers
-        const int r = tid;  // A row
-        const int bx = r / A.nd, ch = r - bx * A.nd;
-        const uint32_t aoff = (uint32_t)(((r >> 3) * 128) + ((r & 7) * 16));
+        // this thread's quarter of the 16 columns of rows 32 warp + 8 i + lane / 4
+        const int qt = lane & 3, r0 = warp * 32 + (lane >> 2);
+        const uint32_t aoff = (uint32_t)qt * LBO_A + (uint32_t)(warp * 4 * 128 + (lane >> 2) * 16);
         long long step = 0;
+        int st_i = 0, full_i = kHtStages - kHtLag;  // stages of step, step - lag
+        uint32_t ph = 1;  // parity of the stage's previous release
         bool ok = true;
         for (int tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x) {
             int cp, q0;
             tile_seg(tile, cp, q0);
-            const int q = q0 + bx;
-            const bool valid = bx < A.tpt && q < A.start[cp] + A.count[cp];
-            const int *qs = A.slots + (size_t)(valid ? q : 0) * kHtSlots;
+            int q[4], ch[4], sb[4], nx[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int r = r0 + 8 * i, bx = r / A.nd;
+                ch[i] = r - bx * A.nd;
+                q[i] = bx < A.tpt && q0 + bx < A.start[cp] + A.count[cp] ? q0 + bx : -1;
+                nx[i] = q[i] >= 0 ? __ldg(A.slots + (size_t)q[i] * kHtSlots + k0) : -1;
+            }
             for (int k = k0; ok && k < k1; k++) {
-                const int sb = valid ? __ldg(qs + k) : -1;
-                const float *src = A.arow + (sb >= 0 ? ((size_t)(sb - A.lstart) * A.nd + ch) * 2 * KP : 0);
-                const uint32_t abytes = sb >= 0 ? 16u : 0u;  // 0: zero fill
+                const float *src[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    sb[i] = nx[i];
+                    src[i] = A.arow + 4 * qt +
+                             (sb[i] >= 0 ? ((size_t)(sb[i] - A.lstart) * A.nd + ch[i]) * 2 * KP : 0);
+                    // (the next slot's sources)
+                    nx[i] = k + 1 < k1 && q[i] >= 0
+                                ? __ldg(A.slots + (size_t)q[i] * kHtSlots + k + 1)
+                                : -1;
+                }
                 const float *bsrc = A.bimg + ((size_t)(cp * kHtSlots + k) * KC) * (2 * NP * 16);
                 for (int kc = 0; kc < KC; kc++, step++) {
-                    const int s = (int)(step % kHtStages);
-                    const long long u = step / kHtStages;
-                    if (u >= 1 &&
-                        !mbar_wait_bounded(HBAR(kHtStages + s), (uint32_t)((u - 1) & 1), abort_flag,
-                                           A.wait_ns)) {
+                    if (step >= kHtStages &&
+                        !mbar_wait_bounded(HBAR(kHtStages + st_i), ph, abort_flag, A.wait_ns)) {
                         ok = false;
                         break;
                     }
-                    const uint32_t st = sbase + (uint32_t)s * STAGE;
-#pragma unroll
-                    for (int cc = 0; cc < 4; cc++) {
-                        const int kk = 16 * kc + 4 * cc;
-                        cp_async16(st + (uint32_t)cc * LBO_A + aoff, src + kk, abytes);
-                        cp_async16(st + A_BYTES + (uint32_t)cc * LBO_A + aoff, src + KP + kk, abytes);
+                    const uint32_t st = sbase + (uint32_t)st_i * STAGE;
+                    if (tid == 0) {
+                        const uint32_t bar = HBAR(2 * kHtStages + 5 + st_i);
+                        mbar_arrive_expect_tx(bar, 2 * B_BYTES);
+                        bulk_g2s(st + 2 * A_BYTES, bsrc + (size_t)kc * (2 * NP * 16), 2 * B_BYTES,
+                                 bar);
                     }
-                    const float *bc = bsrc + (size_t)kc * (2 * NP * 16);
 #pragma unroll
-                    for (int e = r; e < NP * 8; e += kHtRows)
-                        cp_async16(st + 2 * A_BYTES + 16u * (uint32_t)e, bc + 4 * e, 16u);
+                    for (int i = 0; i < 4; i++) {
+                        const uint32_t bytes = sb[i] >= 0 ? 16u : 0u;  // 0: zero fill
+                        const uint32_t d = st + aoff + (uint32_t)i * 128u;
+                        cp_async16(d, src[i] + 32 * kc, bytes);
+                        cp_async16(d + A_BYTES, src[i] + 32 * kc + 16, bytes);
+                    }
                     cp_async_commit();
                     if (step >= kHtLag) {
                         cp_async_wait<kHtLag>();
                         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                        mbar_arrive(HBAR((int)((step - kHtLag) % kHtStages)));
+                        mbar_arrive(HBAR(full_i));
+                    }
+                    full_i = full_i + 1 == kHtStages ? 0 : full_i + 1;
+                    if (++st_i == kHtStages) {
+                        st_i = 0;
+                        ph ^= 1u;
                     }
                 }
             }
@@ -218,20 +244,35 @@ __global__ void __launch_bounds__(kHtThreads, 1) slot_gemm_tc_kernel(HtArgs A) {
         } else {
             *abort_flag = 1;
         }
-    } else if (warp < kHtEpi0 + 4) {
+        if (tid == 0) {
+            // the last bulk copies have landed before the block exits (the
+            // issuer has waited for them unless the block stopped early)
+            int never = 0;
+            for (long long t = step - kHtStages; t < step; t++)
+                if (t >= 0)
+                    mbar_wait_bounded(HBAR(2 * kHtStages + 5 + (int)(t % kHtStages)),
+                                      (uint32_t)((t / kHtStages) & 1), &never, kHtWaitNs);
+        }
+    } else if (warp < kHtEpi0 + kHtEpiWarps) {
         // -------------------------------------------------------- epilogue
         // Each slot's products accumulate in a fresh tensor-memory tile
-        // (two alternate between slots); this thread adds its row of every
+        // (two alternate between slots); this thread adds half a row of every
         // slot's tile in FP64, so the FP32 accumulation spans only the
         // slot's own K chunks.
-        const int e = warp - kHtEpi0;  // tensor-memory lanes 32 e .. 32 e + 31
+        constexpr int NH = NP / 2;
+        static_assert(NH % 8 == 0, "columns per warp");
+        const int e = warp & 3;  // tensor-memory lanes 32 e .. 32 e + 31
+        const int half = (warp - kHtEpi0) >> 2;
         const int r = (e << 5) + lane;
         const int bx = r / A.nd, ch = r - bx * A.nd;
+        double sum[NH];
+        double *sOut = reinterpret_cast<double *>(ht_smem + (size_t)kHtStages * STAGE) +
+                       (warp - kHtEpi0) * 32 * 9;
         long long g = 0;  // slots finished by this block
         bool ok = true;
         for (int tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x) {
-#pragma unroll 4
-            for (int c = 0; c < NP; c++) sSum[c * kHtRows + r] = 0.0;
+#pragma unroll
+            for (int c = 0; c < NH; c++) sum[c] = 0.0;
             for (int k = k0; k < k1; k++) {
                 if ((k - k0) % A.group != A.group - 1 && k != k1 - 1) continue;  // (not a group's end)
                 const int a = (int)(g & 1);
@@ -242,43 +283,58 @@ __global__ void __launch_bounds__(kHtThreads, 1) slot_gemm_tc_kernel(HtArgs A) {
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t taddr = tmem + ((uint32_t)(e << 5) << 16) + (uint32_t)(a * 128);
-                float d[NP];
+                const uint32_t taddr =
+                    tmem + ((uint32_t)(e << 5) << 16) + (uint32_t)(a * 128 + half * NH);
 #pragma unroll
-                for (int c8 = 0; c8 < NP / 8; c8++) {
+                for (int c8 = 0; c8 < NH / 8; c8++) {
                     float v[8];
                     tc_ld8(taddr + (uint32_t)(8 * c8), v);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                    for (int i = 0; i < 8; i++) d[8 * c8 + i] = v[i];
+                    for (int i = 0; i < 8; i++) sum[8 * c8 + i] += (double)v[i];
                 }
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                 mbar_arrive(HBAR(2 * kHtStages + 2 + a));
-#pragma unroll
-                for (int c = 0; c < NP; c++) sSum[c * kHtRows + r] += (double)d[c];
                 g++;
             }
             if (!ok) break;
             int cp, q0;
             tile_seg(tile, cp, q0);
             const int q = q0 + bx;
-            if (bx < A.tpt && q < A.start[cp] + A.count[cp]) {
-                double *o;
-                bool add = true;
-                if (gridDim.y > 1) {  // this slice's partial sums
-                    o = reinterpret_cast<double *>(
-                        A.part + ((size_t)blockIdx.y * A.nq + (q - A.q_lo)) * A.W * A.nd + ch);
-                    add = false;
-                } else {
-                    const int b = A.boxes[q];
-                    o = reinterpret_cast<double *>(A.locl + (size_t)(b - A.lstart) * A.W * A.nd + ch);
-                }
-                const size_t st = 2 * (size_t)A.nd;
+            const bool add = gridDim.y == 1;  // else this slice's partial sums
+            double *o = nullptr;              // this row's coefficient -p
+            if (bx < A.tpt && q < A.start[cp] + A.count[cp])
+                o = add ? reinterpret_cast<double *>(
+                              A.locl + (size_t)(A.boxes[q] - A.lstart) * A.W * A.nd + ch)
+                        : reinterpret_cast<double *>(
+                              A.part +
+                              ((size_t)blockIdx.y * A.nq + (q - A.q_lo)) * A.W * A.nd + ch);
+            // Eight columns at a time through shared memory, so that eight
+            // lanes write one row's neighbouring coefficients (a lane per row
+            // touched 32 lines per access: 0.3 of 2.9 ms).
+            double *orow[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                orow[i] = reinterpret_cast<double *>(
+                    __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(o), 4 * i + (lane >> 3)));
+            const size_t st = 2 * (size_t)A.nd;
+#pragma unroll
+            for (int c8 = 0; c8 < NH; c8 += 8) {
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < 8; i++) sOut[lane * 9 + i] = sum[c8 + i];
+                __syncwarp();
                 // column c: Re L_(c - p) for c < W, Im L_(c - W - p) for W <= c < 2W
-                for (int c = 0; c < 2 * A.W; c++) {
-                    const double v = A.oscale * sSum[c * kHtRows + r];
-                    double &dst = c < A.W ? o[(size_t)c * st] : o[(size_t)(c - A.W) * st + 1];
-                    dst = add ? dst + v : v;
+                const int c = half * NH + c8 + (lane & 7);
+                const size_t at = c < A.W ? (size_t)c * st : (size_t)(c - A.W) * st + 1;
+                double old[8];
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+                    old[i] = add && orow[i] && c < 2 * A.W ? orow[i][at] : 0.0;
+#pragma unroll
+                for (int i = 0; i < 8; i++) {
+                    const double v = A.oscale * sOut[(4 * i + (lane >> 3)) * 9 + (lane & 7)];
+                    if (orow[i] && c < 2 * A.W) orow[i][at] = add ? old[i] + v : v;
                 }
             }
         }
@@ -313,8 +369,12 @@ __global__ void __launch_bounds__(kHtThreads, 1) slot_gemm_tc_kernel(HtArgs A) {
                 for (int kc = 0; kc < KC; kc++, step++) {
                     const int s = (int)(step % kHtStages);
                     const long long u = step / kHtStages;
-                    if (!__all_sync(0xffffffffu, mbar_wait_bounded(HBAR(s), (uint32_t)(u & 1),
-                                                                   abort_flag, A.wait_ns))) {
+                    if (!__all_sync(0xffffffffu,
+                                    mbar_wait_bounded(HBAR(s), (uint32_t)(u & 1), abort_flag,
+                                                      A.wait_ns) &&
+                                        mbar_wait_bounded(HBAR(2 * kHtStages + 5 + s),
+                                                          (uint32_t)(u & 1), abort_flag,
+                                                          A.wait_ns))) {
                         ok = false;
                         break;
                     }
@@ -370,7 +430,7 @@ __global__ void __launch_bounds__(kHtThreads, 1) slot_gemm_tc_kernel(HtArgs A) {
 template <int KP, int NP>
 constexpr size_t ht_smem_bytes() {
     return (size_t)kHtStages * (2 * kHtRows * 16 * 4 + 2 * NP * 16 * 4) +
-           (size_t)NP * kHtRows * sizeof(double);
+           (size_t)kHtEpiWarps * 32 * 9 * sizeof(double);
 }
 
 // x rounded to TF32 (nearest, ties away from zero), as cvt.rna does.
@@ -379,7 +439,7 @@ __device__ __forceinline__ void ht_split(float v, float &hi, float &lo) {
     lo = tc_tf32(v - hi);
 }
 
-// Operand-ready A rows of the level's boxes: [box][ch][hi KP | lo KP] of
+// Operand-ready A rows of the level's boxes: [box][ch][K chunk][hi 16 | lo 16] of
 // [Re M_-p..p | Im M_-p..p | 0].
 __global__ void __launch_bounds__(256) slot_rows_kernel(long long nrow, int nd, int W, int KP,
                                                           const double2 *__restrict__ mpl,
@@ -398,8 +458,9 @@ __global__ void __launch_bounds__(256) slot_rows_kernel(long long nrow, int nd, 
         }
         float hi, lo;
         ht_split(v, hi, lo);
-        arow[row * 2 * KP + k] = hi;
-        arow[row * 2 * KP + KP + k] = lo;
+        float *o = arow + row * 2 * KP + (k >> 4) * 32 + (k & 15);
+        o[0] = hi;
+        o[16] = lo;
     }
 }
 

@@ -188,7 +188,7 @@ struct SlotGemmLevel {
     int level = 0;                // level of the target boxes (>= 2)
     int lstart = 0;               // box of row 0 of arow and out
     int nd = 1, W = 0, KP = 0;    // channels, coefficients, padded K = N
-    const float *arow = nullptr;  // [box - lstart][nd][hi KP | lo KP]
+    const float *arow = nullptr;  // [box - lstart][nd][KP / 16][hi 16 | lo 16]
     const float *bimg = nullptr;  // [cp][27][KP / 16][hi KP x 16 | lo KP x 16]
     double2 *out = nullptr;       // [box - lstart][W][nd]
     double oscale = 1.0;
