@@ -18,8 +18,8 @@
 // separate calls, two of them with their own logarithm, each branching on
 // the argument) and the continued fraction above: 4.72 ms of near field at
 // 2e6 points, zk 200 (1.4e8 pairs), about 640 FP64 instructions per pair;
-// with the table 2.12 ms, bound by the FP64 pipe and its latency (16 warps
-// per SM at 122-128 registers).
+// with the table 2.12 ms and, with its first row in constant memory, 1.76 ms
+// (FP64 pipe and latency: 16 warps per SM at 122-128 registers).
 #pragma once
 
 #include <cmath>
@@ -27,6 +27,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "pairmath.cuh"
 
 namespace fmm2d {
 namespace hb {
@@ -41,21 +42,48 @@ constexpr int kRow = 2 * (kDeg + 1) + 1;
 
 __device__ double2 g_tab[kIntervals * kRow];
 
+// The first interval's row once more, as constant operands of the FMAs.
+__constant__ double2 c_tab0[kRow];
+
 // h0 = H0(x), g = H1(x) / x for x = sqrt(s), 0 < s < 256; si = 1 / s.
+//
+// NEAR: lanes that are all below s = 2 -- the near field of leaves smaller than
+// about a tenth of a wavelength, which is most near fields -- take the row from
+// constant memory, since the 18 table loads of a pair kept the load unit busier
+// (73 %) than the FP64 pipe (39 %), and ln s comes from pairmath.cuh: 2.13 ->
+// 1.76 ms at 2e6 points, zk 200; 0.22 -> 0.19 ms at 1e5 clustered points.  (The
+// expansions' evaluation, bound by its recurrences, took 0.47 -> 0.51 ms with
+// the same.)
+template <bool NEAR>
 __device__ __forceinline__ void hankel01_sq(double s, double si, double2 &h0, double2 &g) {
     const int iv = (int)(s * 0.5);
     const double t = s - (double)(2 * iv + 1);
-    const double2 *__restrict__ r = g_tab + iv * kRow;
-    double2 ab = __ldg(r), cd = __ldg(r + 1);
+    double2 ab, cd;
+    if (NEAR && __all_sync(__activemask(), iv == 0)) {
+        ab = c_tab0[0];
+        cd = c_tab0[1];
 #pragma unroll
-    for (int m = 1; m <= kDeg; m++) {
-        const double2 u = __ldg(r + 2 * m), v = __ldg(r + 2 * m + 1);
-        ab.x = fma(ab.x, t, u.x);
-        ab.y = fma(ab.y, t, u.y);
-        cd.x = fma(cd.x, t, v.x);
-        cd.y = fma(cd.y, t, v.y);
+        for (int m = 1; m <= kDeg; m++) {
+            ab.x = fma(ab.x, t, c_tab0[2 * m].x);
+            ab.y = fma(ab.y, t, c_tab0[2 * m].y);
+            cd.x = fma(cd.x, t, c_tab0[2 * m + 1].x);
+            cd.y = fma(cd.y, t, c_tab0[2 * m + 1].y);
+        }
+    } else {
+        const double2 *__restrict__ r = g_tab + iv * kRow;
+        ab = __ldg(r);
+        cd = __ldg(r + 1);
+#pragma unroll
+        for (int m = 1; m <= kDeg; m++) {
+            const double2 u = __ldg(r + 2 * m), v = __ldg(r + 2 * m + 1);
+            ab.x = fma(ab.x, t, u.x);
+            ab.y = fma(ab.y, t, u.y);
+            cd.x = fma(cd.x, t, v.x);
+            cd.y = fma(cd.y, t, v.y);
+        }
     }
-    const double lg = log(s) * 0.31830988618379067154;
+    const double lg = NEAR ? half_ln_any(s) * 0.63661977236758134308
+                           : log(s) * 0.31830988618379067154;
     h0 = make_double2(ab.x, fma(lg, ab.x, cd.x));
     g = make_double2(ab.y, fma(si, -0.63661977236758134308, fma(lg, ab.y, cd.y)));
 }
@@ -139,6 +167,7 @@ inline void ensure_table() {
     if (done[dev]) return;
     if (tab.empty()) tab = make_table();
     FMM_CUDA(cudaMemcpyToSymbol(g_tab, tab.data(), tab.size() * sizeof(double2)));
+    FMM_CUDA(cudaMemcpyToSymbol(c_tab0, tab.data(), sizeof(c_tab0)));
     done[dev] = 1;
 }
 

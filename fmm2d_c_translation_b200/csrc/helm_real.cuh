@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(256) helm_p2l_real_kernel(
                 em = make_double2(dx * rinv, -dy * rinv);
                 const double x = k * rr, s = x * x;
                 double2 g;
-                if (s < hb::kSMax) hb::hankel01_sq(s, 1.0 / s, h0, g);
+                if (s < hb::kSMax) hb::hankel01_sq<false>(s, 1.0 / s, h0, g);
                 else hankel01_far(s, h0, g);
                 h1 = cscal(g, x * rs);
                 w = 2.0 * rs * rinv / k;
@@ -523,7 +523,7 @@ __global__ void __launch_bounds__(128) helm_far_real_kernel(
                     CoefR<PGH, true> C(coef0(mp, L3, jb, nd) + c, L3.p, nd, 0.5 * k / rs,
                                        0.5 * k * rs, 0);
                     double2 h0, g;
-                    if (s < hb::kSMax) hb::hankel01_sq(s, 1.0 / s, h0, g);
+                    if (s < hb::kSMax) hb::hankel01_sq<false>(s, 1.0 / s, h0, g);
                     else hankel01_far(s, h0, g);
                     const double zr = 2.0 * rs * rinv / k;
                     acc_real(A, C, 0, w, h0);

@@ -1377,12 +1377,15 @@ template <int PGH, bool IFC, bool IFD>
 __device__ __forceinline__ void pair_add_real(Acc &a, double dx, double dy, double k2,
                                               double thresh2, bool le, double2 q, double2 d,
                                               double2 v) {
-    const double s = (dx * dx + dy * dy) * k2;
-    if (le ? (s <= thresh2) : (s < thresh2)) return;
-    const double si = 1.0 / s;
+    double s = (dx * dx + dy * dy) * k2;
+    if (le ? (s <= thresh2) : (s < thresh2)) {  // contributes zero, without a branch
+        s = 1.0;
+        q = d = make_double2(0.0, 0.0);
+    }
+    const double si = rcp_any(s);
     double2 h0, g;
     if (s < hb::kSMax) {
-        hb::hankel01_sq(s, si, h0, g);
+        hb::hankel01_sq<true>(s, si, h0, g);
     } else {
         hankel01_far(s, h0, g);
     }
