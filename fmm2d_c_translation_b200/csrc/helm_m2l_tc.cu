@@ -7,7 +7,7 @@
 // (same scale rs) is
 //     L_i += sum_j B_ij M_j,   B_ij = T(i - j) w_ij,
 // with T(q) the scaled Hankel table of the offset (H_|q|(k|d|) rs^|q| times
-// the phase e^{-i q theta}, shift_table in helmholtz.cu) and w_ij = 1 when
+// the phase e^{-i q theta}, helm_tables.cuh) and w_ij = 1 when
 // i j <= 0, rs^(2 min(|i|, |j|)) otherwise.  B depends only on the level
 // and the lattice offset between the two boxes, and a target box at child
 // position c sees exactly 27 possible offsets (the slot tables of m2l.cu).
@@ -29,15 +29,17 @@
 // Pipeline (one block per SM, persistent over the level's tiles): the K
 // dimension of each slot is cut into chunks of 16, and every (slot, chunk)
 // step stages A (128 x 16, hi and lo: gathered with cp.async from
-// operand-ready rows built once per level) and Bop (N x 16, hi and lo: one bulk
-// copy of a contiguous block of the per-level images) into one of kHtStages
-// shared-memory stages.  Warps 0-3 fill the stages, keeping kHtLag groups of
-// copies in flight; four lanes share an A row, whose chunk (hi and lo) is one
-// 128-byte line, so that a copy instruction touches 8 lines instead of 32.
-// Bound by the producers (issuing the copies, the proxy fence and the hand-over
-// are about half of the 1,300 cycles of a step) and by what every SM reads from
-// L2, 26 KB per step; 2.6 -> 2.3 ms for the levels of 2e6 points at order
-// 19.  Warp 12 issues
+// operand-ready rows built once per level; a lane per row) and Bop (N x 16, hi
+// and lo: a contiguous block of the per-level images, by one bulk copy or by
+// cp.async) into one of kHtStages shared-memory stages.  Warps 0-3 fill the
+// stages, keeping kHtLag groups of copies in flight; a step is handed over
+// kHtLag steps after its copies were issued, so kHtStages - kHtLag steps hide
+// the way through the tensor cores and back.  Bound by the producers (issuing
+// the copies, the proxy fence and the hand-over are about half of the 1,300
+// cycles of a step) and by what every SM reads from L2, 26 KB per step; with
+// four stages and the FP64 sums in shared memory the levels of 2e6 points at
+// order 19 took 2.6 ms, here 2.2.  (Four lanes per row, eight lines per copy
+// instruction instead of 32, measured slower: 2.3 ms.)  Warp 12 issues
 // 3 x 2 MMAs per step and commits the stage back.  Each slot accumulates
 // in a fresh tensor-memory tile (two alternate), and warps 4-11 (two per lane
 // quarter, half of the columns each) add every
@@ -65,7 +67,7 @@ namespace {
 
 constexpr int kHtRows = 128;
 constexpr int kHtStages = 7;
-constexpr int kHtLag = 3;
+constexpr int kHtLag = 2;
 constexpr int kHtEpi0 = 4;             // warps 4-11 read the accumulators
 constexpr int kHtEpiWarps = 8;
 constexpr int kHtThreads = 13 * 32;    // warp 12 issues the MMAs
@@ -113,7 +115,11 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-template <int KP, int NP>
+// BULK: Bop by one bulk copy per step -- taken where every slot is summed on
+// its own (the Helmholtz levels: 2.64 against 2.84 ms of M2L), while the
+// producers' copies are faster where a tile's slots share an accumulator (the
+// split mode on a curve of 8e6 points: 20.1 against 20.8 ms of the call).
+template <int KP, int NP, bool BULK>
 __global__ void __launch_bounds__(kHtThreads, 1) slot_gemm_tc_kernel(HtArgs A) {
     constexpr int KC = KP / 16;                      // K chunks per slot
     constexpr uint32_t A_BYTES = kHtRows * 16 * 4;   // one of hi / lo
@@ -171,9 +177,9 @@ __global__ void __launch_bounds__(kHtThreads, 1) slot_gemm_tc_kernel(HtArgs A) {
 
     if (warp < kHtEpi0) {
         // ------------------------------------------------------- producers
-        // this thread's quarter of the 16 columns of rows 32 warp + 8 i + lane / 4
-        const int qt = lane & 3, r0 = warp * 32 + (lane >> 2);
-        const uint32_t aoff = (uint32_t)qt * LBO_A + (uint32_t)(warp * 4 * 128 + (lane >> 2) * 16);
+        const int r = tid;  // A row
+        const int bx = r / A.nd, ch = r - bx * A.nd;
+        const uint32_t aoff = (uint32_t)(((r >> 3) * 128) + ((r & 7) * 16));
         long long step = 0;
         int st_i = 0, full_i = kHtStages - kHtLag;  // stages of step, step - lag
         uint32_t ph = 1;  // parity of the stage's previous release
@@ -181,26 +187,14 @@ __global__ void __launch_bounds__(kHtThreads, 1) slot_gemm_tc_kernel(HtArgs A) {
         for (int tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x) {
             int cp, q0;
             tile_seg(tile, cp, q0);
-            int q[4], ch[4], sb[4], nx[4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const int r = r0 + 8 * i, bx = r / A.nd;
-                ch[i] = r - bx * A.nd;
-                q[i] = bx < A.tpt && q0 + bx < A.start[cp] + A.count[cp] ? q0 + bx : -1;
-                nx[i] = q[i] >= 0 ? __ldg(A.slots + (size_t)q[i] * kHtSlots + k0) : -1;
-            }
+            const int q = bx < A.tpt && q0 + bx < A.start[cp] + A.count[cp] ? q0 + bx : -1;
+            const int *qs = A.slots + (size_t)(q >= 0 ? q : 0) * kHtSlots;
+            int next = q >= 0 ? __ldg(qs + k0) : -1;
             for (int k = k0; ok && k < k1; k++) {
-                const float *src[4];
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    sb[i] = nx[i];
-                    src[i] = A.arow + 4 * qt +
-                             (sb[i] >= 0 ? ((size_t)(sb[i] - A.lstart) * A.nd + ch[i]) * 2 * KP : 0);
-                    // (the next slot's sources)
-                    nx[i] = k + 1 < k1 && q[i] >= 0
-                                ? __ldg(A.slots + (size_t)q[i] * kHtSlots + k + 1)
-                                : -1;
-                }
+                const int sb = next;
+                next = k + 1 < k1 && q >= 0 ? __ldg(qs + k + 1) : -1;  // the next slot's source
+                const float *src = A.arow + (sb >= 0 ? ((size_t)(sb - A.lstart) * A.nd + ch) * 2 * KP : 0);
+                const uint32_t bytes = sb >= 0 ? 16u : 0u;  // 0: zero fill
                 const float *bsrc = A.bimg + ((size_t)(cp * kHtSlots + k) * KC) * (2 * NP * 16);
                 for (int kc = 0; kc < KC; kc++, step++) {
                     if (step >= kHtStages &&
@@ -209,7 +203,12 @@ __global__ void __launch_bounds__(kHtThreads, 1) slot_gemm_tc_kernel(HtArgs A) {
                         break;
                     }
                     const uint32_t st = sbase + (uint32_t)st_i * STAGE;
-                    if (tid == 0) {
+                    if (!BULK) {
+                        const float *bc = bsrc + (size_t)kc * (2 * NP * 16);
+#pragma unroll
+                        for (int e = tid; e < NP * 8; e += kHtRows)
+                            cp_async16(st + 2 * A_BYTES + 16u * (uint32_t)e, bc + 4 * e, 16u);
+                    } else if (tid == 0) {
                         const uint32_t bar = HBAR(2 * kHtStages + 5 + st_i);
                         mbar_arrive_expect_tx(bar, 2 * B_BYTES);
                         bulk_g2s(st + 2 * A_BYTES, bsrc + (size_t)kc * (2 * NP * 16), 2 * B_BYTES,
@@ -217,10 +216,9 @@ __global__ void __launch_bounds__(kHtThreads, 1) slot_gemm_tc_kernel(HtArgs A) {
                     }
 #pragma unroll
                     for (int i = 0; i < 4; i++) {
-                        const uint32_t bytes = sb[i] >= 0 ? 16u : 0u;  // 0: zero fill
-                        const uint32_t d = st + aoff + (uint32_t)i * 128u;
-                        cp_async16(d, src[i] + 32 * kc, bytes);
-                        cp_async16(d + A_BYTES, src[i] + 32 * kc + 16, bytes);
+                        const uint32_t d = st + (uint32_t)i * LBO_A + aoff;
+                        cp_async16(d, src + 32 * kc + 4 * i, bytes);
+                        cp_async16(d + A_BYTES, src + 32 * kc + 16 + 4 * i, bytes);
                     }
                     cp_async_commit();
                     if (step >= kHtLag) {
@@ -244,7 +242,7 @@ __global__ void __launch_bounds__(kHtThreads, 1) slot_gemm_tc_kernel(HtArgs A) {
         } else {
             *abort_flag = 1;
         }
-        if (tid == 0) {
+        if (BULK && tid == 0) {
             // the last bulk copies have landed before the block exits (the
             // issuer has waited for them unless the block stopped early)
             int never = 0;
@@ -372,9 +370,9 @@ __global__ void __launch_bounds__(kHtThreads, 1) slot_gemm_tc_kernel(HtArgs A) {
                     if (!__all_sync(0xffffffffu,
                                     mbar_wait_bounded(HBAR(s), (uint32_t)(u & 1), abort_flag,
                                                       A.wait_ns) &&
-                                        mbar_wait_bounded(HBAR(2 * kHtStages + 5 + s),
-                                                          (uint32_t)(u & 1), abort_flag,
-                                                          A.wait_ns))) {
+                                        (!BULK || mbar_wait_bounded(HBAR(2 * kHtStages + 5 + s),
+                                                                    (uint32_t)(u & 1), abort_flag,
+                                                                    A.wait_ns)))) {
                         ok = false;
                         break;
                     }
@@ -505,9 +503,13 @@ __global__ void __launch_bounds__(256) helm_tc_bimg_kernel(int p, int KP, int NP
 template <int KP, int NP>
 void launch_ht(const HtArgs &a, int ntiles, int nslice, cudaStream_t s) {
     const size_t smem = ht_smem_bytes<KP, NP>();
-    raise_smem_limit((const void *)slot_gemm_tc_kernel<KP, NP>, smem);
     const dim3 grid(std::max(1, std::min(ntiles, kNumSM)), nslice);
-    slot_gemm_tc_kernel<KP, NP><<<grid, kHtThreads, smem, s>>>(a);
+    auto launch = [&](auto kern) {
+        raise_smem_limit((const void *)kern, smem);
+        kern<<<grid, kHtThreads, smem, s>>>(a);
+    };
+    if (a.group == 1) launch(slot_gemm_tc_kernel<KP, NP, true>);
+    else launch(slot_gemm_tc_kernel<KP, NP, false>);
     FMM_CHECK_LAUNCH();
 }
 
