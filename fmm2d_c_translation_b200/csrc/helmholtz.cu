@@ -13,13 +13,18 @@
 //     sources.  Each lane generates its Bessel sequence (Miller's downward
 //     recurrence for J, two passes so the normalisation is known before the
 //     coefficients are emitted; the upward recurrence for H) and the
-//     coefficient contributions are summed across the warp per order.
+//     coefficient contributions are summed across the warp per order.  A
+//     positive real wavenumber takes real recurrences (helm_real.cuh).
 //   * M2M, M2L, L2L (h2dmpmp, h2dmploc, h2dlocloc): all three are
 //     out_i = S_i sum_j in_j T(i - j) r1^e(i, j) with T a table of J_m or H_m
 //     times e^{-i m theta} for the (fixed, per level) offset between the two
-//     centers, S_i and r1^e powers of the two scales.  One thread per output
-//     coefficient; the tables are built on the host per level and offset.
-//   * M2P + L2P (h2dmpeval*, h2dtaeval*): one thread per point, upward H
+//     centers, S_i and r1^e powers of the two scales.  The tables are built
+//     on the device for every call (helm_tables.cuh); M2M and L2L fold the
+//     four children by quarter turns (helm_shift.cuh), the M2L takes tiles of
+//     boxes of all levels in one launch (helm_m2l_stage_kernel), and the
+//     general forms have one thread per output coefficient.
+//   * M2P + L2P (h2dmpeval*, h2dtaeval*): one thread per point (several per
+//     point in small calls with a real wavenumber, helm_real.cuh), upward H
 //     (multipoles of list 3) and downward J (the leaf's local expansion),
 //     derivatives from the mk_mpoleg / mk_mpoleh coefficient recurrences
 //     evaluated on the fly.

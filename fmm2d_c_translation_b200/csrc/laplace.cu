@@ -507,8 +507,8 @@ template <bool FAST> __device__ __forceinline__ float half_ln_pair(float x) {
 // arithmetic, in the same order, as eval_far_points_kernel.
 // Whether steps 6-7 run with one warp per leaf (coefficients staged once per
 // box) or one thread per point.  Measured on a B200 (10^7 + 10^7 uniform
-// points): per leaf is faster in FP64 at p = 37 (3.9 against 4.1 ms), per
-// point in the mixed mode at p = 18 (2.0 against 2.4 ms), where a leaf's
+// points): per leaf is faster in FP64 at p = 37 (3.2 against 4.7 ms), per
+// point in the mixed mode at p = 18 (1.3 against 2.2 ms), where a leaf's
 // ~19 points leave a third of the warp idle.  FMM2D_B200_FAR=leaf / point
 // overrides.
 bool far_per_leaf(const CauchyProblem &P) {
@@ -1127,9 +1127,10 @@ void launch_p2p_t(const Tree &T, const CauchyProblem &P, int c0, double th2,
     const PT *spos = MIXED ? (const PT *)P.src_hl : (const PT *)P.src;
     const PT *tpos = MIXED ? (const PT *)P.trg_hl : (const PT *)P.tset.pos;
     // Flattened items in the mixed mode, equal lane groups in FP64: measured
-    // on a B200 (10^7 + 10^7 uniform points, lfmm2d_st_cd_g) 5.56 against
-    // 5.75 ms mixed, 19.1 against 17.1 ms FP64, where the flattened form's
-    // larger register and shared-memory footprint costs occupancy.
+    // on a B200 (10^7 + 10^7 uniform points, lfmm2d_st_cd_g) 4.6 against
+    // 5.8 ms mixed, 16.6 against 10.6 ms FP64, where the flattened form's
+    // larger register and shared-memory footprint costs occupancy (and it
+    // divides and calls log()).
     // FMM2D_B200_P2P=flat / group overrides.  In FP64 the groups take the
     // reciprocal and logarithm of normal numbers: the pairs that count lie
     // between thresh^2 and 2^103 thresh^2 (the threshold is 2^-51 of the
