@@ -8,12 +8,11 @@
 // per level for the counts, they took 1.08 ms on 4e5 clustered points (12
 // levels; here 0.43), 0.87 ms on 5e4 (0.35), 2.76 ms on the 8e6 points of a
 // boundary curve (18 levels; 2.10, bound by the colleagues' loads).  Here they
-// are
-// phases of one kernel with a grid-wide barrier between them; counts stay on
-// the device, and one status read at the end gives the host the new level
-// ranges.  The boxes' arrays are sized with room for the added boxes; when
-// that does not suffice the kernel stops before writing past the end and
-// the host builds again with more room.
+// are phases of one kernel with a grid-wide barrier between them; counts stay
+// on the device, and one status read at the end gives the host the new level
+// ranges.  The boxes' arrays are sized with room for the added boxes; when that
+// does not suffice the kernel stops before writing past the end and the host
+// builds again with more room.
 #pragma once
 
 // The arrays of one numbering of the boxes (the reorganisations copy from
