@@ -1714,8 +1714,9 @@ inline int pascal_grid(int64_t nthreads) {
 constexpr int kPowSrc = 8;
 constexpr int kPowWarps = 8;
 
-// Row of a source's powers: an odd number of 16-byte words.
-__host__ __device__ inline int pow_row(int p) { return (p + 1) | 1; }
+// Row of a source's powers: an odd number of 16-byte words, and room for the
+// first power of each of its four lanes (orders 1 and 2 use two or three).
+__host__ __device__ inline int pow_row(int p) { return (p < 3 ? 4 : p + 1) | 1; }
 
 inline size_t pow_warp_smem(int p, int CH) {
     // per warp: powers [kPowSrc][row], strengths [kPowSrc][2 CH]
