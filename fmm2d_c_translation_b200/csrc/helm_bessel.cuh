@@ -155,8 +155,10 @@ inline std::vector<double2> make_table() {
     return tab;
 }
 
-// Puts the table on the current device, once per device and process.
-inline void ensure_table() {
+// Puts the table on the current device, once per device and process.  On the
+// call's own stream and waited for: the library's streams do not order with
+// the legacy one, and a pageable copy there may return before it has landed.
+inline void ensure_table(cudaStream_t s) {
     static std::mutex mu;
     static std::vector<char> done;
     static std::vector<double2> tab;
@@ -166,8 +168,11 @@ inline void ensure_table() {
     if ((int)done.size() <= dev) done.resize(dev + 1, 0);
     if (done[dev]) return;
     if (tab.empty()) tab = make_table();
-    FMM_CUDA(cudaMemcpyToSymbol(g_tab, tab.data(), tab.size() * sizeof(double2)));
-    FMM_CUDA(cudaMemcpyToSymbol(c_tab0, tab.data(), sizeof(c_tab0)));
+    FMM_CUDA(cudaMemcpyToSymbolAsync(g_tab, tab.data(), tab.size() * sizeof(double2), 0,
+                                     cudaMemcpyHostToDevice, s));
+    FMM_CUDA(cudaMemcpyToSymbolAsync(c_tab0, tab.data(), sizeof(c_tab0), 0,
+                                     cudaMemcpyHostToDevice, s));
+    FMM_CUDA(cudaStreamSynchronize(s));
     done[dev] = 1;
 }
 

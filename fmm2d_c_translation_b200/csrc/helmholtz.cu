@@ -1864,7 +1864,7 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
     const bool realk = zk.y == 0.0 && zk.x > 0.0;
     int lreal = nl + 1;
     if (realk) {
-        hb::ensure_table();
+        hb::ensure_table(s);
         while (lreal > 0 && hl[lreal - 1].p <= kRealOrderMax &&
                zk.x * T.boxsize[lreal - 1] * 0.7072 <= kRealXMax)
             lreal--;
@@ -2185,7 +2185,7 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
             if (!realk) {
                 HP2PK(0);
             } else {
-                hb::ensure_table();
+                hb::ensure_table(s);
                 if (ifc && ifd) HP2PK(3);
                 else if (ifd) HP2PK(2);
                 else HP2PK(1);
