@@ -29,7 +29,8 @@ constexpr double const_ln(double x) {  // 2 atanh((x - 1) / (x + 1))
     return 2.0 * s;
 }
 
-struct LnTable {
+// (aligned for the 16-byte load of an entry)
+struct alignas(sizeof(double2)) LnTable {
     double v[2 * kLnEntries];  // c, -ln(c) / 2
     constexpr LnTable() : v() {
         for (int i = 0; i < kLnEntries; i++) {
@@ -42,6 +43,7 @@ struct LnTable {
     }
 };
 static __device__ LnTable g_ln_table = LnTable();
+static_assert(alignof(decltype(g_ln_table)) >= alignof(double2), "entries are read as double2");
 
 __device__ __forceinline__ double rcp_pos(double x) {
     double y;
