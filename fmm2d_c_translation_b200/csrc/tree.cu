@@ -1384,18 +1384,18 @@ bool build_by_keys(const double2 *d_src, int ns, const double2 *d_targ, int nt, 
         const size_t ncnt = (size_t)(ds + 1) * nwarp;
         DevBuf<int> cnt(ncnt, s), off(ncnt + 1, s);
         const int nw = (ds + 15) / 16, blocks = (nwarp + 7) / 8;
-        refine_runs_kernel<true><<<blocks, 256, 0, s>>>(B.kvs, ks.prob.get(), ns, ndiv, ds, nw,
-                                                        chunk, nwarp, cnt.get(), nullptr);
-        FMM_CHECK_LAUNCH();
-        exclusive_scan_i32(cnt.get(), off.get(), (int64_t)ncnt, off.get() + ncnt, s);
-        DevBuf<int> lo(ds + 2, s);
-        {
+        std::vector<int> h(ds + 2, 0);
+        if (ns > 0) {  // (without sources: the roots alone)
+            refine_runs_kernel<true><<<blocks, 256, 0, s>>>(B.kvs, ks.prob.get(), ns, ndiv, ds, nw,
+                                                            chunk, nwarp, cnt.get(), nullptr);
+            FMM_CHECK_LAUNCH();
+            exclusive_scan_i32(cnt.get(), off.get(), (int64_t)ncnt, off.get() + ncnt, s);
+            DevBuf<int> lo(ds + 2, s);
             int *lp = lo.get();
             const int *op = off.get();
             for_each(ds + 2, s, [=] __device__(int64_t l) { lp[l] = op[(size_t)l * nwarp]; });
+            read_small(h.data(), lo.get(), h.size() * sizeof(int), s);
         }
-        std::vector<int> h(ds + 2);
-        read_small(h.data(), lo.get(), h.size() * sizeof(int), s);
         // a box of the deepest digit level still to be split: more digits
         if (ds < 64 && ds <= nlmax - 1 && h[ds + 1] > h[ds]) return false;
         sort_targets();
