@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(128) hf_apply_kernel(
             const int k = t / nd;
             double2 a = make_double2(0.0, 0.0);
             for (int e = 0; e < n2; e++) {
-                const int sb = list2[b * 27 + e];
+                const int sb = list2[b * kMaxList2 + e];
                 const double2 cs = centers[sb];
                 const int ix = (int)rint((cb.x - cs.x) / bs), iy = (int)rint((cb.y - cs.y) / bs);
                 const double2 f = F[(size_t)((iy + 3) * 7 + (ix + 3)) * N + k];

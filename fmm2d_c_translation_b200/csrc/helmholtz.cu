@@ -631,7 +631,7 @@ __global__ void __launch_bounds__(256) helm_m2l_kernel(
         const double2 cb = centers[b];
         double2 acc = make_double2(0.0, 0.0);
         for (int e = 0; e < n2l; e++) {
-            const int sb = list2[b * 27 + e];
+            const int sb = list2[b * kMaxList2 + e];
             const double2 cs = centers[sb];
             const int ix = (int)rint((cb.x - cs.x) / bs), iy = (int)rint((cb.y - cs.y) / bs);
             const double2 *Tt = T + (size_t)((iy + 3) * 7 + (ix + 3)) * tw + 2 * p;

@@ -1008,7 +1008,7 @@ LrOut restrict_levels(Builder &B, const double *d_bsl, int nroots, cudaStream_t 
     A.L = L;
     A.nroots = nroots;
     A.nboxes = T.nboxes;
-    A.cap = T.cap;
+    A.cap = std::min(T.cap, kMaxBoxes);
     A.leaf_sort = kLeafSort;
     for (int l = 0; l <= L; l++) {
         A.lstart[l] = T.lstart[l];
@@ -1410,7 +1410,7 @@ bool build_by_keys(const double2 *d_src, int ns, const double2 *d_targ, int nt, 
             R.off[l + 1] = h[l + 1];
             R.base[l + 1] = (int)nb;
             nb += 4 * (int64_t)(h[l + 1] - h[l]);
-            if (nb > INT32_MAX / 20) throw FmmError(4, "tree too large");
+            if (nb > kMaxBoxes) throw FmmError(4, "tree too large");
             T.boxsize.push_back(T.boxsize[l] / 2);
             T.lstart.push_back(R.base[l + 1]);
             T.lend.push_back((int)nb);
@@ -1431,14 +1431,17 @@ bool build_by_keys(const double2 *d_src, int ns, const double2 *d_targ, int nt, 
     }
     // with room for the boxes the level restriction adds: none on uniform
     // points, a tenth on clusters, more than the first build's own number on
-    // curves (trees much deeper than uniform points would make)
+    // curves (trees much deeper than uniform points would make); as far as a
+    // tree may grow.  FMM2D_B200_TREE_ROOM sets the first build's share.
     int flat = 2;
     for (int64_t q = std::max(ndiv, 1); q < std::max(ns, nt) && flat < nlmax; q *= 4) flat++;
     auto with_room = [&](int n) {
-        const double f = std::max(room, T.boxsize.size() > (size_t)flat + 2 ? 2.0 : 0.5);
-        const double c = n + std::max(1024.0, f * n);
-        if (c > INT32_MAX / 20) throw FmmError(4, "tree too large");
-        return (int)c;
+        const char *e = getenv("FMM2D_B200_TREE_ROOM");
+        double f = T.boxsize.size() > (size_t)flat + 2 ? 2.0 : 0.5;
+        if (e) f = std::max(0.0, atof(e));
+        f = std::max(room, f);
+        if (n > kMaxBoxes) throw FmmError(4, "tree too large");
+        return (int)std::min<double>(kMaxBoxes, n + std::max(1024.0, f * n));
     };
     B.ensure(with_room(std::max(4 * nroots, nboxes)));
     T.nboxes = nroots;
@@ -1514,6 +1517,7 @@ bool build_by_keys(const double2 *d_src, int ns, const double2 *d_targ, int nt, 
     B.ensure(with_room(T.nboxes));
     const LrOut lr = restrict_levels(B, d_bsl.get(), nroots, s);
     if (lr.status != 0) {
+        if (T.cap >= kMaxBoxes) throw FmmError(4, "tree too large");
         T.boxsize.resize(1);
         return build_by_keys(d_src, ns, d_targ, nt, ndiv, idivflag, nlmax, c0, ds, s, T, F,
                              std::max(4.0, 4.0 * room));
@@ -1631,6 +1635,7 @@ void build_forest(const double2 *d_src, const std::vector<int> &soff, const doub
 
 void compute_lists(Tree &T, cudaStream_t s) {
     const int nb = T.nboxes;
+    if (nb > kMaxBoxes) throw FmmError(4, "tree too large");
     T.nlist1.alloc(nb, s);
     T.list1.alloc((size_t)kMaxList1 * nb, s);
     T.nlist2.alloc(nb, s);

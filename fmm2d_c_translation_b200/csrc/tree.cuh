@@ -14,10 +14,12 @@ namespace fmm2d {
 
 // List capacities of the reference (c_translation/src/tree_routs2d.c:325-345).
 constexpr int kMaxList1 = 13;
-constexpr int kMaxList2 = 27;
+constexpr int64_t kMaxList2 = 27;  // (64-bit: kMaxBoxes times it is more than 2^31)
 constexpr int kMaxList3 = 20;
 constexpr int kMaxList4 = 5;
 constexpr int kMaxLevels = 51;  // nlmax of the reference drivers
+// Boxes of a tree: the other lists' places are 32-bit.
+constexpr int kMaxBoxes = INT32_MAX / kMaxList3;
 
 struct Tree {
     int nlevels = 0;
