@@ -27,6 +27,8 @@
 #include "sort.cuh"
 
 #include <algorithm>
+#include <stdlib.h>
+#include <string.h>
 
 namespace fmm2d {
 namespace {
@@ -35,9 +37,15 @@ constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kRadix = 256;
 constexpr int kMaxPasses = 4;
-// tile states: 2 flag bits over a 30-bit count
-constexpr uint32_t kOwn = 1u << 30, kIncl = 2u << 30, kCount = kOwn - 1;
 constexpr int kMaxSpin = 1 << 20;
+
+// Tile states: 2 flag bits over a count, of 30 bits in the 32-bit form and of
+// 62 in the 64-bit one, which 2^30 and more items take.
+template <class St>
+struct TileState {
+    static constexpr int kBits = 8 * sizeof(St) - 2;
+    static constexpr St kOwn = (St)1 << kBits, kIncl = (St)2 << kBits, kCount = kOwn - 1;
+};
 
 // Digit counts of every pass.
 __global__ void __launch_bounds__(kThreads) radix_hist_kernel(const uint32_t *__restrict__ keys,
@@ -120,12 +128,13 @@ __device__ __forceinline__ void rank_tile(TileSmem<ROUNDS> &S, const uint32_t *k
 }
 
 // One pass over all tiles; vin null: the values are the positions.
-template <int ROUNDS>
+template <int ROUNDS, class St>
 __global__ void __launch_bounds__(kThreads) radix_pass_kernel(
     const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vin,
     uint32_t *__restrict__ kout, uint32_t *__restrict__ vout, int64_t n, int shift,
-    const int *__restrict__ hist, int *__restrict__ next, volatile uint32_t *state) {
+    const int *__restrict__ hist, int *__restrict__ next, volatile St *state) {
     constexpr int kTile = kThreads * ROUNDS;
+    constexpr St kOwn = TileState<St>::kOwn, kIncl = TileState<St>::kIncl;
     __shared__ TileSmem<ROUNDS> S;
     const int tid = threadIdx.x;
     if (tid == 0) S.tile = atomicAdd(next, 1);
@@ -146,8 +155,8 @@ __global__ void __launch_bounds__(kThreads) radix_pass_kernel(
         if (r * kThreads + tid < cnt) atomicAdd(&S.run[(kr[r] >> shift) & 0xff], 1);
     __syncthreads();
     const int own = S.run[tid];
-    volatile uint32_t *st = state + (size_t)tile * kRadix + tid;
-    *st = (tile == 0 ? kIncl : kOwn) | (uint32_t)own;
+    volatile St *st = state + (size_t)tile * kRadix + tid;
+    *st = (tile == 0 ? kIncl : kOwn) | (St)own;
     const int lst = block_excl(own, S.wsum);
     const int gst = block_excl(hist[tid], S.wsum);  // the digit's first place
     S.lstart[tid] = lst;
@@ -157,9 +166,9 @@ __global__ void __launch_bounds__(kThreads) radix_pass_kernel(
     uint32_t before = 0;
     int spins = 0;
     for (int t = tile - 1; t >= 0;) {
-        const uint32_t v = state[(size_t)t * kRadix + tid];
+        const St v = state[(size_t)t * kRadix + tid];
         if (v >= kOwn) {
-            before += v & kCount;
+            before += (uint32_t)(v & TileState<St>::kCount);
             if (v >= kIncl) break;
             t--;
         } else if (++spins > kMaxSpin) {
@@ -168,7 +177,7 @@ __global__ void __launch_bounds__(kThreads) radix_pass_kernel(
             break;
         }
     }
-    if (tile > 0) *st = kIncl | (before + (uint32_t)own);
+    if (tile > 0) *st = kIncl | (St)(before + (uint32_t)own);
     S.gdelta[tid] = gst + (int)before - lst;
     __syncthreads();
     for (int i = tid; i < cnt; i += kThreads) {
@@ -224,22 +233,22 @@ __global__ void __launch_bounds__(kThreads) radix_one_kernel(
     }
 }
 
-template <int ROUNDS>
+template <int ROUNDS, class St>
 void sort_passes(const uint32_t *kin, const uint32_t *vin, uint32_t *const k[2],
                  uint32_t *const v[2], int64_t n, int lo_bit, int passes, cudaStream_t s) {
     const int64_t tile = (int64_t)kThreads * ROUNDS;
     const int ntiles = (int)((n + tile - 1) / tile);
-    // per pass: digit counts and the tile counter, then the tile states
-    const size_t head = (size_t)passes * (kRadix + 1), per = (size_t)ntiles * kRadix;
-    DevBuf<int> work(head + passes * per, s);
+    // per pass the tile states, then digit counts and the tile counter
+    const size_t per = (size_t)ntiles * kRadix, head = (size_t)passes * (kRadix + 1);
+    DevBuf<int> work(passes * per * (sizeof(St) / sizeof(int)) + head, s);
     work.zero(s);
-    int *hist = work.get(), *next = hist + passes * kRadix;
-    uint32_t *state = reinterpret_cast<uint32_t *>(work.get()) + head;
+    St *state = reinterpret_cast<St *>(work.get());
+    int *hist = reinterpret_cast<int *>(state + passes * per), *next = hist + passes * kRadix;
     const int blocks = (int)std::min<int64_t>((n + 2047) / 2048, kNumSM * 4);
     radix_hist_kernel<<<blocks, kThreads, 0, s>>>(kin, n, lo_bit, passes, hist);
     FMM_CHECK_LAUNCH();
     for (int p = 0; p < passes; p++) {
-        radix_pass_kernel<ROUNDS><<<ntiles, kThreads, 0, s>>>(
+        radix_pass_kernel<ROUNDS, St><<<ntiles, kThreads, 0, s>>>(
             p == 0 ? kin : k[(p - 1) & 1], p == 0 ? vin : v[(p - 1) & 1], k[p & 1], v[p & 1], n,
             lo_bit + 8 * p, hist + p * kRadix, next + p, state + p * per);
         FMM_CHECK_LAUNCH();
@@ -251,7 +260,6 @@ void sort_passes(const uint32_t *kin, const uint32_t *vin, uint32_t *const k[2],
 int radix_sort_into(const uint32_t *kin, const uint32_t *vin, uint32_t *const k[2],
                     uint32_t *const v[2], int64_t n, int key_bits, cudaStream_t s, int lo_bit) {
     if (n <= 0) return 0;
-    if (n >= (int64_t)kOwn) throw FmmError(4, "sort: more than 2^30 items");
     const int passes = std::max(1, (key_bits - lo_bit + 7) / 8);
     if (passes > kMaxPasses) throw FmmError(4, "sort: more than 32 key bits");
     if (n <= kThreads * kOneRounds) {
@@ -259,11 +267,14 @@ int radix_sort_into(const uint32_t *kin, const uint32_t *vin, uint32_t *const k[
         FMM_CHECK_LAUNCH();
         return 0;
     }
-    // tiles of 1,024 items while larger ones would leave SMs without one
-    if (n < (int64_t)kThreads * 16 * kNumSM)
-        sort_passes<4>(kin, vin, k, v, n, lo_bit, passes, s);
-    else
-        sort_passes<16>(kin, vin, k, v, n, lo_bit, passes, s);
+    // 64-bit states from 2^30 items on (FMM2D_B200_SORT_WIDE=1: always); tiles
+    // of 1,024 items while larger ones would leave SMs without one
+    const char *e = getenv("FMM2D_B200_SORT_WIDE");
+    const bool wide = n > (int64_t)TileState<uint32_t>::kCount || (e && !strcmp(e, "1"));
+    const bool small = n < (int64_t)kThreads * 16 * kNumSM;
+    auto sort = wide ? (small ? sort_passes<4, unsigned long long> : sort_passes<16, unsigned long long>)
+                     : (small ? sort_passes<4, uint32_t> : sort_passes<16, uint32_t>);
+    sort(kin, vin, k, v, n, lo_bit, passes, s);
     return (passes - 1) & 1;
 }
 
