@@ -10,6 +10,9 @@
 #include "runtime.cuh"
 #include "tree.cuh"
 
+#include <cuda.h>
+
+#include <algorithm>
 #include <atomic>
 #include <memory>
 #include <mutex>
@@ -880,19 +883,42 @@ __global__ void __launch_bounds__(256) copy_items_kernel(const CopyItem *__restr
     }
 }
 
+// Whether n bytes at p lie inside one allocation on device dev.
+bool in_device_memory(const void *p, size_t n, int dev) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (a.type != cudaMemoryTypeDevice || a.device != dev) return false;
+    typedef CUresult (*Range)(CUdeviceptr *, size_t *, CUdeviceptr);
+    static const Range range = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult r;
+        if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &f, 12000, cudaEnableDefault,
+                                             &r) != cudaSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<Range>(f);
+    }();
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    const CUdeviceptr q = reinterpret_cast<CUdeviceptr>(p);
+    return range && range(&base, &size, q) == CUDA_SUCCESS && q - base <= size &&
+           n <= size - (q - base);
+}
+
 // Copies between the concatenated arrays and the caller's: those on this
-// device in one launch, any other (host, another device) by a copy of its own.
+// device in one launch, any other (host, another device, not at a multiple of
+// 8 bytes, or not inside one allocation, which the copy then reports) by a copy
+// of its own.
 class ItemCopies {
   public:
     explicit ItemCopies(int dev) : dev_(dev) {}
     void add(void *dst, const void *src, const void *user, size_t bytes, cudaStream_t s) {
         if (!bytes) return;
-        cudaPointerAttributes a;
-        if (cudaPointerGetAttributes(&a, user) != cudaSuccess) {
-            cudaGetLastError();
-            a.type = cudaMemoryTypeUnregistered;
-        }
-        if (a.type == cudaMemoryTypeDevice && a.device == dev_)
+        if ((reinterpret_cast<uintptr_t>(user) & 7) == 0 && in_device_memory(user, bytes, dev_))
             items_.push_back({static_cast<const double *>(src), static_cast<double *>(dst),
                               (long long)(bytes / sizeof(double))});
         else
@@ -900,6 +926,11 @@ class ItemCopies {
     }
     void run(cudaStream_t s) {
         if (items_.empty()) return;
+        if (overlapping()) {  // (the later problem's values stay)
+            for (const CopyItem &i : items_)
+                FMM_CUDA(cudaMemcpyAsync(i.dst, i.src, i.n * sizeof(double), cudaMemcpyDefault, s));
+            return;
+        }
         buf_.alloc(items_.size(), s);
         FMM_CUDA(cudaMemcpyAsync(buf_.get(), items_.data(), items_.size() * sizeof(CopyItem),
                                  cudaMemcpyHostToDevice, s));
@@ -914,6 +945,15 @@ class ItemCopies {
     }
 
   private:
+    // whether two items write the same place
+    bool overlapping() const {
+        std::vector<std::pair<const double *, const double *>> r;
+        for (const CopyItem &i : items_) r.push_back({i.dst, i.dst + i.n});
+        std::sort(r.begin(), r.end());
+        for (size_t k = 1; k < r.size(); k++)
+            if (r[k].first < r[k - 1].second) return true;
+        return false;
+    }
     int dev_;
     std::vector<CopyItem> items_;
     DevBuf<CopyItem> buf_;
