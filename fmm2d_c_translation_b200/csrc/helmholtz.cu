@@ -2182,7 +2182,9 @@ void helmholtz_fmm(const Tree &T, const HelmProblem &P, cudaStream_t s) {
         else if (X.pgh == 2) HP2PF(2, KD); \
         else HP2PF(3, KD);                 \
     } while (0)
-            if (!realk) {
+            // (the real pairs form (k r)^2 with k^2, which has to be a normal number)
+            const double k2 = zk.x * zk.x;
+            if (!realk || !(k2 >= 2.3e-308 && k2 <= 1e300)) {
                 HP2PK(0);
             } else {
                 hb::ensure_table(s);
