@@ -355,7 +355,7 @@ void laplace_evaluate(const FmmCall &c, const LapGeometry &G, bool on_dev, cudaS
     // the M2L's error flag comes with the call's last synchronisation instead
     // of one of its own (about 15 us of a call of 300 to 10^5 points)
     DevBuf<int> m2l_err;
-    if (sync && G.mixed && !m2l) {
+    if (sync && G.mixed && !m2l && T.nlevels >= 2) {
         m2l_err.alloc(1, s);
         FMM_CUDA(cudaMemsetAsync(m2l_err.get(), 0, sizeof(int), s));
         P.m2l_err = m2l_err.get();
