@@ -1337,32 +1337,40 @@ __device__ __forceinline__ int child_pos(const int *__restrict__ child, int pb, 
 // with the fixed shift matrices A of the four child positions.
 // The parents visited come from a BoxList or, with ids null, are all boxes of
 // [lo, hi) with children.
-// Four lanes per output, one per child.
-template <int CH>
+// LANES = 4: a lane per child, for small levels, which take one output's
+// latency; LANES = 1: a thread per output, whose warp's loads are one or two
+// boxes' coefficients and neighbouring table entries, for the large levels of
+// the orders above 39 (4e6 points, order 43: 1.30 ms; four lanes over the whole
+// of the triangular table took 3.69).
+template <int CH, int LANES>
 __global__ void __launch_bounds__(256) m2m_coef_kernel(
     int lo, int hi, int p, const int *__restrict__ ids, const int *__restrict__ nids,
     const int *__restrict__ nchild, const int *__restrict__ child, const int2 *__restrict__ sse,
     const double2 *__restrict__ A, int ndc, int c0, double2 *__restrict__ mp) {
     const int np1 = p + 1, stride = np1 * ndc;
-    const int64_t n = (int64_t)(ids ? *nids : hi - lo) * np1 * 4;
+    const int64_t n = (int64_t)(ids ? *nids : hi - lo) * np1 * LANES;
     // warp-uniform trip count: the lanes of an output meet in the shuffles
     for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n;
          base += (int64_t)gridDim.x * blockDim.x) {
         const int64_t t = base + threadIdx.x;
         const bool valid = t < n;
-        const int64_t o = valid ? t >> 2 : 0;
-        const int k = (int)(o / np1), i = (int)(o % np1), cp = (int)(t & 3);
+        const int64_t o = valid ? t / LANES : 0;
+        const int k = (int)(o / np1), i = (int)(o % np1), lane = (int)(t % LANES);
         const int b = ids ? ids[k] : lo + k;
         const bool par = valid && nchild[b] != 0;
-        const int cb = par ? child[4 * b + cp] : -1;
+        const int nj = min(np1, (i & ~7) + 8);  // (entries j > i are zero)
         double2 acc[CH];
 #pragma unroll
         for (int q = 0; q < CH; q++) acc[q] = make_double2(0.0, 0.0);
-        if (cb >= 0 && count(sse, cb) > 0) {
+#pragma unroll
+        for (int u = 0; u < 4 / LANES; u++) {
+            const int cp = LANES == 4 ? lane : u;
+            const int cb = par ? child[4 * b + cp] : -1;
+            if (cb < 0 || count(sse, cb) <= 0) continue;
             const double2 *At = A + (size_t)cp * np1 * np1 + i;
             const double2 *M = mp + (size_t)cb * stride + c0;
 #pragma unroll 8
-            for (int j = 0; j < np1; j++) {  // (entries j > i are zero)
+            for (int j = 0; j < nj; j++) {
                 const double2 a = __ldg(At + (size_t)j * np1);
 #pragma unroll
                 for (int q = 0; q < CH; q++) cfma(acc[q], a, M[(size_t)j * ndc + q]);
@@ -1371,11 +1379,11 @@ __global__ void __launch_bounds__(256) m2m_coef_kernel(
 #pragma unroll
         for (int q = 0; q < CH; q++) {
 #pragma unroll
-            for (int d = 1; d < 4; d <<= 1) {
+            for (int d = 1; d < LANES; d <<= 1) {
                 acc[q].x += __shfl_xor_sync(0xffffffffu, acc[q].x, d);
                 acc[q].y += __shfl_xor_sync(0xffffffffu, acc[q].y, d);
             }
-            if (par && cp == 0) mp[(size_t)b * stride + (size_t)i * ndc + c0 + q] = acc[q];
+            if (par && lane == 0) mp[(size_t)b * stride + (size_t)i * ndc + c0 + q] = acc[q];
         }
     }
 }
@@ -2135,8 +2143,12 @@ void upward_chunk(const Tree &T, const CauchyProblem &P, int c0,
         const int64_t nt = (int64_t)(hi - lo) * CH * 4;
         const int *ids = P.m2m_ids ? P.m2m_ids + lo : nullptr;
         const int *nid = P.m2m_ids ? P.m2m_cnt + l : nullptr;
-        if (shift_matrix(P, nt))
-            m2m_coef_kernel<CH><<<blocks(4 * (hi - lo)), 256, 0, s>>>(
+        if (shift_matrix(P, nt) && nt <= kShiftMatrixPairs)
+            m2m_coef_kernel<CH, 4><<<blocks(4 * (hi - lo)), 256, 0, s>>>(
+                lo, hi, p, ids, nid, T.nchild.get(), T.child.get(), T.srcse.get(), A, P.ndc,
+                c0, mp);
+        else if (shift_matrix(P, nt))
+            m2m_coef_kernel<CH, 1><<<blocks(hi - lo), 256, 0, s>>>(
                 lo, hi, p, ids, nid, T.nchild.get(), T.child.get(), T.srcse.get(), A, P.ndc,
                 c0, mp);
         else if (p + 1 <= 20)
