@@ -1023,11 +1023,19 @@ LrOut restrict_levels(Builder &B, const double *d_bsl, int nroots, cudaStream_t 
     A.blkcnt = A.levcnt + kRefLevels;
     int per_sm = 0;
     FMM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tree_lr_kernel, kLrThreads, 0));
-    // (a block takes 32 boxes at a time with a warp per four)
-    const int blocks = std::max(1, std::min(std::min(kLrBlocks, per_sm * kNumSM), T.nboxes / 64));
+    // (a block takes 32 boxes at a time with a warp per four; where the stream
+    // has fewer SMs than the chip, the launch is refused and fewer blocks go)
+    int blocks = std::max(1, std::min(std::min(kLrBlocks, per_sm * kNumSM), T.nboxes / 64));
     void *args[] = {&A};
-    FMM_CUDA(cudaLaunchCooperativeKernel((const void *)tree_lr_kernel, dim3(blocks),
-                                         dim3(kLrThreads), args, 0, s));
+    cudaError_t err;
+    while ((err = cudaLaunchCooperativeKernel((const void *)tree_lr_kernel, dim3(blocks),
+                                              dim3(kLrThreads), args, 0, s)) ==
+               cudaErrorCooperativeLaunchTooLarge &&
+           blocks > 1) {
+        cudaGetLastError();
+        blocks = (blocks + 1) / 2;
+    }
+    FMM_CUDA(err);
     FMM_CHECK_LAUNCH();
     LrOut o;
     read_small(&o, w.get(), sizeof(o), s);
