@@ -1391,13 +1391,13 @@ __global__ void __launch_bounds__(256) m2m_coef_kernel(
 // Step 5, L2L (l2dlocloc, laprouts2d.c:777-884) for the children of one
 // level whose parent holds points:  L_i += sum_{j>=i} A[cpos][i][j] Lp_j.
 // The children visited come from a BoxList or, with ids null, are all boxes
-// of [lo, hi); loc32 (optional) receives the FP32 copy of the final sums.
+// of [lo, hi).
 template <int CH>
 __global__ void __launch_bounds__(256) l2l_coef_kernel(
     int lo, int hi, int p, EvalCounts ec, const int *__restrict__ ids,
     const int *__restrict__ nids, const int *__restrict__ parent,
     const int *__restrict__ child, const double2 *__restrict__ A, int ndc,
-    int c0, double2 *__restrict__ loc, float2 *__restrict__ loc32) {
+    int c0, double2 *__restrict__ loc) {
     const int np1 = p + 1, stride = np1 * ndc;
     const int64_t n = (int64_t)(ids ? *nids : hi - lo) * np1;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n;
@@ -1420,10 +1420,8 @@ __global__ void __launch_bounds__(256) l2l_coef_kernel(
         }
 #pragma unroll
         for (int q = 0; q < CH; q++) {
-            const size_t o = (size_t)b * stride + (size_t)i * ndc + c0 + q;
-            const double2 r = cadd(loc[o], acc[q]);
-            loc[o] = r;
-            if (loc32) loc32[o] = make_float2((float)r.x, (float)r.y);
+            double2 &o = loc[(size_t)b * stride + (size_t)i * ndc + c0 + q];
+            o = cadd(o, acc[q]);
         }
     }
 }
@@ -2240,7 +2238,7 @@ void downward_chunk(const Tree &T, const CauchyProblem &P, int c0,
         const int *nid = P.l2l_ids ? P.l2l_cnt + l + 1 : nullptr;
         if (shift_matrix(P, nt))
             l2l_coef_kernel<CH><<<blocks(hi - lo), 256, 0, s>>>(
-                lo, hi, p, ec, ids, nid, T.parent.get(), T.child.get(), A, P.ndc, c0, loc, loc32);
+                lo, hi, p, ec, ids, nid, T.parent.get(), T.child.get(), A, P.ndc, c0, loc);
         else if (p + 1 <= 20)
             l2l_pascal_kernel<20><<<pascal_grid(nt), 128, 0, s>>>(
                 lo, hi, p, ec, ids, nid, T.parent.get(), T.child.get(), T.nchild.get(), P.ndc,

@@ -452,7 +452,6 @@ struct Builder {
         const int nref = read_scalar(tot.get(), s);
         if (nref == 0) return 0;
         ensure(T.nboxes + 4 * nref);
-        const int cap = T.cap;
         const int nb0 = T.nboxes;
         double2 *cen = T.centers.get();
         int *lev = T.level.get(), *par = T.parent.get(), *nch = T.nchild.get();
@@ -463,7 +462,6 @@ struct Builder {
             if (!fp[i]) return;
             const int b = lo + (int)i;
             const int base = nb0 + 4 * op[i];
-            if (base + 4 > cap) return;
             const double2 c = cen[b];
             const int cf = (set_flags && flg[b] == 1) ? 3 : 0;
             nch[b] = 4;
