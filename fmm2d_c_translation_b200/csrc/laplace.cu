@@ -1358,7 +1358,9 @@ __global__ void __launch_bounds__(256) m2m_coef_kernel(
         const int k = (int)(o / np1), i = (int)(o % np1), lane = (int)(t % LANES);
         const int b = ids ? ids[k] : lo + k;
         const bool par = valid && nchild[b] != 0;
-        const int nj = min(np1, (i & ~7) + 8);  // (entries j > i are zero)
+        // (entries j > i are zero; small levels are faster with one count for
+        // all lanes: a plan on 2e5 points of a curve 0.733 against 0.741 ms)
+        const int nj = LANES == 4 ? np1 : min(np1, (i & ~7) + 8);
         double2 acc[CH];
 #pragma unroll
         for (int q = 0; q < CH; q++) acc[q] = make_double2(0.0, 0.0);
