@@ -378,6 +378,7 @@ struct Builder {
     // Grow every per-box array to hold at least `need` boxes.
     void ensure(int need) {
         if (need <= T.cap) return;
+        if (need > kMaxBoxes) throw FmmError(4, "tree too large");
         int nc = std::max(need, T.cap + T.cap / 2 + 64);
         size_t keep = (size_t)T.nboxes;
         T.centers.grow(nc, keep, s);
